@@ -14,6 +14,7 @@
 // conv_zone_kernel: one CTA per (zone, set), 256 threads x 16 output bins,
 // register-tiled (16 x 16 products per 47 shared-memory loads).
 #include "relx_device.cuh"
+#include "relx_kernels.h"
 #include "relx_tma.cuh"
 
 namespace relx {
@@ -25,7 +26,6 @@ constexpr int kConvD = 16;         // window bins per step of the register tile
 constexpr int kN = RELX_NCONV;
 constexpr int kPre = 4;            // prefix sums are kept at every kPre-th bin
 constexpr int kXStage = 3072;      // xillver bins staged in shared memory (larger tables read global memory)
-constexpr int kTsumStage = 256;    // (tile, zone) profile sums staged in shared memory at once        // conv bins per thread whose rebin map entries are loaded together
 static_assert(kN % (kConvThreads * kPre) == 0, "scan tiling");
 
 // xs is stored in rows of 16 bins, each followed by 4 padding floats: the 16-byte loads of the
@@ -39,7 +39,6 @@ struct ConvSmem {
   float2 wsum[kConvThreads / 32];
   double dred[kConvThreads / 32 + 2];
   double zsum[RELX_NZMAX];
-  double tz[kTsumStage];       // the set's per-(tile, zone) profile sums
   float bc[2];                 // broadcast scalars
   float2 sxw;                  // band sum of xs
   int abort_flag;
@@ -85,40 +84,54 @@ __device__ __forceinline__ void conv_tile(const ConvSmem &m, int k0, int p, int 
   }
 }
 
-// relline renormalisation factor (renorm_relline_profile, Relprofile.cpp:766-781) and the zone
-// sums of the profile, from the per-(tile, zone) sums of the line kernel.  Warp 0: one lane per
-// zone sums its tiles in order, lane 0 sums the zones in order.  Results in m.zsum (scaled) and
-// m.bc[0] (scale).
-__device__ void profile_sums(ConvSmem &m, const RelxSetState &s, const double *tsum, int set, int ntile_max, int nza,
-                             int tile_bins) {
-  const int tid = threadIdx.x;
-  const int ntiles = (s.win_hi - s.win_lo + tile_bins - 1) / tile_bins;
-  const bool staged = ntiles * s.nz <= kTsumStage;
-  if (staged) {  // every (tile, zone) sum loaded at once
-    for (int q = tid; q < ntiles * s.nz; q += kConvThreads) {
-      const int t = q / s.nz, z = q - t * s.nz;
-      m.tz[q] = tsum[((size_t) set * ntile_max + t) * nza + z];
+// Profile sum of zone z, by one warp (every lane returns it): the line kernel's sums of 32 bins, added
+// in order within 256 bins (counted from the set's first profile bin), those in order.
+__device__ __forceinline__ double zone_sum_warp(const RelxSetState &s, const double *__restrict__ tsum, int set,
+                                                int nblk, int nza, int z) {
+  constexpr int per = 256 / kSumBinsH;
+  const int lane = threadIdx.x & 31;
+  if (s.zw_hi[z] <= s.zw_lo[z]) return 0.0;
+  // blocks outside the zone's window hold nothing
+  const int b0 = (s.zw_lo[z] - s.win_lo) / kSumBinsH, b1 = (s.zw_hi[z] - s.win_lo + kSumBinsH - 1) / kSumBinsH;
+  const double *t = tsum + (size_t) set * nblk * nza + z;
+  double zs = 0.0;
+  for (int g0 = b0 / per; g0 * per < b1; g0 += 32) {
+    const int g = g0 + lane;
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < per; q++) {
+      const int b = g * per + q;
+      if (b >= b0 && b < b1) v += t[(size_t) b * nza];
+    }
+    const int n = min(32, (b1 + per - 1) / per - g0);
+    for (int k = 0; k < n; k++) zs += __shfl_sync(0xffffffffu, v, k);
+  }
+  return zs;
+}
+
+// relline renormalisation factor (renorm_relline_profile, Relprofile.cpp:766-781) in m.bc[0] and the
+// (scaled) profile sum of zone z in m.zsum[z].  Without renormalisation (lamp post) the other zones'
+// sums are not needed.
+__device__ void profile_sums(ConvSmem &m, const RelxSetState &s, const double *tsum, int set, int nblk, int nza,
+                             int z) {
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (s.relline_norm > 0.0) {
+    for (int q = warp; q < s.nz; q += kConvThreads / 32) {
+      const double zs = zone_sum_warp(s, tsum, set, nblk, nza, q);
+      if ((tid & 31) == 0) m.zsum[q] = zs;
     }
     __syncthreads();
-  }
-  if (tid < 32) {
-    for (int z = tid; z < s.nz; z += 32) {
-      double zs = 0.0;
-      for (int t = 0; t < ntiles; t++) zs += staged ? m.tz[t * s.nz + z] : tsum[((size_t) set * ntile_max + t) * nza + z];
-      m.zsum[z] = zs;
+    if (tid == 0) {  // the zones' total in zone order, then the zone scaled
+      double sum = 0.0;
+      for (int q = 0; q < s.nz; q++) sum += m.zsum[q];
+      const double scale = s.relline_norm / sum;
+      m.bc[0] = (float) scale;
+      m.zsum[z] *= scale;
     }
-    if (s.relline_norm > 0.0) {  // renormalised profile: the zones' total in zone order, then each zone scaled
-      __syncwarp();
-      double scale = 0.0;
-      if (tid == 0) {
-        double sum = 0.0;
-        for (int z = 0; z < s.nz; z++) sum += m.zsum[z];
-        scale = s.relline_norm / sum;
-        m.bc[0] = (float) scale;
-      }
-      scale = __shfl_sync(0xffffffffu, scale, 0);
-      for (int z = tid; z < s.nz; z += 32) m.zsum[z] *= scale;
-    } else if (tid == 0) {
+  } else if (warp == 0) {
+    const double zs = zone_sum_warp(s, tsum, set, nblk, nza, z);
+    if (tid == 0) {
+      m.zsum[z] = zs;
       m.bc[0] = 1.0f;
     }
   }
@@ -243,8 +256,8 @@ __device__ void conv_normalize_store(ConvSmem &m, const RelxTables &tab, int wlo
 
 __global__ void __launch_bounds__(kConvThreads) conv_zone_kernel(RelxTables tab, const RelxSetState *__restrict__ sst,
                                                                  const float *__restrict__ prof,
-                                                                 const double *__restrict__ tsum, int ntile_max,
-                                                                 int tile_bins, const float *__restrict__ xill, int nza,
+                                                                 const double *__restrict__ tsum, int nblk,
+                                                                 const float *__restrict__ xill, int nza,
                                                                  float *__restrict__ cout, int *__restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ConvSmem &m = *reinterpret_cast<ConvSmem *>(smem_raw);
@@ -252,7 +265,7 @@ __global__ void __launch_bounds__(kConvThreads) conv_zone_kernel(RelxTables tab,
   const RelxSetState &s = sst[set];
   if (s.status != RELX_OK || s.model < RELX_RELXILL || z >= s.nz) return;
   float *out = cout + ((size_t) set * nza + z) * kN;
-  profile_sums(m, s, tsum, set, ntile_max, nza, tile_bins);
+  profile_sums(m, s, tsum, set, nblk, nza, z);
   // relxill_convolution_multizone skips zones without flux (Relxill.cpp:455-457)
   if (m.zsum[z] < 1e-12) {
     for (int k = s.out_lo + tid; k <= s.out_hi; k += kConvThreads) out[k] = 0.0f;
@@ -315,8 +328,8 @@ __global__ void __launch_bounds__(kConvThreads) conv_zone_kernel(RelxTables tab,
 __global__ void __launch_bounds__(kConvThreads) relconv_conv_kernel(RelxTables tab, const RelxSetIn *__restrict__ sin,
                                                                     const RelxSetState *__restrict__ sst,
                                                                     const float *__restrict__ prof,
-                                                                    const double *__restrict__ tsum, int ntile_max,
-                                                                    int tile_bins, int nza, const double *__restrict__ user_e,
+                                                                    const double *__restrict__ tsum, int nblk, int nza,
+                                                                    const double *__restrict__ user_e,
                                                                     const double *__restrict__ user_f, float *__restrict__ cout,
                                                                     int *__restrict__ sflag) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -337,15 +350,16 @@ __global__ void __launch_bounds__(kConvThreads) relconv_conv_kernel(RelxTables t
     if (tid == 0) sflag[set] = RELX_ERR_INPUT;
     return;
   }
-  profile_sums(m, s, tsum, set, ntile_max, nza, tile_bins);
+  profile_sums(m, s, tsum, set, nblk, nza, 0);
   const int wlo = s.win_lo, whi = s.win_hi;
+  const int zlo = s.zw_lo[0], zhi = s.zw_hi[0];  // the convolved zone's profile is zero outside
   const float fscale = m.bc[0];
   const float *pz = prof + (size_t) set * nza * kN;
   float2 pr = make_float2(0.0f, 0.0f);
   for (int i = tid; i < whi - wlo + kConvR; i += kConvThreads) {
     const int j = wlo + i;
     float v = 0.0f;
-    if (j < whi) {
+    if (j >= zlo && j < zhi) {
       const float fr = pz[j] * fscale;
       v = fr * tab.conv_cf[j];
       if (j >= tab.conv_band_lo && j <= tab.conv_band_hi) pr = ff_addf(pr, fr);
@@ -521,8 +535,8 @@ __global__ void __launch_bounds__(kFinThreads) finalize_relconv_kernel(RelxTable
 __global__ void __launch_bounds__(kFinThreads) finalize_relline_kernel(const RelxSetIn *__restrict__ sin,
                                                                         const RelxSetState *__restrict__ sst,
                                                                         const float *__restrict__ prof,
-                                                                        const double *__restrict__ tsum, int ntile_max,
-                                                                        int tile_bins, int nza, double *__restrict__ flux) {
+                                                                        const double *__restrict__ tsum, int nblk, int nza,
+                                                                        double *__restrict__ flux) {
   const int set = blockIdx.x, tid = threadIdx.x;
   const RelxSetState &s = sst[set];
   const RelxSetIn &in = sin[set];
@@ -534,28 +548,24 @@ __global__ void __launch_bounds__(kFinThreads) finalize_relline_kernel(const Rel
     return;
   }
   __shared__ double scale_sh;
-  if (tid == 0) {
-    // renorm_relline_profile (Relprofile.cpp:766-781): zones in order, tiles in order within a zone
+  if (tid < 32) {
+    // renorm_relline_profile (Relprofile.cpp:766-781): zones in order
     double scale = 1.0;
     if (s.relline_norm > 0.0) {
-      const int ntiles = (s.win_hi - s.win_lo + tile_bins - 1) / tile_bins;
       double sum = 0.0;
-      for (int z = 0; z < s.nz; z++) {
-        double zs = 0.0;
-        for (int t = 0; t < ntiles; t++) zs += tsum[((size_t) set * ntile_max + t) * nza + z];
-        sum += zs;
-      }
+      for (int z = 0; z < s.nz; z++) sum += zone_sum_warp(s, tsum, set, nblk, nza, z);
       scale = s.relline_norm / sum;
     }
-    scale_sh = scale;
+    if (tid == 0) scale_sh = scale;
   }
   __syncthreads();
   const double scale = scale_sh;
   const float *p = prof + in.e_off;
-  // bins outside the window hold 0; with an empty profile the reference's
-  // renormalisation multiplies 0 by relline_norm/0 and returns NaN, as here
-  for (int i = tid; i < nu; i += kFinThreads)
-    fo[i] = ((i >= s.win_lo && i < s.win_hi) ? (double) p[i] : 0.0) * scale;
+  // the profile is that of the last zone (line models have one); bins outside its window hold 0; with
+  // an empty profile the reference's renormalisation multiplies 0 by relline_norm/0 and returns NaN,
+  // as here
+  const int lo = s.zw_lo[s.nz - 1], hi = s.zw_hi[s.nz - 1];
+  for (int i = tid; i < nu; i += kFinThreads) fo[i] = ((i >= lo && i < hi) ? (double) p[i] : 0.0) * scale;
 }
 
 size_t conv_smem_bytes() { return sizeof(ConvSmem); }

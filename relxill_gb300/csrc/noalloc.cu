@@ -89,7 +89,7 @@ struct NoallocPtrs {
 };
 
 // carve the arrays of one call from the scratch; returns the bytes used
-static size_t carve(unsigned char *base, int model, int nza, int nbins, int ntile_max, int x_pad, int nrg,
+static size_t carve(unsigned char *base, int model, int nza, int nbins, int nblk, int x_pad, int nrg,
                     NoallocPtrs *p) {
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -106,7 +106,7 @@ static size_t carve(unsigned char *base, int model, int nza, int nbins, int ntil
   p->line_e = (double *) take(line ? sizeof(double) * (nbins + 1) : 0);
   p->prof = (float *) take(sizeof(float) * (line ? (size_t) nbins : (size_t) nza * RELX_NCONV));
   p->dist = (float *) take(sizeof(float) * nza * RELX_MAX_INCL);
-  p->tsum = (double *) take(sizeof(double) * ntile_max * nza);
+  p->tsum = (double *) take(sizeof(double) * nblk * nza);
   p->xill = (float *) take(sizeof(float) * (size_t) nza * x_pad);
   p->cout = (float *) take(sizeof(float) * (size_t) nza * RELX_NCONV);
   const bool cp = relx_is_cp(model);
@@ -228,12 +228,12 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
   if (model == RELX_RELXILLLPCP) nza = std::max(nza, runtime_zones(model, 1, nullptr, nullptr));
   if (nza < 1 || nza > RELX_NZMAX) return fail(RELX_ERR_ARG, "relx_eval_one_noalloc: zone count out of range");
   const int gbins = (kind == RELX_RELLINE) ? n_bins : RELX_NCONV;
-  const int ntile_max = (gbins + kSumBinsH - 1) / kSumBinsH;  // 256-bin profile-sum blocks
+  const int nblk = (gbins + kSumBinsH - 1) / kSumBinsH;  // profile-sum blocks
   unsigned char *base = nullptr;
   int st = scratch_for_device(dev, &base);
   if (st) return st;
   NoallocPtrs p;
-  if (carve(base, model, nza, n_bins, ntile_max, tab.x_cpad, tab.rel_nr * tab.rel_ng, &p) > kScratchBytes)
+  if (carve(base, model, nza, n_bins, nblk, tab.x_cpad, tab.rel_nr * tab.rel_ng, &p) > kScratchBytes)
     return fail(RELX_ERR_ARG, "relx_eval_one_noalloc: request exceeds the static scratch");
 
   noalloc_pack_kernel<<<1, 32, 0, s>>>(runtime_nparams(model), d_params, n_bins, ion_grad_type, iongrad_index,
@@ -250,24 +250,23 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
   setup_kernel<<<1, kSetupThreadsH, setup_smem_bytes(), s>>>(tab, model, p.sin, d_energy, p.line_e, p.sst, p.rad,
                                                             p.cor, p.zcor);
   if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, nza, false, p.nthq, p.nth, p.cor, p.zcor, p.nthscr, nza + 1, 0));
-  NOALLOC_CUDA(launch_line_table(1, s, tab, p.sst, p.htab));
-  NOALLOC_CUDA(launch_relline(relx_is_relxill(kind), 1, ntile_max, s, tab, p.sin, p.sst, p.rad, p.line_e, nza, p.prof,
-                              p.dist, p.tsum, kind == RELX_RELLINE || kind == RELX_RELCONV, nza > 1, p.htab));
+  NOALLOC_CUDA(launch_line_table(1, nza, s, tab, p.sst, p.htab, p.rad, nullptr, nullptr));
+  NOALLOC_CUDA(launch_relline(1, nblk, s, tab, p.sin, p.sst, p.rad, p.line_e, nza, p.prof, p.tsum,
+                              kind == RELX_RELLINE || kind == RELX_RELCONV, p.htab, nullptr, nullptr));
+  if (relx_is_relxill(kind)) NOALLOC_CUDA(launch_hist(1, s, tab, p.sst, p.rad, nza, p.dist, nza > 1, p.htab));
   if (relx_is_relxill(kind)) {
     NOALLOC_CUDA(launch_xillver(s, tab, 1, nza, nza > RELX_ZDENSE || cp, true, p.sst, p.cor, p.zcor, p.dist, p.xill,
                                 p.err, nullptr));
-    conv_zone_kernel<<<dim3(nza, 1), kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sst, p.prof, p.tsum, ntile_max,
-                                                                            kSumBinsH, p.xill, nza, p.cout,
+    conv_zone_kernel<<<dim3(nza, 1), kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sst, p.prof, p.tsum, nblk, p.xill, nza, p.cout,
                                                                             p.err);
     NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, tab, p.sin, p.sst, p.cout, nza, d_energy, d_flux,
                                          cp ? p.nth : nullptr));
   } else if (kind == RELX_RELCONV) {
-    relconv_conv_kernel<<<1, kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sin, p.sst, p.prof, p.tsum, ntile_max,
-                                                                    kSumBinsH, nza, d_energy, d_flux_in, p.cout,
+    relconv_conv_kernel<<<1, kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sin, p.sst, p.prof, p.tsum, nblk, nza, d_energy, d_flux_in, p.cout,
                                                                     p.sflag);
     finalize_relconv_kernel<<<1, kFinThreadsH, 0, s>>>(tab, p.sin, p.sst, p.cout, nza, d_energy, p.sflag, d_flux);
   } else {
-    finalize_relline_kernel<<<1, kFinThreadsH, 0, s>>>(p.sin, p.sst, p.prof, p.tsum, ntile_max, kSumBinsH, nza,
+    finalize_relline_kernel<<<1, kFinThreadsH, 0, s>>>(p.sin, p.sst, p.prof, p.tsum, nblk, nza,
                                                         d_flux);
   }
   noalloc_status_kernel<<<1, 32, 0, s>>>(p.sst, p.sflag, p.err, p.status, d_status);

@@ -18,6 +18,7 @@
 // fill before the line kernels, store after them).
 #include "relcache.h"
 #include "relx_device.cuh"
+#include "relx_kernels.h"
 
 namespace relx {
 
@@ -83,23 +84,20 @@ __global__ void cache_lookup_kernel(RelCacheDev c, const RelxSetIn *__restrict__
 
 // copy a cached entry into the batch's profile, tile-sum and histogram arrays
 __global__ void cache_fill_kernel(RelCacheDev c, const RelxSetState *__restrict__ sst, const int *__restrict__ slot_of,
-                                  int nza, int ntile_max, int tile_bins, float *__restrict__ prof,
+                                  int nza, int nblk, float *__restrict__ prof,
                                   double *__restrict__ tsum, float *__restrict__ dist) {
   const int set = blockIdx.x;
   const RelxSetState &s = sst[set];
   if (!s.cached) return;
   const int slot = slot_of[set];
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int wlo = s.win_lo, whi = s.win_hi;
-  for (int z = 0; z < s.nz; z++) {
+  for (int z = 0; z < s.nz; z++) {  // a zone's profile and sums exist in its own window only
     const float *src = c.prof + ((size_t) slot * kCacheZones + z) * RELX_NCONV;
     float *dst = prof + ((size_t) set * nza + z) * RELX_NCONV;
-    for (int j = wlo + tid; j < whi; j += nt) dst[j] = src[j];
-  }
-  const int ntiles = (whi - wlo + tile_bins - 1) / tile_bins;
-  for (int i = tid; i < ntiles * s.nz; i += nt) {
-    const int t = i / s.nz, z = i - t * s.nz;
-    tsum[((size_t) set * ntile_max + t) * nza + z] = c.tsum[((size_t) slot * kCacheTiles + t) * kCacheZones + z];
+    for (int j = s.zw_lo[z] + tid; j < s.zw_hi[z]; j += nt) dst[j] = src[j];
+    const int b1 = (s.zw_hi[z] - s.win_lo + kSumBinsH - 1) / kSumBinsH;
+    for (int t = (s.zw_lo[z] - s.win_lo) / kSumBinsH + tid; t < b1; t += nt)
+      tsum[((size_t) set * nblk + t) * nza + z] = c.tsum[((size_t) slot * kCacheTiles + t) * kCacheZones + z];
   }
   for (int i = tid; i < s.nz * RELX_MAX_INCL; i += nt)
     dist[(size_t) set * nza * RELX_MAX_INCL + i] = c.dist[(size_t) slot * kCacheZones * RELX_MAX_INCL + i];
@@ -108,23 +106,20 @@ __global__ void cache_fill_kernel(RelCacheDev c, const RelxSetState *__restrict_
 // store the results of the sets that claimed their slot
 __global__ void cache_store_kernel(RelCacheDev c, const RelxSetIn *__restrict__ sin,
                                    const RelxSetState *__restrict__ sst, const int *__restrict__ slot_of, int nza,
-                                   int ntile_max, int tile_bins, const float *__restrict__ prof,
+                                   int nblk, const float *__restrict__ prof,
                                    const double *__restrict__ tsum, const float *__restrict__ dist) {
   const int set = blockIdx.x;
   const RelxSetState &s = sst[set];
   const int slot = slot_of[set];
   if (slot < 0 || s.cached || s.status != RELX_OK || c.claim[slot] != set) return;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int wlo = s.win_lo, whi = s.win_hi;
   for (int z = 0; z < s.nz; z++) {
     const float *src = prof + ((size_t) set * nza + z) * RELX_NCONV;
     float *dst = c.prof + ((size_t) slot * kCacheZones + z) * RELX_NCONV;
-    for (int j = wlo + tid; j < whi; j += nt) dst[j] = src[j];
-  }
-  const int ntiles = (whi - wlo + tile_bins - 1) / tile_bins;
-  for (int i = tid; i < ntiles * s.nz; i += nt) {
-    const int t = i / s.nz, z = i - t * s.nz;
-    c.tsum[((size_t) slot * kCacheTiles + t) * kCacheZones + z] = tsum[((size_t) set * ntile_max + t) * nza + z];
+    for (int j = s.zw_lo[z] + tid; j < s.zw_hi[z]; j += nt) dst[j] = src[j];
+    const int b1 = (s.zw_hi[z] - s.win_lo + kSumBinsH - 1) / kSumBinsH;
+    for (int t = (s.zw_lo[z] - s.win_lo) / kSumBinsH + tid; t < b1; t += nt)
+      c.tsum[((size_t) slot * kCacheTiles + t) * kCacheZones + z] = tsum[((size_t) set * nblk + t) * nza + z];
   }
   const bool has_dist = relx_is_relxill(s.model);
   for (int i = tid; i < s.nz * RELX_MAX_INCL; i += nt)
@@ -195,15 +190,15 @@ cudaError_t cache_lookup(const RelCache &c, cudaStream_t s, const RelxSetIn *sin
 }
 
 cudaError_t cache_fill(const RelCache &c, cudaStream_t s, const RelxSetState *sst, const int *slot_of, int n_sets,
-                       int nza, int ntile_max, int tile_bins, float *prof, double *tsum, float *dist) {
-  cache_fill_kernel<<<n_sets, 256, 0, s>>>(c.d, sst, slot_of, nza, ntile_max, tile_bins, prof, tsum, dist);
+                       int nza, int nblk, float *prof, double *tsum, float *dist) {
+  cache_fill_kernel<<<n_sets, 256, 0, s>>>(c.d, sst, slot_of, nza, nblk, prof, tsum, dist);
   return cudaGetLastError();
 }
 
 cudaError_t cache_store(const RelCache &c, cudaStream_t s, const RelxSetIn *sin, const RelxSetState *sst,
-                        const int *slot_of, int n_sets, int nza, int ntile_max, int tile_bins, const float *prof,
+                        const int *slot_of, int n_sets, int nza, int nblk, const float *prof,
                         const double *tsum, const float *dist) {
-  cache_store_kernel<<<n_sets, 256, 0, s>>>(c.d, sin, sst, slot_of, nza, ntile_max, tile_bins, prof, tsum, dist);
+  cache_store_kernel<<<n_sets, 256, 0, s>>>(c.d, sin, sst, slot_of, nza, nblk, prof, tsum, dist);
   return cudaGetLastError();
 }
 

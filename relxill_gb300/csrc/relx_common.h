@@ -225,6 +225,8 @@ struct RelxRadial {
   double re[RELX_NFRAD];
   double ifac[RELX_NFRAD];    // FP64 radial factor (emission-angle bin decisions near bin edges)
   float  wt[RELX_NFRAD];      // trapez weight / 2
+  // lowest and highest line-profile bin that each group of eight consecutive radii of a zone reaches
+  int2 gr[RELX_NFRAD / 8 + RELX_NZMAX + 1];
 };
 static_assert(sizeof(RelxRadial) % 16 == 0, "per-set radial records stay 16-byte aligned");
 

@@ -11,14 +11,13 @@ namespace relx {
 
 constexpr int kSetupThreadsH = 256;
 constexpr int kLineThreadsH = 256;
-constexpr int kSumBinsH = 256;   // bins per profile-sum block (tsum)
-constexpr int kLineTileH = 512;  // energy bins per line-profile CTA
+constexpr int kSumBinsH = 32;    // bins per profile-sum block (tsum)
+constexpr int kLineTileH = 128;   // bins per task of the line profile of many sets
 constexpr int kConvThreadsH = 256;
 constexpr int kFinThreadsH = 128;
 constexpr int kXmodThreadsH = 256;  // xillver model kernel
 
 size_t setup_smem_bytes();
-size_t line_smem_bytes(int nr, int ng, bool limb, int tile);
 size_t hist_smem_bytes(int nr, int ng);
 size_t conv_smem_bytes();
 size_t fin_smem_bytes();
@@ -27,15 +26,17 @@ __global__ void setup_kernel(RelxTables tab, int model, const RelxSetIn *sin, co
                              RelxSetState *sout, RelxRadial *rout, RelxCorners *cout, RelxZoneCorners *zcout);
 
 cudaError_t relline_set_smem(int nr, int ng);
+// entries of the line profile's task list for n_sets sets
+size_t line_list_entries(int n_sets, int nza, int nblk);
 // the sets' (a, mu0)-interpolated transfer-function tables (rel_nr x rel_ng float4 per set), read
-// by the line profile and the emission-angle histogram
-cudaError_t launch_line_table(int n_sets, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
-                              float4 *htab);
-// nblk: 256-bin profile-sum blocks per set; htab: written by launch_line_table
-cudaError_t launch_relline(bool hist, int n_sets, int nblk, cudaStream_t s, const RelxTables &tab,
-                           const RelxSetIn *sin, const RelxSetState *sst, const RelxRadial *srad, const double *line_e,
-                           int nza, float *prof, float *dist, double *tsum, bool any_limb, bool zsplit,
-                           const float4 *htab);
+// by the line profile and the emission-angle histogram; the ranges of the groups of radii; and the
+// line profile's task list (line_list_entries entries and two zeroed counters; null: none)
+cudaError_t launch_line_table(int n_sets, int nza, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
+                              float4 *htab, RelxRadial *srad, uint2 *list, int *cnt);
+// nblk: 32-bin profile-sum blocks per set; htab, srad->gr, list, cnt: from launch_line_table
+cudaError_t launch_relline(int n_sets, int nblk, cudaStream_t s, const RelxTables &tab, const RelxSetIn *sin,
+                           const RelxSetState *sst, const RelxRadial *srad, const double *line_e, int nza, float *prof,
+                           double *tsum, bool any_limb, const float4 *htab, const uint2 *list, int *cnt);
 // the emission-angle histograms alone (relxill models), for a launch on its own stream
 cudaError_t launch_hist(int n_sets, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
                         const RelxRadial *srad, int nza, float *dist, bool zsplit, const float4 *htab);
@@ -99,9 +100,9 @@ cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_se
                                  const NthTable *nth);
 
 __global__ void conv_zone_kernel(RelxTables tab, const RelxSetState *sst, const float *prof, const double *tsum,
-                                 int ntile_max, int tile_bins, const float *xill, int nza, float *cout, int *err);
+                                 int nblk, const float *xill, int nza, float *cout, int *err);
 __global__ void relconv_conv_kernel(RelxTables tab, const RelxSetIn *sin, const RelxSetState *sst, const float *prof,
-                                    const double *tsum, int ntile_max, int tile_bins, int nza, const double *user_e,
+                                    const double *tsum, int nblk, int nza, const double *user_e,
                                     const double *user_f, float *cout, int *sflag);
 // nth: the nthcomp tables of the sets (Cp models), or null
 // zone sum, primary continuum and rebin to the caller's grid; wide: 512 threads per set (for few sets)
@@ -112,6 +113,6 @@ __global__ void finalize_relconv_kernel(RelxTables tab, const RelxSetIn *sin, co
                                         const float *cout, int nza, const double *user_e, const int *sflag,
                                         double *flux);
 __global__ void finalize_relline_kernel(const RelxSetIn *sin, const RelxSetState *sst, const float *prof,
-                                        const double *tsum, int ntile_max, int tile_bins, int nza, double *flux);
+                                        const double *tsum, int nblk, int nza, double *flux);
 
 }  // namespace relx

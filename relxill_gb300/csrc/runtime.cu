@@ -898,12 +898,12 @@ static int zones_for(int model, int ion_grad_type, int envn) {
 
 struct Workspace {
   DevBuf setin, st, rad, corners, zcorners, line_e, prof, dist, tsum, xill, cout, user_e, user_f, flux, sflag,
-      status, err, params, eoff, igt, igi, order, cslot, nthq, nthtab, nthscr, htab;
+      status, err, params, eoff, igt, igi, order, cslot, nthq, nthtab, nthscr, htab, list;
   Arena arena;  // set by use_arena: every buffer is carved from it
-  std::array<DevBuf *, 27> all() {
+  std::array<DevBuf *, 28> all() {
     return {&setin, &st, &rad, &corners, &zcorners, &line_e, &prof, &dist, &tsum, &xill, &cout, &user_e,
             &user_f, &flux, &sflag, &status, &err, &params, &eoff, &igt, &igi, &order, &cslot, &nthq,
-            &nthtab, &nthscr, &htab};
+            &nthtab, &nthscr, &htab, &list};
   }
   // carve the buffers from [base, base + bytes) from now on (the workspace holds no allocation)
   void use_arena(void *base, size_t bytes) {
@@ -1102,12 +1102,14 @@ static int prof_collect() {
 struct BatchShape {
   int model, n_sets, nza;
   int nz_min = 1;     // the smallest zone count of the batch's sets
-  int nblk;           // 256-bin profile-sum blocks per set
-  int line_tile = kLineTileH;  // energy bins per line-kernel CTA
+  int nblk;           // profile-sum blocks (kSumBinsH bins) per set
   int chunk = 0;      // sets per pipelined chunk (0: one range)
   bool any_limb = false;  // some set uses a limb-darkening law (relline / relconv limb parameter)
   int64_t n_edges;  // total energy edges
 };
+
+// the error flag, then the two task counters of the range of sets that starts at a set
+static size_t err_bytes(size_t n_sets) { return sizeof(int) * (4 + 2 * n_sets); }
 
 static int reserve_workspace(const Tables &T, Workspace &W, const BatchShape &b, bool need_zone_corners) {
   const size_t S = b.n_sets;
@@ -1117,7 +1119,7 @@ static int reserve_workspace(const Tables &T, Workspace &W, const BatchShape &b,
   if ((st = W.setin.reserve(S * sizeof(RelxSetIn))) || (st = W.st.reserve(S * sizeof(RelxSetState))) ||
       (st = W.user_e.reserve(b.n_edges * sizeof(double))) || (st = W.flux.reserve(b.n_edges * sizeof(double))) ||
       (st = W.sflag.reserve(S * sizeof(int))) || (st = W.status.reserve(S * sizeof(int))) ||
-      (st = W.err.reserve(sizeof(int))) || (st = W.cslot.reserve(S * sizeof(int))))
+      (st = W.err.reserve(err_bytes(S))) || (st = W.cslot.reserve(S * sizeof(int))))
     return st;
   if (relx_is_cp(b.model) &&
       ((st = W.nthq.reserve(S * (RELX_NZMAX + 1) * sizeof(double))) || (st = W.nthtab.reserve(S * sizeof(NthTable))) ||
@@ -1126,7 +1128,8 @@ static int reserve_workspace(const Tables &T, Workspace &W, const BatchShape &b,
   if (kind == RELX_XILLVER) return 0;  // no line profile, no convolution
   if ((st = W.rad.reserve(S * sizeof(RelxRadial))) || (st = W.dist.reserve(S * nza * RELX_MAX_INCL * sizeof(float))) ||
       (st = W.tsum.reserve(S * b.nblk * nza * sizeof(double))) ||
-      (st = W.htab.reserve(S * (size_t) T.d.rel_nr * T.d.rel_ng * sizeof(float4))))
+      (st = W.htab.reserve(S * (size_t) T.d.rel_nr * T.d.rel_ng * sizeof(float4))) ||
+      (st = W.list.reserve(line_list_entries((int) S, (int) nza, b.nblk) * sizeof(uint2))))
     return st;
   if (kind == RELX_RELLINE) {
     if ((st = W.line_e.reserve(b.n_edges * sizeof(double))) || (st = W.prof.reserve(b.n_edges * sizeof(float))))
@@ -1218,7 +1221,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     ProfScope ps(PK_SETUP, s, 2);
     if (C.cache_ev_valid) RELX_CUDA(cudaStreamWaitEvent(s, C.cache_ev, 0));
     RELX_CUDA(cache_lookup(C.cache, s, sin, sst, n, W.cslot.as<int>() + base));
-    RELX_CUDA(cache_fill(C.cache, s, sst, W.cslot.as<int>() + base, n, b.nza, b.nblk, kSumBinsH, prof, tsum,
+    RELX_CUDA(cache_fill(C.cache, s, sst, W.cslot.as<int>() + base, n, b.nza, b.nblk, prof, tsum,
                          dist));
   }
   // relxill models: the emission-angle histograms and the xillver zone spectra depend on the set-up
@@ -1230,19 +1233,17 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   const bool relxill = relx_is_relxill(kind);
   Context::Side *sd = (relxill && !g_prof.on) ? side_of(C, s) : nullptr;
   cudaStream_t xs = sd ? sd->side : s;
-  // few sets: a CTA per zone as well, so that the line profile and the histograms of a single
-  // spectrum spread over more SMs (the same numbers: zones are summed separately either way)
-  const int ntile = (b.nblk * kSumBinsH + kLineTileH - 1) / kLineTileH;
-  const bool zsplit = b.nza > 1 && (int64_t) n * ntile < 2 * 152;
+  uint2 *list = W.list.as<uint2>() ? W.list.as<uint2>() + line_list_entries(base, b.nza, b.nblk) : nullptr;
+  int *cnt = W.err.as<int>() + 4 + 2 * base;  // the range's task counters
   {
     ProfScope ps(PK_LINE, s, 2 + (b.any_limb ? 1 : 0));
-    RELX_CUDA(launch_line_table(n, s, tab, sst, htab));
+    RELX_CUDA(launch_line_table(n, b.nza, s, tab, sst, htab, rad, list, cnt));
     if (sd) {
       RELX_CUDA(cudaEventRecord(sd->fork, s));
       RELX_CUDA(cudaStreamWaitEvent(xs, sd->fork, 0));
     }
-    RELX_CUDA(launch_relline(false, n, b.nblk, s, tab, sin, sst, rad, W.line_e.as<double>(), b.nza, prof, dist, tsum,
-                             b.any_limb, zsplit, htab));
+    RELX_CUDA(launch_relline(n, b.nblk, s, tab, sin, sst, rad, W.line_e.as<double>(), b.nza, prof, tsum, b.any_limb,
+                             htab, list, cnt));
   }
   if (relxill) {
     {
@@ -1266,7 +1267,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   }
   if (cached) {
     ProfScope ps(PK_LINE, s);
-    RELX_CUDA(cache_store(C.cache, s, sin, sst, W.cslot.as<int>() + base, n, b.nza, b.nblk, kSumBinsH, prof,
+    RELX_CUDA(cache_store(C.cache, s, sin, sst, W.cslot.as<int>() + base, n, b.nza, b.nblk, prof,
                           tsum, dist));
     if (!C.cache_ev) RELX_CUDA(cudaEventCreateWithFlags(&C.cache_ev, cudaEventDisableTiming));
     RELX_CUDA(cudaEventRecord(C.cache_ev, s));
@@ -1275,8 +1276,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   if (relxill) {
     {
       ProfScope ps(PK_CONV, s);
-      conv_zone_kernel<<<dim3(b.nza, n), kConvThreadsH, conv_smem_bytes(), s>>>(tab, sst, prof, tsum, b.nblk,
-                                                                              kSumBinsH, xill, b.nza, cout,
+      conv_zone_kernel<<<dim3(b.nza, n), kConvThreadsH, conv_smem_bytes(), s>>>(tab, sst, prof, tsum, b.nblk, xill, b.nza, cout,
                                                                               W.err.as<int>());
     }
     {
@@ -1285,13 +1285,12 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
   } else if (kind == RELX_RELCONV) {
     ProfScope ps(PK_CONV, s, 2);  // convolution and finalize
-    relconv_conv_kernel<<<n, kConvThreadsH, conv_smem_bytes(), s>>>(tab, sin, sst, prof, tsum, b.nblk,
-                                                                    kSumBinsH, b.nza, user_e, W.user_f.as<double>(),
+    relconv_conv_kernel<<<n, kConvThreadsH, conv_smem_bytes(), s>>>(tab, sin, sst, prof, tsum, b.nblk, b.nza, user_e, W.user_f.as<double>(),
                                                                     cout, sflag);
     finalize_relconv_kernel<<<n, kFinThreadsH, 0, s>>>(tab, sin, sst, cout, b.nza, user_e, sflag, flux);
   } else {
     ProfScope ps(PK_FIN, s);
-    finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, kSumBinsH, b.nza, flux);
+    finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, b.nza, flux);
   }
   {
     ProfScope ps(PK_STATUS, s);
@@ -1313,7 +1312,7 @@ static int chunk_sets() {
 static int launch_direct(Context &C, Workspace &W, const BatchShape &b, cudaStream_t s, bool cached) {
   const int S = b.n_sets;
   RELX_CUDA(cudaMemsetAsync(W.sflag.p, 0, S * sizeof(int), s));
-  RELX_CUDA(cudaMemsetAsync(W.err.p, 0, sizeof(int), s));
+  RELX_CUDA(cudaMemsetAsync(W.err.p, 0, err_bytes(S), s));  // the error flag and the line tasks' counters
   const int chunk = b.chunk;
   if (cached || chunk <= 0 || S < 2 * chunk) return launch_range(C, W, b, s, 0, S, cached);
   for (int k = 0; k < 2; k++) {
@@ -1336,10 +1335,11 @@ static int launch_direct(Context &C, Workspace &W, const BatchShape &b, cudaStre
 
 static std::vector<uintptr_t> graph_key(const Workspace &W, const BatchShape &b) {
   std::vector<uintptr_t> k = {(uintptr_t) b.model, (uintptr_t) b.n_sets, (uintptr_t) b.nza, (uintptr_t) b.nz_min,
-                              (uintptr_t) b.nblk, (uintptr_t) b.line_tile, (uintptr_t) b.chunk,
+                              (uintptr_t) b.nblk, (uintptr_t) b.chunk,
                               (uintptr_t) b.any_limb, (uintptr_t) b.n_edges};
   for (const DevBuf *d : {&W.setin, &W.st, &W.rad, &W.corners, &W.zcorners, &W.line_e, &W.prof, &W.dist, &W.tsum,
-                          &W.xill, &W.cout, &W.user_e, &W.user_f, &W.flux, &W.sflag, &W.status, &W.err, &W.order})
+                          &W.xill, &W.cout, &W.user_e, &W.user_f, &W.flux, &W.sflag, &W.status, &W.err, &W.order,
+                          &W.htab, &W.list, &W.nthq, &W.nthtab, &W.nthscr})
     k.push_back((uintptr_t) d->p);
   return k;
 }
@@ -1438,7 +1438,6 @@ static int tuned_launch(Context &C, Workspace &W, BatchShape &b, cudaStream_t s,
   for (const auto &t : C.tune)
     if (t.model == b.model && t.sclass == sclass && t.nza == b.nza) known = &t;
   const bool explicit_choice = std::getenv("RELX_CHUNK_SETS") != nullptr;
-  b.line_tile = kLineTileH;
   if (known && !cached && !explicit_choice) b.chunk = known->chunk;
   // the candidates: one range, or pipelined chunks of 1024 sets for large batches
   if (known || !allow_tune || !C.autotune_on || g_prof.on || cached || explicit_choice ||
@@ -1448,17 +1447,15 @@ static int tuned_launch(Context &C, Workspace &W, BatchShape &b, cudaStream_t s,
     C.tune.push_back(Context::TuneEntry{b.model, sclass, b.nza, kLineTileH, 0, {0, 0, 0, 0}});
     return launch_batch(C, W, b, s, use_cache);
   }
-  struct Cand { int tile, chunk; };
-  std::vector<Cand> cands = {{kLineTileH, 0}, {kLineTileH, 1024}};
+  const std::vector<int> cands = {0, 1024};
   cudaEvent_t e0, e1;
   RELX_CUDA(cudaEventCreate(&e0));
   RELX_CUDA(cudaEventCreate(&e1));
-  Context::TuneEntry t{b.model, sclass, b.nza, 512, 0, {0, 0, 0, 0}};
+  Context::TuneEntry t{b.model, sclass, b.nza, kLineTileH, 0, {0, 0, 0, 0}};
   float best = 1e30f;
   int st = 0;
   for (size_t i = 0; i < cands.size() && !st; i++) {
-    b.line_tile = cands[i].tile;
-    b.chunk = cands[i].chunk;
+    b.chunk = cands[i];
     // an untimed launch first: the first launches of a process also load the kernels
     if ((st = launch_direct(C, W, b, s, false))) break;
     cudaEventRecord(e0, s);
@@ -1470,8 +1467,7 @@ static int tuned_launch(Context &C, Workspace &W, BatchShape &b, cudaStream_t s,
       t.ms[i] = ms;
       if (ms < best) {
         best = ms;
-        t.line_tile = cands[i].tile;
-        t.chunk = cands[i].chunk;
+        t.chunk = cands[i];
       }
     }
   }
@@ -1479,7 +1475,6 @@ static int tuned_launch(Context &C, Workspace &W, BatchShape &b, cudaStream_t s,
   cudaEventDestroy(e1);
   if (st) return st;
   C.tune.push_back(t);
-  b.line_tile = t.line_tile;
   b.chunk = t.chunk;
   return 0;  // the workspace holds the last trial's results
 }
@@ -1775,12 +1770,12 @@ size_t batch_device_bytes(int model, int n_sets, int64_t n_edges, int max_bins, 
   const int kind = relx_kind(model);
   const size_t S = (size_t) n_sets, E = (size_t) n_edges;
   // parameters, grid offsets and the ionisation-gradient arrays (enqueue_host_batch), and the
-  // 256-byte rounding of each of the workspace's 27 buffers
+  // 256-byte rounding of each of the workspace's 28 buffers
   const size_t staged = S * (sizeof(double) * RELX_NPARAM_MAX + sizeof(int64_t) + sizeof(int) + sizeof(double)) +
-                        sizeof(int64_t) + 27 * 256 + 256;
+                        sizeof(int64_t) + 28 * 256 + 256;
   const size_t cp = relx_is_cp(model) ? S * (sizeof(NthTable) + sizeof(double) * (RELX_NZMAX + 1)) : 0;
   if (kind == RELX_XILLVER)
-    return staged + cp + S * (sizeof(RelxSetIn) + sizeof(RelxSetState) + sizeof(int) * 4) + sizeof(int) +
+    return staged + cp + S * (sizeof(RelxSetIn) + sizeof(RelxSetState) + sizeof(int) * 4) + err_bytes(S) +
            (relx_is_cp(model) ? nthcomp_scratch_bytes(n_sets, 1, true) : 0) + sizeof(double) * 2 * E;
   const int gmax = (kind == RELX_RELLINE) ? std::max(max_bins, 1) : RELX_NCONV;
   const size_t nblk = (size_t) (gmax + kSumBinsH - 1) / kSumBinsH;
@@ -1794,7 +1789,8 @@ size_t batch_device_bytes(int model, int n_sets, int64_t n_edges, int max_bins, 
   if (relx_is_relxill(kind))
     per_set += sizeof(RelxCorners) + sizeof(float) * (size_t) nza * 4096;
   if (relx_is_cp(model) || nza > RELX_ZDENSE) per_set += sizeof(RelxZoneCorners);
-  return staged + cp + per_set * S + per_edge * E + sizeof(int) +
+  return staged + cp + per_set * S + per_edge * E + err_bytes(S) +
+         line_list_entries(n_sets, nza, (int) nblk) * sizeof(uint2) +
          (relx_is_cp(model) ? nthcomp_scratch_bytes(n_sets, nza, false) : 0);
 }
 
