@@ -44,6 +44,8 @@ cudaError_t launch_hist(int n_sets, cudaStream_t s, const RelxTables &tab, const
 cudaError_t xillver_set_smem(int n_incl);
 // bounded-wait self-test: writes the status of a wait that cannot complete (RELX_ERR_TIMEOUT)
 cudaError_t launch_wait_selftest(cudaStream_t s, unsigned long long limit_ns, int *out);
+// whether the dense kernel visits this many sets in table-row order (launch_xill_order)
+bool xill_sorted(int n_sets);
 // order: the sets in visiting order (launch_xill_order), or null for batch order
 cudaError_t launch_xillver(cudaStream_t s, const RelxTables &tab, int n_sets, int nza, bool zone, bool dense,
                            const RelxSetState *sst, const RelxCorners *cor, const RelxZoneCorners *zcor,

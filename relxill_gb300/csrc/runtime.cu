@@ -1255,9 +1255,10 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
       // corners do not fit the de-duplicated list; the dense kernel, in table-row order, for the rest
       const bool zone = b.nza > RELX_ZDENSE || cp;
       const bool dense = b.nz_min <= RELX_ZDENSE;
-      ProfScope ps(PK_XILL, xs, (zone ? 1 : 0) + (dense ? 2 : 0));
-      int *order = dense ? W.order.as<int>() + base : nullptr;
-      if (dense) launch_xill_order(xs, sst, cor, zcor, n, order);
+      const bool sort = dense && xill_sorted(n);
+      ProfScope ps(PK_XILL, xs, (zone ? 1 : 0) + (dense ? 1 : 0) + (sort ? 1 : 0));
+      int *order = sort ? W.order.as<int>() + base : nullptr;
+      if (sort) launch_xill_order(xs, sst, cor, zcor, n, order);
       RELX_CUDA(launch_xillver(xs, tab, n, b.nza, zone, dense, sst, cor, zcor, dist, xill, W.err.as<int>(), order));
     }
     if (sd) {

@@ -20,14 +20,17 @@
 // waits are bounded and report a timeout through the error flag instead of
 // hanging.
 #include "relx_device.cuh"
+#include "relx_kernels.h"
 #include "relx_tma.cuh"
 
 namespace relx {
 
 constexpr int kXillThreads = 128;
-constexpr int kXillTile = 512;    // floats per row segment (2 KB), one float4 per thread
+constexpr int kXillTile = 4 * kXillThreads;  // floats per row segment (2 KB), one float4 per thread
 constexpr int kXillStages = 2;
-static_assert(kXillTile == 4 * kXillThreads, "one float4 per thread");
+// few sets: tiles of 128 floats, so that a set spreads over 20 CTAs instead of 5, and eight corners in flight
+// instead of two (a single set waits for its copies)
+constexpr int kXillFewThreads = 32, kXillFewStages = 8;
 
 // Self-test of the timeout path: one thread waits, with a short limit, on an mbarrier that
 // expects 16 bytes no copy will deliver, and reports what the wait returned.  No copy is issued,
@@ -46,15 +49,15 @@ cudaError_t launch_wait_selftest(cudaStream_t s, unsigned long long limit_ns, in
   return cudaGetLastError();
 }
 
-template <int NZ>
+template <int NZ, int STAGES>
 struct XillSmem {
-  uint64_t full[kXillStages];
+  uint64_t full[STAGES];
   float w[RELX_MAX_UCORNER][NZ];        // corner weight per zone
   float dist[NZ][RELX_MAX_INCL];        // normalised emission-angle distribution per zone
   int row[RELX_MAX_UCORNER];
   int abort_flag;
   int pad_[3];
-  float4 stage[1];  // [kXillStages][n_incl][kXillTile/4], dynamic tail
+  float4 stage[1];  // [STAGES][n_incl][threads], dynamic tail
 };
 
 // Order in which the xillver kernel visits the sets: sets whose zones use the same table rows run
@@ -70,7 +73,9 @@ __global__ void __launch_bounds__(kOrderThreads) xill_order_kernel(const RelxSet
   __shared__ unsigned long long key[kOrderN];
   const int base = blockIdx.x * kOrderN;
   const int n = min(kOrderN, n_sets - base);
-  for (int i = threadIdx.x; i < kOrderN; i += kOrderThreads) {
+  int N = 2;  // the power of two that holds the chunk's sets
+  while (N < n) N <<= 1;
+  for (int i = threadIdx.x; i < N; i += kOrderThreads) {
     unsigned long long k = ~0ull;
     if (i < n) {
       const int set = base + i;
@@ -88,9 +93,9 @@ __global__ void __launch_bounds__(kOrderThreads) xill_order_kernel(const RelxSet
     key[i] = k;
   }
   __syncthreads();
-  for (int size = 2; size <= kOrderN; size <<= 1) {
+  for (int size = 2; size <= N; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < kOrderN / 2; i += kOrderThreads) {
+      for (int i = threadIdx.x; i < N / 2; i += kOrderThreads) {
         const int lo = 2 * i - (i & (stride - 1));
         const int hi = lo + stride;
         const bool up = (lo & size) == 0;
@@ -110,14 +115,15 @@ void launch_xill_order(cudaStream_t s, const RelxSetState *sst, const RelxCorner
 
 // NZ: zones held in registers (a set with more zones runs in a wider instance);
 // NI: inclinations unrolled at compile time (0: any count up to RELX_MAX_INCL).
-template <int NZ, int NI>
-__global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTables tab, const RelxSetState *__restrict__ sst,
+// THREADS: tile of 4 THREADS floats; STAGES: corners in flight.
+template <int NZ, int NI, int THREADS, int STAGES>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) xillver_dense_kernel(RelxTables tab, const RelxSetState *__restrict__ sst,
                                                                         const RelxCorners *__restrict__ scor,
                                                                         const float *__restrict__ dist_raw, int nza,
                                                                         float *__restrict__ xout, int *__restrict__ err,
                                                                         const int *__restrict__ order) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  XillSmem<NZ> &m = *reinterpret_cast<XillSmem<NZ> *>(smem_raw);
+  XillSmem<NZ, STAGES> &m = *reinterpret_cast<XillSmem<NZ, STAGES> *>(smem_raw);
   const int set = order ? order[blockIdx.y] : blockIdx.y, tile = blockIdx.x;
   const RelxSetState &s = sst[set];
   if (s.status != RELX_OK || s.model < RELX_RELXILL || !s.xdense || s.nz > NZ) return;
@@ -125,18 +131,18 @@ __global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTabl
   const int tid = threadIdx.x;
   const int nz = s.nz, U = s.ucount, ni = NI > 0 ? NI : tab.x_nincl;
   const int pitch = tab.x_cpad;  // table rows on the conv grid
-  const int e0 = tile * kXillTile;
+  const int e0 = tile * (4 * THREADS);
   if (e0 >= pitch) return;
-  const int len = min(kXillTile, pitch - e0);  // multiple of 4 floats (16 bytes)
+  const int len = min((4 * THREADS), pitch - e0);  // multiple of 4 floats (16 bytes)
   const uint32_t bytes_row = (uint32_t) len * 4u;
 
   // weights and normalised emission-angle distributions (renorm_relline_profile, Relprofile.cpp:783-795)
   const RelxCorners &C = scor[set];
-  for (int i = tid; i < U * NZ; i += kXillThreads) {
+  for (int i = tid; i < U * NZ; i += THREADS) {
     const int u = i / NZ, z = i - u * NZ;
     m.w[u][z] = (z < nz) ? C.w[u][z] : 0.0f;
   }
-  for (int i = tid; i < U; i += kXillThreads) m.row[i] = C.row[i];
+  for (int i = tid; i < U; i += THREADS) m.row[i] = C.row[i];
   if (tid < nz) {
     const float *d = dist_raw + ((size_t) set * nza + tid) * RELX_MAX_INCL;
     float sum = 0.0f;
@@ -145,20 +151,20 @@ __global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTabl
   }
   if (tid == 0) {
     m.abort_flag = 0;
-    for (int st = 0; st < kXillStages; st++) mbar_init(&m.full[st], 1);
+    for (int st = 0; st < STAGES; st++) mbar_init(&m.full[st], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   auto issue = [&](int u) {
-    const int st = u % kXillStages;
+    const int st = u % STAGES;
     mbar_expect_tx(&m.full[st], bytes_row * (uint32_t) ni);
     const float *src = tab.x_cspec + (size_t) m.row[u] * pitch + e0;
     for (int i = 0; i < ni; i++)
-      bulk_g2s(&m.stage[(st * ni + i) * (kXillTile / 4)], src + (size_t) i * pitch, bytes_row, &m.full[st]);
+      bulk_g2s(&m.stage[(st * ni + i) * THREADS], src + (size_t) i * pitch, bytes_row, &m.full[st]);
   };
   int issued = 0;  // meaningful in thread 0 only
   if (tid == 0)
-    for (int u = 0; u < min(U, kXillStages); u++) { issue(u); issued = u + 1; }
+    for (int u = 0; u < min(U, STAGES); u++) { issue(u); issued = u + 1; }
 
   float4 acc[NZ];
 #pragma unroll
@@ -167,8 +173,8 @@ __global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTabl
   const bool active = q * 4 < len;
   int u_stop = U;
   for (int u = 0; u < U; u++) {
-    const int st = u % kXillStages;
-    const uint32_t parity = (uint32_t) ((u / kXillStages) & 1);
+    const int st = u % STAGES;
+    const uint32_t parity = (uint32_t) ((u / STAGES) & 1);
     if (!mbar_wait_bounded(&m.full[st], parity)) atomicExch(&m.abort_flag, 1);
     __syncthreads();
     if (m.abort_flag) { u_stop = u; break; }
@@ -176,7 +182,7 @@ __global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTabl
       float4 v[NIU];
 #pragma unroll
       for (int i = 0; i < NIU; i++)
-        if (i < ni) v[i] = m.stage[(st * ni + i) * (kXillTile / 4) + q];
+        if (i < ni) v[i] = m.stage[(st * ni + i) * THREADS + q];
 #pragma unroll
       for (int z = 0; z < NZ; z++) {
         const float wz = m.w[u][z];
@@ -194,13 +200,13 @@ __global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTabl
       }
     }
     __syncthreads();  // stage st is free again
-    if (tid == 0 && u + kXillStages < U) { issue(u + kXillStages); issued = u + kXillStages + 1; }
+    if (tid == 0 && u + STAGES < U) { issue(u + STAGES); issued = u + STAGES + 1; }
   }
   if (m.abort_flag) {
     // wait (bounded) for the copies this CTA still has in flight, then report
     if (tid == 0) {
       for (int u = u_stop; u < issued; u++)
-        (void) mbar_wait_bounded(&m.full[u % kXillStages], (uint32_t) ((u / kXillStages) & 1));
+        (void) mbar_wait_bounded(&m.full[u % STAGES], (uint32_t) ((u / STAGES) & 1));
       atomicExch(err, RELX_ERR_TIMEOUT);
     }
     return;
@@ -216,9 +222,9 @@ __global__ void __launch_bounds__(kXillThreads, 4) xillver_dense_kernel(RelxTabl
   }
 }
 
-template <int NZ>
+template <int NZ, int THREADS, int STAGES>
 static size_t xill_smem_nz(int n_incl) {
-  return sizeof(XillSmem<NZ>) + sizeof(float4) * ((size_t) kXillStages * n_incl * (kXillTile / 4) - 1);
+  return sizeof(XillSmem<NZ, STAGES>) + sizeof(float4) * ((size_t) STAGES * n_incl * THREADS - 1);
 }
 
 // Sets without the de-duplicated corner list (more than RELX_ZDENSE zones, or more distinct rows than
@@ -408,22 +414,38 @@ __global__ void __launch_bounds__(kXillThreads) xillver_zone_kernel(RelxTables t
 
 #define RELX_XILL_INSTANCES(X) X(1, 10) X(10, 10) X(16, 10) X(1, 0) X(10, 0) X(16, 0)
 
+template <int NZ, int NI, int THREADS, int STAGES>
+static cudaError_t dense_smem(int n_incl) {
+  return cudaFuncSetAttribute(xillver_dense_kernel<NZ, NI, THREADS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int) xill_smem_nz<NZ, THREADS, STAGES>(n_incl));
+}
+template <int NZ, int NI, int THREADS, int STAGES>
+static void dense_launch(cudaStream_t s, const RelxTables &tab, int n_sets, int nza, const RelxSetState *sst,
+                         const RelxCorners *cor, const float *dist, float *xout, int *err, const int *order) {
+  const dim3 grid((tab.x_cpad + 4 * THREADS - 1) / (4 * THREADS), n_sets);
+  xillver_dense_kernel<NZ, NI, THREADS, STAGES><<<grid, THREADS, xill_smem_nz<NZ, THREADS, STAGES>(tab.x_nincl), s>>>(
+      tab, sst, cor, dist, nza, xout, err, order);
+}
+
 cudaError_t xillver_set_smem(int n_incl) {
+  cudaError_t e;
 #define X(nz, ni)                                                                                   \
-  {                                                                                                 \
-    cudaError_t e = cudaFuncSetAttribute(xillver_dense_kernel<nz, ni>,                              \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,               \
-                                         (int) xill_smem_nz<nz>(n_incl));                           \
-    if (e != cudaSuccess) return e;                                                                 \
-  }
+  if ((e = dense_smem<nz, ni, kXillThreads, kXillStages>(n_incl)) != cudaSuccess) return e;         \
+  if ((e = dense_smem<nz, ni, kXillFewThreads, kXillFewStages>(n_incl)) != cudaSuccess) return e;
   RELX_XILL_INSTANCES(X)
 #undef X
-  const cudaError_t e = cudaFuncSetAttribute(xillver_zone_kernel<10>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(xillver_zone_kernel<10>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int) xill_zone_smem(RELX_NZMAX, 32));
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(xillver_zone_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int) xill_zone_smem(RELX_NZMAX, 32));
 }
+
+// up to 64 sets every CTA is resident at once: nothing is gained by rows shared in time, and the sort
+// would be a tenth of the stage
+bool xill_sorted(int n_sets) { return n_sets > 64; }
+// the dense kernel's small tiles; us with small / large tiles, 10 zones: 1 set 19 / 24, 16 24 / 30, 32 37 / 32
+static bool xill_few(int n_sets) { return n_sets <= 16; }
 
 // xillver stage of a batch: the dense kernel (instance by the batch's zone count and the table's
 // inclination count) for the sets with the de-duplicated corner list, the zone kernel for the others.
@@ -440,10 +462,12 @@ cudaError_t launch_xillver(cudaStream_t s, const RelxTables &tab, int n_sets, in
   if (!dense) return cudaGetLastError();
   const int nzk = nza <= 1 ? 1 : (nza <= 10 ? 10 : 16);
   const int nik = tab.x_nincl == 10 ? 10 : 0;
-#define X(nz, ni)                                                                                           \
-  if (nzk == nz && nik == ni)                                                                               \
-    xillver_dense_kernel<nz, ni><<<grid, kXillThreads, xill_smem_nz<nz>(tab.x_nincl), s>>>(tab, sst, cor, dist, \
-                                                                                         nza, xout, err, order);
+  const bool few = xill_few(n_sets);
+#define X(nz, ni)                                                                                                      \
+  if (nzk == nz && nik == ni) {                                                                                        \
+    if (few) dense_launch<nz, ni, kXillFewThreads, kXillFewStages>(s, tab, n_sets, nza, sst, cor, dist, xout, err, order); \
+    else dense_launch<nz, ni, kXillThreads, kXillStages>(s, tab, n_sets, nza, sst, cor, dist, xout, err, order);       \
+  }
   RELX_XILL_INSTANCES(X)
 #undef X
   return cudaGetLastError();
