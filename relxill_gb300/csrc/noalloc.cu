@@ -247,8 +247,7 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
     runtime_set_error(RELX_OK, "");
     return RELX_OK;
   }
-  setup_kernel<<<1, kSetupThreadsH, setup_smem_bytes(), s>>>(tab, model, p.sin, d_energy, p.line_e, p.sst, p.rad,
-                                                            p.cor, p.zcor);
+  NOALLOC_CUDA(launch_setup(s, 1, tab, model, p.sin, d_energy, p.line_e, p.sst, p.rad, p.cor, p.zcor));
   if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, nza, false, p.nthq, p.nth, p.cor, p.zcor, p.nthscr, nza + 1, 0));
   NOALLOC_CUDA(launch_line_table(1, nza, s, tab, p.sst, p.htab, p.rad, nullptr, nullptr));
   NOALLOC_CUDA(launch_relline(1, nblk, s, tab, p.sin, p.sst, p.rad, p.line_e, nza, p.prof, p.tsum,

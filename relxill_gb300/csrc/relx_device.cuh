@@ -271,14 +271,15 @@ __device__ __forceinline__ float2 block_sum_ff(float2 v, float2 *scratch) {
   return r;
 }
 
-// block-wide sum in FP64 with a fixed reduction tree (deterministic)
+// block-wide sum in FP64 with a fixed reduction tree (deterministic); in a block of more than NT threads
+// the sum over the first NT
 template <int NT>
 __device__ __forceinline__ double block_sum_d(double v, double *scratch) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
-  if (lane == 0) scratch[w] = v;
+  if (lane == 0 && w < NT / 32) scratch[w] = v;
   __syncthreads();
   double r = 0.0;
   if (threadIdx.x == 0) {

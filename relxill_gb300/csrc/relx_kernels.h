@@ -9,7 +9,6 @@
 
 namespace relx {
 
-constexpr int kSetupThreadsH = 256;
 constexpr int kLineThreadsH = 256;
 constexpr int kSumBinsH = 32;    // bins per profile-sum block (tsum)
 constexpr int kLineTileH = 128;   // bins per task of the line profile of many sets
@@ -17,13 +16,14 @@ constexpr int kConvThreadsH = 256;
 constexpr int kFinThreadsH = 128;
 constexpr int kXmodThreadsH = 256;  // xillver model kernel
 
-size_t setup_smem_bytes();
 size_t hist_smem_bytes(int nr, int ng);
 size_t conv_smem_bytes();
 size_t fin_smem_bytes();
 
-__global__ void setup_kernel(RelxTables tab, int model, const RelxSetIn *sin, const double *user_e, double *line_e,
-                             RelxSetState *sout, RelxRadial *rout, RelxCorners *cout, RelxZoneCorners *zcout);
+cudaError_t setup_set_smem();
+cudaError_t launch_setup(cudaStream_t s, int n_sets, const RelxTables &tab, int model, const RelxSetIn *sin,
+                         const double *user_e, double *line_e, RelxSetState *sout, RelxRadial *rout,
+                         RelxCorners *cout, RelxZoneCorners *zcout);
 
 cudaError_t relline_set_smem(int nr, int ng);
 // entries of the line profile's task list for n_sets sets

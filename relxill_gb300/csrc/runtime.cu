@@ -976,9 +976,7 @@ static Context &ctx() {
 }
 
 static int set_kernel_attrs(const Tables &T) {
-  RELX_CUDA(cudaFuncSetAttribute(setup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) setup_smem_bytes()));
-  // four set-up CTAs per SM (52 KB each): the largest shared-memory carve-out
-  RELX_CUDA(cudaFuncSetAttribute(setup_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  RELX_CUDA(setup_set_smem());
   RELX_CUDA(relline_set_smem(T.d.rel_nr, T.d.rel_ng));
   RELX_CUDA(nthcomp_set_smem());
   RELX_CUDA(xillver_set_smem(T.d.x_nincl));
@@ -1209,8 +1207,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   }
   {
     ProfScope ps(PK_SETUP, s);
-    setup_kernel<<<n, kSetupThreadsH, setup_smem_bytes(), s>>>(tab, b.model, sin, user_e, W.line_e.as<double>(), sst,
-                                                               rad, cor, zcor);
+    RELX_CUDA(launch_setup(s, n, tab, b.model, sin, user_e, W.line_e.as<double>(), sst, rad, cor, zcor));
   }
   if (cp) {  // the nthcomp continua of the source and the zones, their normalisations on the corner weights
     ProfScope ps(PK_NTH, s, 2);

@@ -13,10 +13,13 @@
 // normalisation sums; per-radius transcendental work that has no
 // cancellation runs in FP32.
 #include "relx_device.cuh"
+#include "relx_kernels.h"
 
 namespace relx {
 
-constexpr int kSetupThreads = 256;
+constexpr int kSetupThreads = 256;      // threads of a set's CTA; the order of the block sums is theirs
+constexpr int kSetupFewThreads = 1024;  // few sets: more threads for the per-radius and per-sample loops
+constexpr int kStageVals = 256;         // xillver parameter values staged in shared memory
 constexpr int kQGroup = 8;
 constexpr double kDeg75 = 75.0 / 180.0 * 3.14159265358979323846;  // 75 degrees in radians  // continua summed together (normalisation of the primary continuum)
 // the table normalisation's unit factor (Xillspec.cpp:179-205), one product
@@ -55,7 +58,8 @@ struct SetupSmem {
   unsigned char lp_log[RELX_MAX_NRADLP];  // logarithmic radial factor (emission angle above 75 deg)
   double qsum[RELX_NZMAX + 1];       // normalisation sums of the primary continuum
   float qecut[RELX_NZMAX + 1];       // their cut-off energies
-  float2 qpart[kSetupThreads / 32][8];  // per-warp partial sums of a group of continua
+  float2 qpart[kSetupFewThreads / 32][8];  // per-warp partial sums of a group of continua
+  float xvals[kStageVals];           // the xillver table's parameter values
   float cpow[RELX_NCOARSE];          // E^-Gamma at the coarse-grid bin centres
   double jet_rad[RELX_MAX_NRADLP], d_tab[RELX_MAX_NRADLP];
   double red[40];
@@ -247,6 +251,26 @@ __device__ void map_params(int model, const RelxSetIn &in, SetupSmem &m) {
   }
 }
 
+// bsearch_asc (largest k in [0, n - 2] with a[k] <= v, 0 below) of an ascending array, by one warp: one round of
+// loads instead of a chain of them
+template <typename T>
+__device__ __forceinline__ int bsearch_asc_warp(const T *a, int n, T v) {
+  int cnt = 0;
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    const int k = k0 + (threadIdx.x & 31);
+    cnt += __popc(__ballot_sync(0xffffffffu, k < n && !(a[k] > v)));
+  }
+  return max(0, min(cnt - 1, n - 2));
+}
+
+// by one warp of a 1024-thread CTA, by its first lane in a 256-thread one (where a chain of loads is covered by
+// the SM's other CTAs)
+template <int NT, typename T>
+__device__ __forceinline__ int bsearch_asc_nt(const T *a, int n, T v) {
+  if constexpr (NT != kSetupThreads) return bsearch_asc_warp<T>(a, n, v);
+  else return bsearch_asc<T>(a, n, v);
+}
+
 // get_rzone_grid / RadialGrid::calculate_radial_grid (relutility.c:265-308, IonGradient.cpp:457-492),
 // one warp: every lane computes its own edges (the same formula per edge as the serial loop)
 __device__ void zone_grid_warp(double rmin, double rmax, int nz, double h, double *rg) {
@@ -294,24 +318,25 @@ __device__ double rebin_mean_at(const double *x0, const float *y0, int n0, doubl
 // returning radiation (Relreturn_Table.cpp:393-611, Relreturn_Corona.cpp:37-321)
 // ---------------------------------------------------------------------------
 
-// get_rrad_fractions for the set, serial part (thread 0): spin index (the first table spin >= a),
+// get_rrad_fractions for the set, serial part (warp 0): spin index (the first table spin >= a),
 // the table bins covering [rin, rout] and the ring-area corrections of the end bins, whose first
-// and last bin are reset to rin and rout.  rin, rout: the ends of the fine radial grid
+// and last bin are reset to rin and rout (lane 0 has the status).  rin, rout: the ends of the fine radial grid
 // (determine_rlo_rhi).
 __device__ int rrad_bins(const RelxTables &tab, RradSmem &q, double a, double rms, double rin, double rout) {
   const int NR = RELX_RR_NR;
-  int k = bsearch_asc<double>(tab.rr_spin, tab.rr_nspin, a);
+  int k = bsearch_asc_warp<double>(tab.rr_spin, tab.rr_nspin, a);
   if (tab.rr_spin[k] < a) k++;
   if (k >= tab.rr_nspin || k < 0) return RELX_ERR_TABLE;
   const double *rlo = tab.rr_rlo + (size_t) k * NR, *rhi = tab.rr_rhi + (size_t) k * NR;
-  int klo = bsearch_asc<double>(rlo, NR, rin);
-  int khi = bsearch_asc<double>(rhi, NR, rout);
+  int klo = bsearch_asc_warp<double>(rlo, NR, rin);
+  int khi = bsearch_asc_warp<double>(rhi, NR, rout);
   if (fabs(rout - rhi[NR - 1]) < 1e-6) khi = NR - 1;
   else khi++;
   if (fabs(rin - rlo[0]) < 1e-6) klo = 0;
   const int n = (khi + 1) - klo;
   // the reference asserts these (Relreturn_Table.cpp:455-456, 480; Rellp.cpp:150-151)
   if (n < 2 || n > NR || !(rin >= rlo[klo] - 1e-4)) return RELX_ERR_GRID;
+  if ((threadIdx.x & 31) != 0) return RELX_OK;  // the rest is FP64 on one lane
   q.n = n;
   q.klo = klo;
   q.spin = k;
@@ -378,12 +403,13 @@ __device__ __forceinline__ float rrad_corrected_boost_over_g(float cg, float2 ab
 // samples of frac_g times g^(gamma-1), or the corrected boost / g where the emitting bin's
 // g-shift correction differs from 1 by more than 1e-3.  One warp per incident bin, lanes over
 // the emitting bins, FP32, a fixed reduction order.
+template <int NT>
 __device__ void rrad_pass(const RelxTables &tab, RradSmem &q, float gamma, bool corr) {
   const int NR = RELX_RR_NR, NG = RELX_RR_NG;
   const int n = q.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double *tfr = tab.rr_tfr + (size_t) q.spin * NR * NR;
   const float4 *gt = tab.rr_g + (size_t) q.spin * NR * NR * NG;
-  for (int i = warp; i < n; i += kSetupThreads / 32) {
+  for (int i = warp; i < n; i += NT / 32) {
     const int ro = q.klo + i;
     float acc = 0.0f;
     for (int j = lane; j < n; j += 32) {
@@ -436,10 +462,16 @@ __device__ void zone_ionisation(SetupSmem &m, const RelxSetState &s, int z) {
   else if (m.zlxi[z] > 4.7) m.zlxi[z] = 4.7;
 }
 
-__global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab, int model, const RelxSetIn *__restrict__ sin,
-                                                               const double *__restrict__ user_e, double *__restrict__ line_e,
-                                                               RelxSetState *__restrict__ sout, RelxRadial *__restrict__ rout,
-                                                               RelxCorners *__restrict__ cout, RelxZoneCorners *__restrict__ zcout) {
+// NT: threads of the CTA.  The block sums keep the order of 256 threads in either (kSetupThreads).
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(RelxTables tab, int model,
+                                                                                const RelxSetIn *__restrict__ sin,
+                                                                                const double *__restrict__ user_e,
+                                                                                double *__restrict__ line_e,
+                                                                                RelxSetState *__restrict__ sout,
+                                                                                RelxRadial *__restrict__ rout,
+                                                                                RelxCorners *__restrict__ cout,
+                                                                                RelxZoneCorners *__restrict__ zcout) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SetupSmem &m = *reinterpret_cast<SetupSmem *>(smem_raw);
   RelxSetState &s = m.s;
@@ -453,7 +485,8 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     map_params(model, in, m);
     m.status = s.status;
   }
-  for (int z = tid; z < RELX_NZMAX; z += kSetupThreads) { m.zlo[z] = 1 << 30; m.zhi[z] = -1; }
+  for (int i = tid; i < min(kStageVals, tab.x_npar * tab.x_maxvals); i += NT) m.xvals[i] = tab.x_vals[i];
+  for (int z = tid; z < RELX_NZMAX; z += NT) { m.zlo[z] = 1 << 30; m.zhi[z] = -1; }
   __syncthreads();
   if (m.status != RELX_OK) {
     if (tid == 0) { s.win_lo = 0; s.win_hi = 0; s.nz = 0; sout[set] = s; }
@@ -467,7 +500,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     const double *ue = user_e + in.e_off;
     double *le = line_e + in.e_off;
     gn = in.n_ener;
-    for (int j = tid; j <= gn; j += kSetupThreads) {
+    for (int j = tid; j <= gn; j += NT) {
       double e = ue[j];
       if (s.z > 0) e *= (1 + s.z);       // shift_energy_grid_redshift, XspecSpectrum.h:70-76
       le[j] = e / s.lineE;               // shift_energy_grid_1keV, XspecSpectrum.h:61-65
@@ -480,16 +513,21 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
 
   // ---- relline table in the (a, mu0) plane on the table radii (Relprofile.cpp:159-223)
   const int nr = tab.rel_nr, nm = tab.rel_nmu0;
-  if (tid == 32) {  // warp 1, beside warp 0's zone grid
-    double mu0 = cos(s.incl);
-    const float af = d2f(s.a), muf = d2f(mu0);
-    int ia = bsearch_asc<float>(tab.rel_a, tab.rel_na, af);
-    int im = bsearch_asc<float>(tab.rel_mu0, nm, muf);
-    s.ind_a = ia;
-    s.ind_mu0 = im;
-    s.ifac_a = (af - tab.rel_a[ia]) / (tab.rel_a[ia + 1] - tab.rel_a[ia]);
-    s.ifac_mu0 = (muf - tab.rel_mu0[im]) / (tab.rel_mu0[im + 1] - tab.rel_mu0[im]);
-    s.g_n = gn;
+  constexpr int kLanes = NT != kSetupThreads ? 32 : 1;  // lanes of a search (bsearch_asc_nt)
+  if (tid >= 32 && tid < 32 + kLanes) {  // warp 1
+    float muf = 0.0f;
+    if (tid == 32) muf = d2f(cos(s.incl));  // FP64 on one lane: 32 lanes hold the FP64 pipe 16 times as long
+    if constexpr (kLanes == 32) muf = __shfl_sync(0xffffffffu, muf, 0);
+    const float af = d2f(s.a);
+    const int ia = bsearch_asc_nt<NT, float>(tab.rel_a, tab.rel_na, af);
+    const int im = bsearch_asc_nt<NT, float>(tab.rel_mu0, nm, muf);
+    if (tid == 32) {
+      s.ind_a = ia;
+      s.ind_mu0 = im;
+      s.ifac_a = (af - tab.rel_a[ia]) / (tab.rel_a[ia + 1] - tab.rel_a[ia]);
+      s.ifac_mu0 = (muf - tab.rel_mu0[im]) / (tab.rel_mu0[im + 1] - tab.rel_mu0[im]);
+      s.g_n = gn;
+    }
   }
   if (tid == 96) {  // warp 3: the set's FP64 constants of the per-radius loops, computed once
     m.fg_r1 = 1.0 / sqrt(s.rout);
@@ -519,11 +557,49 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     }
   }
   if (tid == 64) m.ginf_pow = pow(s.g_inf, s.gam);
+  // the lamp-post brackets (interpol_lptable, Rellp.cpp:190-247) of spin bracket q, by kLanes lanes of a warp
+  auto lp_brackets = [&](int q) {
+    const float fa = d2f(s.a), fh = d2f(s.height);
+    const int ia = bsearch_asc_nt<NT, float>(tab.lp_a, tab.lp_na, fa);
+    const float *hg = tab.lp_h + (size_t) (ia + q) * tab.lp_nh;
+    const int ih = bsearch_asc_nt<NT, float>(hg, tab.lp_nh, fh);
+    if ((tid & 31) == 0) {
+      m.ind_h[q] = ih;
+      m.ifac_h[q] = (fh - hg[ih]) / (hg[ih + 1] - hg[ih]);
+      if (q == 0) {
+        m.lp_ind_a = ia;
+        m.lp_ifac_a = (fa - tab.lp_a[ia]) / (tab.lp_a[ia + 1] - tab.lp_a[ia]);
+      }
+    }
+  };
+  // conv-grid bins the final rebin to the caller's grid reads (Relxill.cpp:267-278, Relbase.cpp:281-284)
+  auto conv_range = [&]() {
+    const double *ue = user_e + in.e_off;
+    double zf = (kind != RELX_RELCONV && s.z > 0) ? (1 + s.z) : 1.0;
+    double elo = ue[0] * zf, ehi = ue[in.n_ener] * zf;
+    const double *ce = tab.conv_e;
+    int lo = conv_index(tab, elo);  // as bsearch_asc over the N + 1 edges
+    int hi = conv_index(tab, ehi);
+    if (in.flags & 2) {  // RELXILL_RENORMALIZE reads the bin at 3 keV
+      int k3 = bsearch_asc<double>(ce, RELX_NCONV, 3.0);
+      lo = min(lo, k3);
+      hi = max(hi, k3);
+    }
+    s.out_lo = max(0, lo - 1);
+    s.out_hi = min(RELX_NCONV - 1, hi + 1);
+  };
+  // 1024 threads: warps beyond the table interpolation's; 256 threads: later, where other CTAs of the SM
+  // cover their latency (here they would hold two of the eight warps back: 0.78 -> 0.85 ms for 4096 sets)
+  if constexpr (NT != kSetupThreads) {
+    const int w = (tid >> 5) - 8;
+    if ((w == 0 || w == 1) && s.emis_type == RELX_EMIS_LP) lp_brackets(w);
+    if (tid == 320 && kind != RELX_RELLINE) conv_range();
+  }
   {
     const size_t b00 = (size_t) s.ind_a * nm + s.ind_mu0, b10 = (size_t) (s.ind_a + 1) * nm + s.ind_mu0;
     const size_t b01 = b00 + 1, b11 = b10 + 1;
     const double fa = f2d(s.ifac_a), fm = f2d(s.ifac_mu0);
-    for (int i = tid; i < nr; i += kSetupThreads) {
+    for (int i = tid; i < nr; i += NT) {
       // the float table values widened on the integer pipes (f2d is exact)
       m.re_tab[i] = lerp1(fa, f2d(tab.rel_r[b00 * nr + i]), f2d(tab.rel_r[b10 * nr + i]));
       m.gmin_t[i] = lerp2(fa, fm, f2d(tab.rel_gmin[b00 * nr + i]), f2d(tab.rel_gmin[b10 * nr + i]),
@@ -535,7 +611,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   // fine radial grid (relutility.c:666-677)
   {
     const double r1 = m.fg_r1, du = m.fg_du;  // 1/sqrt(rout) and the step in u
-    for (int ii = tid; ii < NR; ii += kSetupThreads) {
+    for (int ii = tid; ii < NR; ii += NT) {
       double u = f2d((float) ii) * du + r1;  // ii < 2^24: exact
       // 1/u: the float reciprocal refined by two Newton steps in FP64 (within an ulp of the
       // correctly rounded quotient)
@@ -556,7 +632,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     if (m.re_tab[m.ind_rmax] < 1000.0 && m.re_tab[m.ind_rmax] * 1.01 > 1000.0) m.re_tab[m.ind_rmax] = 1000.0;
   }
   __syncthreads();
-  for (int i = tid; i < nr - 1; i += kSetupThreads) {
+  for (int i = tid; i < nr - 1; i += NT) {
     m.inv_dtab[i] = 1.0 / (m.re_tab[i] - m.re_tab[i + 1]);
     m.dgmin_t[i] = m.gmin_t[i] - m.gmin_t[i + 1];  // the interpolation below as lo + f (hi - lo)
     m.dgmax_t[i] = m.gmax_t[i] - m.gmax_t[i + 1];
@@ -572,7 +648,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   int my_lo = 1 << 30, my_hi = -1;
   const double ge0 = ge[0], gen = ge[gn];
   const float wt_c = (float) (kPi / 2);
-  for (int ii = tid; ii < NR; ii += kSetupThreads) {
+  for (int ii = tid; ii < NR; ii += NT) {
     const double r = m.re[ii];
     // index ind with re_tab[ind+1] <= r < re_tab[ind], as the walk of Relprofile.cpp:252-266
     const int lo = count_gt_desc_pos(m.re_tab, nr, r);  // count of table radii > r
@@ -633,13 +709,13 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     rr.iehi = iehi;
     R.rec[ii] = rr;
   }
-  int wlo = block_min_i<kSetupThreads>(my_lo, m.ired);
-  int whi = block_max_i<kSetupThreads>(my_hi, m.ired);
+  int wlo = block_min_i<NT>(my_lo, m.ired);
+  int whi = block_max_i<NT>(my_hi, m.ired);
   if (tid == 0) {
     s.win_lo = (whi >= 0) ? wlo : 0;
     s.win_hi = (whi >= 0) ? whi + 1 : 0;
   }
-  for (int z = tid; z < s.nz; z += kSetupThreads) {
+  for (int z = tid; z < s.nz; z += NT) {
     // profile bins outside a zone's window stay exactly zero
     s.zw_lo[z] = (m.zhi[z] >= 0) ? m.zlo[z] : s.win_lo;
     s.zw_hi[z] = (m.zhi[z] >= 0) ? m.zhi[z] + 1 : s.win_lo;
@@ -653,40 +729,39 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     const float inv_rbr = m.inv_rbr;
     const float a1 = d2f(-m.emis1), a2 = d2f(-m.emis2);
     float2 part = make_float2(0.0f, 0.0f);
-    for (int ii = tid; ii < NR; ii += kSetupThreads) {
+    for (int ii = tid; ii < NR; ii += NT) {
       const double r = m.re[ii];
       const float e = powf(d2f(r) * inv_rbr, dgt(r, m.rbr) ? a2 : a1);
       m.pr.emis[ii] = e;
       m.pr.del_emit[ii] = -1.0f;
       m.pr.del_inc[ii] = -1.0f;
-      part = ff_add(part, ff_mulf(make_float2(e, 0.0f), 4.0f * R.wt[ii]));
+      if constexpr (NT == kSetupThreads) part = ff_add(part, ff_mulf(make_float2(e, 0.0f), 4.0f * R.wt[ii]));
+    }
+    if constexpr (NT != kSetupThreads) {
+      __syncthreads();
+      if (tid < kSetupThreads)
+        for (int ii = tid; ii < NR; ii += kSetupThreads)
+          part = ff_add(part, ff_mulf(make_float2(m.pr.emis[ii], 0.0f), 4.0f * R.wt[ii]));
     }
     const double inv_integ = 1.0 / block_sum_d<kSetupThreads>(ff_to_double(part), m.red);
-    for (int ii = tid; ii < NR; ii += kSetupThreads) m.pr.emis[ii] = d2f(f2d(m.pr.emis[ii]) * inv_integ);
+    for (int ii = tid; ii < NR; ii += NT) m.pr.emis[ii] = d2f(f2d(m.pr.emis[ii]) * inv_integ);
     __syncthreads();
     if (tid == 0) { s.f_inf_rest = 0; s.refl_frac_lp = 0; }
   } else {
     // lamp post: interpol_lptable (Rellp.cpp:190-247)
     const int nh = tab.lp_nh, nrad = tab.lp_nrad;
-    if (tid == 0) {
-      float fa = d2f(s.a);
-      int ia = bsearch_asc<float>(tab.lp_a, tab.lp_na, fa);
-      m.lp_ind_a = ia;
-      m.lp_ifac_a = (fa - tab.lp_a[ia]) / (tab.lp_a[ia + 1] - tab.lp_a[ia]);
-      float fh = d2f(s.height);
-      for (int q = 0; q < 2; q++) {
-        const float *hg = tab.lp_h + (size_t) (ia + q) * nh;
-        int ih = bsearch_asc<float>(hg, nh, fh);
-        m.ind_h[q] = ih;
-        m.ifac_h[q] = (fh - hg[ih]) / (hg[ih + 1] - hg[ih]);
+    if constexpr (NT == kSetupThreads) {
+      if (tid == 0) {
+        lp_brackets(0);
+        lp_brackets(1);
       }
+      __syncthreads();
     }
-    __syncthreads();
     {
       const int ia = m.lp_ind_a;
       const double fa = m.lp_ifac_a;
       const float faf = d2f(fa), f0f = d2f(m.ifac_h[0]), f1f = d2f(m.ifac_h[1]);
-      for (int k = tid; k < nrad; k += kSetupThreads) {
+      for (int k = tid; k < nrad; k += NT) {
         m.jet_rad[k] = lerp1(fa, f2d(tab.lp_rad[(size_t) ia * nrad + k]), f2d(tab.lp_rad[(size_t) (ia + 1) * nrad + k]));
 #define TV(arr, q, h) (arr)[(((size_t) (ia + (q)) * nh) + (h)) * nrad + k]
         const int h0 = m.ind_h[0], h1 = m.ind_h[1];
@@ -703,7 +778,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
       }
     }
     __syncthreads();
-    for (int k = tid; k < nrad; k += kSetupThreads) {
+    for (int k = tid; k < nrad; k += NT) {
       if (k < nrad - 1) {
         const float djr = d2f(m.jet_rad[k + 1] - m.jet_rad[k]);
         m.inv_drad_f[k] = 1.0f / djr;
@@ -725,7 +800,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     const bool moving = fabs(s.beta) >= 1e-6, boosted = s.beta > 1e-6;
     const float gam_f = d2f(s.gamma);
     const double jr_last = m.jet_rad[nrad - 1];
-    for (int ii = tid; ii < NR; ii += kSetupThreads) {
+    for (int ii = tid; ii < NR; ii += NT) {
       const double r = m.re[ii], sr = m.sqre[ii];
       const int kk = bsearch_asc_pos(m.jet_rad, nrad, r);
       if (dge(r, jr_last) && r - RELX_RELTABLE_MAX_R > 1e-6) atomicExch(&m.status, RELX_ERR_GRID);
@@ -754,7 +829,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
       m.pr.emis[ii] = m.lp_e[kk] * expf(inter * m.lp_dle[kk]) * boost;
     }
     __syncthreads();
-    if (tid >= kSetupThreads - 32) {
+    if (tid >= NT - 32) {
       // calc_refl_frac (Rellp.cpp:36-89) on the last warp, which joins the next loops after it (its
       // results are read at the end); the three cosines on three lanes
       double ad_max = m.d_tab[nrad - 1];
@@ -783,55 +858,41 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   // ---- returning radiation without xillver corrections (calc_emis_profile, Rellp.cpp:556-558)
   const bool rrad = m.return_rad != 0 && m.status == RELX_OK;
   if (rrad) {
-    if (tid == 0) {
+    if (tid < 32) {
       const int e = (tab.rr_nspin > 0) ? rrad_bins(tab, m.rt.rr, s.a, m.rms, m.re[NR - 1], m.re[0]) : RELX_ERR_TABLE;
-      if (e != RELX_OK) m.status = e;
+      if (e != RELX_OK && tid == 0) m.status = e;
     }
     __syncthreads();
-    if (m.status == RELX_OK) rrad_centres(tab, m.rt.rr, m.re[NR - 1], m.re[0], kSetupThreads);
+    if (m.status == RELX_OK) rrad_centres(tab, m.rt.rr, m.re[NR - 1], m.re[0], NT);
   }
   if (rrad && m.status == RELX_OK) {
     RradSmem &q = m.rt.rr;
-    for (int j = tid; j < q.n; j += kSetupThreads) q.emis_in[j] = d2f(rebin_mean_at(m.re, m.pr.emis, NR, q.rad[j]));
+    for (int j = tid; j < q.n; j += NT) q.emis_in[j] = d2f(rebin_mean_at(m.re, m.pr.emis, NR, q.rad[j]));
     __syncthreads();
-    rrad_pass(tab, q, d2f(s.gamma), false);
+    rrad_pass<NT>(tab, q, d2f(s.gamma), false);
     __syncthreads();
-    for (int k = tid; k + 1 < q.n; k += kSetupThreads) q.dl[k] = log2f(q.er[k + 1] / q.er[k]);
+    for (int k = tid; k + 1 < q.n; k += NT) q.dl[k] = log2f(q.er[k + 1] / q.er[k]);
     __syncthreads();
-    for (int ii = tid; ii < NR; ii += kSetupThreads) {
+    for (int ii = tid; ii < NR; ii += NT) {
       m.rt.emis_lp[ii] = m.pr.emis[ii];
       const double r = rrad_at(q, m.re[ii]);
       m.pr.emis[ii] = d2f((m.return_rad == 1) ? f2d(m.pr.emis[ii]) + r : r);
     }
     __syncthreads();
   }
-  for (int ii = tid; ii < NR; ii += kSetupThreads) R.rec[ii].ew = m.pr.emis[ii] * R.wt[ii];
+  for (int ii = tid; ii < NR; ii += NT) R.rec[ii].ew = m.pr.emis[ii] * R.wt[ii];
 
   // ---- zones: fine-radius index ranges (zone is non-increasing with the radius index)
-  for (int z = tid; z < s.nz; z += kSetupThreads) { s.zi0[z] = 1; s.zi1[z] = 0; }
+  for (int z = tid; z < s.nz; z += NT) { s.zi0[z] = 1; s.zi1[z] = 0; }
   __syncthreads();
-  for (int ii = tid; ii < NR; ii += kSetupThreads) {
+  for (int ii = tid; ii < NR; ii += NT) {
     const int z = R.rec[ii].zone;
     if (ii == 0 || R.rec[ii - 1].zone != z) s.zi0[z] = ii;
     if (ii == NR - 1 || R.rec[ii + 1].zone != z) s.zi1[z] = ii;
   }
   __syncthreads();
-  // conv-grid bins the final rebin to the caller's grid reads (Relxill.cpp:267-278, Relbase.cpp:281-284)
-  if (tid == 0 && kind != RELX_RELLINE) {
-    const double *ue = user_e + in.e_off;
-    double zf = (kind != RELX_RELCONV && s.z > 0) ? (1 + s.z) : 1.0;
-    double elo = ue[0] * zf, ehi = ue[in.n_ener] * zf;
-    const double *ce = tab.conv_e;
-    int lo = conv_index(tab, elo);  // as bsearch_asc over the N + 1 edges
-    int hi = conv_index(tab, ehi);
-    if (in.flags & 2) {  // RELXILL_RENORMALIZE reads the bin at 3 keV
-      int k3 = bsearch_asc<double>(ce, RELX_NCONV, 3.0);
-      lo = min(lo, k3);
-      hi = max(hi, k3);
-    }
-    s.out_lo = max(0, lo - 1);
-    s.out_hi = min(RELX_NCONV - 1, hi + 1);
-  }
+  if constexpr (NT == kSetupThreads)
+    if (tid == 0 && kind != RELX_RELLINE) conv_range();
   if (!m.is_relxill) {
     __syncthreads();
     if (tid == 0) {
@@ -873,6 +934,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
 
   // ---- xillver brackets and factors per zone (xilltable.c:278-323, 1090-1142)
   const int npar = tab.x_npar;
+  const bool staged_vals = npar * tab.x_maxvals <= kStageVals;
   if (tid < nz) {
     int z = tid;
     double ect_z = s.ect_src * m.shift[z];
@@ -885,7 +947,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     inp[4] = d2f(m.zdens[z]);
     inp[7] = (float) (s.incl * 180 / kPi);
     for (int q = 0; q < npar; q++) {
-      const float *pv = tab.x_vals + q * tab.x_maxvals;
+      const float *pv = (staged_vals ? m.xvals : tab.x_vals) + q * tab.x_maxvals;
       int nv = tab.x_nvals[q];
       int pi = tab.x_pindex[q];
       int ind = bsearch_asc<float>(pv, nv, inp[pi]);
@@ -909,36 +971,39 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   // per continuum (source, then every zone), float-float sums of FP32 terms times the bin centre
   // The nthcomp continuum of the Cp models is normalised by nthcomp_kernel after this kernel
   // (nthcomp.cu), which also applies the zones' normalisation changes to their corner weights.
-  for (int z = tid; z < nz; z += kSetupThreads) s.zshift[z] = m.shift[z];
+  for (int z = tid; z < nz; z += NT) s.zshift[z] = m.shift[z];
   if (s.prim == 1) {
     if (tid == 0) s.src_norm = 0.0;
-    for (int z = tid; z < nz; z += kSetupThreads) m.xscale[z] = 1.0;
+    for (int z = tid; z < nz; z += NT) m.xscale[z] = 1.0;
   } else {
     const float gam = d2f(s.gam);
     const int lane = tid & 31, warp = tid >> 5;
-    for (int b = tid; b < RELX_NCOARSE; b += kSetupThreads) m.cpow[b] = powf(tab.coarse_t[b].x, -gam);
-    for (int qq = tid; qq <= nz; qq += kSetupThreads) m.qecut[qq] = d2f(s.ect_src * (qq == 0 ? 1.0 : m.shift[qq - 1]));
+    for (int b = tid; b < RELX_NCOARSE; b += NT) m.cpow[b] = powf(tab.coarse_t[b].x, -gam);
+    for (int qq = tid; qq <= nz; qq += NT) m.qecut[qq] = d2f(s.ect_src * (qq == 0 ? 1.0 : m.shift[qq - 1]));
     __syncthreads();
     // the continua (the source, then the zones) in groups of kQGroup over the whole block: every
     // thread sums the terms of its coarse bins for each continuum of the group (independent sums),
     // the warps reduce with shuffles and one thread per continuum adds the warps' sums in warp order;
     // float-float sums of FP32 terms (calcNormWrtXillverTableSpec, Xillspec.cpp:179-233)
-    for (int q0 = 0; q0 <= nz; q0 += kQGroup) {
-      const int nq = min(kQGroup, nz + 1 - q0);
+    constexpr int kTeams = NT / kSetupThreads;  // 256 threads per group
+    const int team = tid / kSetupThreads, ttid = tid % kSetupThreads;
+    for (int q00 = 0; q00 <= nz; q00 += kTeams * kQGroup) {
+      const int q0 = q00 + team * kQGroup;
+      const int nq = max(0, min(kQGroup, nz + 1 - q0));
       float2 part[kQGroup];
       float ecut[kQGroup], e0[kQGroup];
 #pragma unroll
       for (int k = 0; k < kQGroup; k++) {
         part[k] = make_float2(0.0f, 0.0f);
-        ecut[k] = m.qecut[q0 + min(k, nq - 1)];
+        ecut[k] = m.qecut[nq > 0 ? q0 + min(k, nq - 1) : 0];
         e0[k] = expf(1.0f / ecut[k]);
       }
-      for (int b = tid; b < RELX_NCOARSE; b += kSetupThreads) {
+      for (int b = ttid; b < RELX_NCOARSE && nq > 0; b += kSetupThreads) {
         const float4 t = tab.coarse_t[b];  // bin centre, width, centre as float-float (0 outside the band)
         const float pw = m.cpow[b];
 #pragma unroll
         for (int k = 0; k < kQGroup; k++) {
-          if (k < nq) {  // uniform over the block
+          if (k < nq) {  // uniform over the 256 threads
             const float term = e0[k] * pw * expf(-t.x / ecut[k]) * t.y;
             part[k] = ff_add(part[k], ff_mulf(make_float2(t.z, t.w), term));
           }
@@ -956,10 +1021,11 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
         if (lane == 0) m.qpart[warp][k] = part[k];
       }
       __syncthreads();
-      if (tid < nq) {
-        float2 a = m.qpart[0][tid];
-        for (int w = 1; w < kSetupThreads / 32; w++) a = ff_add(a, m.qpart[w][tid]);
-        m.qsum[q0 + tid] = (f2d(a.x) + f2d(a.y)) * kQsumScale;
+      if (ttid < nq) {
+        constexpr int kW = kSetupThreads / 32;
+        float2 a = m.qpart[team * kW][ttid];
+        for (int w = 1; w < kW; w++) a = ff_add(a, m.qpart[team * kW + w][ttid]);
+        m.qsum[q0 + ttid] = (f2d(a.x) + f2d(a.y)) * kQsumScale;
       }
       __syncthreads();
     }
@@ -981,7 +1047,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   if (six && !tab.x_has_dens && tid == 0) m.status = RELX_ERR_TABLE;
   const bool listed = nz * ncz <= RELX_NZMAX * 16;  // the entries fit the de-duplication arrays
   if (!listed) {  // 6-parameter table and more than 25 zones: per-zone lists, no de-duplication
-    for (int e = tid; e < nz * 32; e += kSetupThreads) {
+    for (int e = tid; e < nz * 32; e += NT) {
       const int z = e >> 5, c = e & 31;
       long row = 0;
       double w = 1.0;
@@ -1001,7 +1067,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   }
   // ---- the corners of every zone, first-zone density scaling, de-duplication
   const int ncor = listed ? nz * ncz : 0;
-  for (int e = tid; e < ncor; e += kSetupThreads) {
+  for (int e = tid; e < ncor; e += NT) {
     const int z = e / ncz, c = e - z * ncz;
     // corner c: bit q -> upper bracket of parameter q
     long row = 0;
@@ -1010,14 +1076,14 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     m.cr.crow[e] = (int) row;
   }
   __syncthreads();
-  for (int e = tid; e < ncor; e += kSetupThreads) {
+  for (int e = tid; e < ncor; e += NT) {
     int first = e;
     for (int f = 0; f < e; f++)
       if (m.cr.crow[f] == m.cr.crow[e]) { first = f; break; }
     m.cr.cfirst[e] = (short) first;
   }
   __syncthreads();
-  for (int e = tid; e < ncor; e += kSetupThreads) {
+  for (int e = tid; e < ncor; e += NT) {
     const int z = e / ncz, c = e - z * ncz;
     double w = 1.0;
     for (int q = 0; q < nbits; q++) {
@@ -1036,7 +1102,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   __syncthreads();
   // a row is read only if some zone gives it a non-zero weight (a parameter on a grid value
   // puts exactly zero weight on the upper bracket)
-  for (int e = tid; e < ncor; e += kSetupThreads)
+  for (int e = tid; e < ncor; e += NT)
     if (m.cr.cw[e] != 0.0f) m.cr.clive[m.cr.cfirst[e]] = 1;
   __syncthreads();
   if (tid < 32 && listed) {  // number the live rows in entry order (warp prefix sums)
@@ -1056,7 +1122,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     }
   }
   __syncthreads();
-  for (int e = tid; e < ncor; e += kSetupThreads)
+  for (int e = tid; e < ncor; e += NT)
     if (m.cr.cfirst[e] != e) m.cr.cuniq[e] = m.cr.cuniq[m.cr.cfirst[e]];  // the first entry is numbered above
   // dense: at most RELX_ZDENSE zones and RELX_MAX_UCORNER distinct live rows (always so for the
   // 5-parameter table: 16 corners x 16 zones)
@@ -1065,10 +1131,10 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
   if (tid == 0 && listed) s.xdense = dense ? 1 : 0;
   if (dense) {
     RelxCorners &C = cout[set];
-    for (int i = tid; i < RELX_MAX_UCORNER * RELX_ZDENSE; i += kSetupThreads) (&C.w[0][0])[i] = 0.0f;
+    for (int i = tid; i < RELX_MAX_UCORNER * RELX_ZDENSE; i += NT) (&C.w[0][0])[i] = 0.0f;
     __syncthreads();
   }
-  for (int e = tid; e < ncor; e += kSetupThreads) {
+  for (int e = tid; e < ncor; e += NT) {
     const int z = e / ncz, c = e - z * ncz;
     if (dense) {
       RelxCorners &C = cout[set];
@@ -1093,7 +1159,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
     const int nq = tab.x_npar - 1, ncorner = 1 << nq;  // parameters bracketed per corner (<= 5)
     const int lane = tid & 31, warp = tid >> 5;
     const float p15 = powf(1.5f, d2f(s.gam));
-    for (int z = warp; z < nz; z += kSetupThreads / 32) {
+    for (int z = warp; z < nz; z += NT / 32) {
       double ef = 0.0, pf = 0.0, pfz = 0.0;
       if (lane < ncorner) {
         const int c = lane;
@@ -1147,7 +1213,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
       }
     }
     __syncthreads();
-    for (int k = tid; k < q.n; k += kSetupThreads) {  // rebin_to_grid (Relreturn_Corona.cpp:208-222)
+    for (int k = tid; k < q.n; k += NT) {  // rebin_to_grid (Relreturn_Corona.cpp:208-222)
       int zi = bsearch_asc_pos(s.rgrid, nz + 1, q.rad[k]);
       if (q.rad[k] < s.rgrid[0]) zi = 0;
       else if (q.rad[k] > s.rgrid[nz]) zi = nz - 1;
@@ -1156,11 +1222,11 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
       q.use_corr[k] = fabs(q.zcf_g[zi] - 1) > 1e-3;
     }
     __syncthreads();
-    rrad_pass(tab, q, d2f(s.gamma), true);
+    rrad_pass<NT>(tab, q, d2f(s.gamma), true);
     __syncthreads();
-    for (int k = tid; k + 1 < q.n; k += kSetupThreads) q.dl[k] = log2f(q.er[k + 1] / q.er[k]);
+    for (int k = tid; k + 1 < q.n; k += NT) q.dl[k] = log2f(q.er[k + 1] / q.er[k]);
     __syncthreads();
-    for (int ii = tid; ii < NR; ii += kSetupThreads) {
+    for (int ii = tid; ii < NR; ii += NT) {
       const double r = rrad_at(q, m.re[ii]);
       const double e = (m.return_rad == 1) ? f2d(m.rt.emis_lp[ii]) + r : r;
       R.rec[ii].ew = d2f(e) * R.wt[ii];
@@ -1183,18 +1249,43 @@ __global__ void __launch_bounds__(kSetupThreads, 4) setup_kernel(RelxTables tab,
       s.prim_fac = pf;
       s.norm_fac_refl = fabs(rfi) / s.refl_frac_lp;
     }
-    for (int z = 0; z < nz; z++) s.inv_nc[z] = d2f(m.xscale[z]);
     if (m.status != RELX_OK) s.status = m.status;
   }
+  for (int z = tid; z < nz; z += NT) s.inv_nc[z] = d2f(m.xscale[z]);
   __syncthreads();
   {  // the set state out, by all threads
     static_assert(sizeof(RelxSetState) % 8 == 0, "copied as 8-byte words");
     const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&s);
     unsigned long long *dst = reinterpret_cast<unsigned long long *>(&sout[set]);
-    for (int i = tid; i < (int) (sizeof(RelxSetState) / 8); i += kSetupThreads) dst[i] = src[i];
+    for (int i = tid; i < (int) (sizeof(RelxSetState) / 8); i += NT) dst[i] = src[i];
   }
 }
 
-size_t setup_smem_bytes() { return sizeof(SetupSmem); }
+static size_t setup_smem_bytes() { return sizeof(SetupSmem); }
+
+cudaError_t setup_set_smem() {
+  cudaError_t e;
+  const int bytes = (int) setup_smem_bytes();
+  if ((e = cudaFuncSetAttribute(setup_kernel<kSetupThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) ||
+      (e = cudaFuncSetAttribute(setup_kernel<kSetupFewThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return e;
+  // four CTAs of 256 threads per SM (54 KB each): the largest shared-memory carve-out
+  return cudaFuncSetAttribute(setup_kernel<kSetupThreads>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
+// Few sets: 1024 threads per set while every set has an SM of its own (then four CTAs of 256 threads per SM,
+// which cover each other's serial FP64 chains).  us with 1024 / 256 threads: 1 relxilllp set 58 / 76, 152 sets
+// 78 / 92, 192 138 / 93; with returning radiation 1 set 103 / 186, 152 sets 133 / 226.
+cudaError_t launch_setup(cudaStream_t s, int n_sets, const RelxTables &tab, int model, const RelxSetIn *sin,
+                         const double *user_e, double *line_e, RelxSetState *sout, RelxRadial *rout,
+                         RelxCorners *cout, RelxZoneCorners *zcout) {
+  if (n_sets <= 152)
+    setup_kernel<kSetupFewThreads><<<n_sets, kSetupFewThreads, setup_smem_bytes(), s>>>(tab, model, sin, user_e, line_e,
+                                                                                       sout, rout, cout, zcout);
+  else
+    setup_kernel<kSetupThreads><<<n_sets, kSetupThreads, setup_smem_bytes(), s>>>(tab, model, sin, user_e, line_e, sout,
+                                                                                 rout, cout, zcout);
+  return cudaGetLastError();
+}
 
 }  // namespace relx
