@@ -12,7 +12,9 @@
 // FP32 FFT (absolute error ~1e-7 of the peak) would not.
 //
 // conv_zone_kernel: one CTA per (zone, set), 256 threads x 16 output bins,
-// register-tiled (16 x 16 products per 47 shared-memory loads).
+// register-tiled (16 x 16 products per 12 16-byte shared-memory loads); bound by issue (2.8 instructions per
+// clock and SM): a third of the time for the products, a fifth for the normalisation.  Not kept: all zones of
+// a set by one CTA, summed on the way (2000 sets 519 us against 490), packed FP32 pairs (1217 us against 1168).
 #include "relx_device.cuh"
 #include "relx_kernels.h"
 #include "relx_tma.cuh"
@@ -24,46 +26,46 @@ constexpr int kFinThreads = 128;   // finalize kernels
 constexpr int kConvR = 16;         // output bins per thread and work item
 constexpr int kConvD = 16;         // window bins per step of the register tile
 constexpr int kN = RELX_NCONV;
-constexpr int kPre = 4;            // prefix sums are kept at every kPre-th bin
-constexpr int kXStage = 3072;      // xillver bins staged in shared memory (larger tables read global memory)
-static_assert(kN % (kConvThreads * kPre) == 0, "scan tiling");
+constexpr int kConvWarps = kConvThreads / 32;
+static_assert(kConvWarps == 8, "the warps' sums are added by groups of 8 lanes");
 
-// xs is stored in rows of 16 bins, each followed by 4 padding floats: the 16-byte loads of the
-// threads of a quarter warp (16 bins apart) then fall in distinct banks
-__device__ __forceinline__ int skew(int m) { return m + ((m >> 4) << 2); }
+// xs is stored in rows of 16 bins, each followed by 4 padding floats (conv_skew): the 16-byte loads of
+// the threads of a quarter warp (16 bins apart) then fall in distinct banks
+__device__ __forceinline__ int skew(int m) { return conv_skew(m); }
 
 struct ConvSmem {
   alignas(16) float xs[kN + kN / 4];  // x * cf, skewed
   float hr[kN + kConvR];       // rel * cf over the zone's profile window, zero padded (16-byte aligned)
-  float2 red[kConvThreads / 32 + 2];
-  float2 wsum[kConvThreads / 32];
-  double dred[kConvThreads / 32 + 2];
+  float2 wsum[kConvWarps];     // the warps' sums of the profile, for its prefix sums
+  float2 wred[4 * kConvWarps]; // the warps' parts of the normalisation's sums, sum k at k * kConvWarps
+  // the convolution, in tiles of 16 bins and a padding float: threads a tile apart write distinct banks, and
+  // it is read back by neighbouring threads
+  float y[(kN / kConvR + 2) * (kConvR + 1)];
+  double dred[kConvWarps + 2];
   double zsum[RELX_NZMAX];
-  float bc[2];                 // broadcast scalars
-  float2 sxw;                  // band sum of xs
-  int abort_flag;
-  uint64_t bar;                // completion of the bulk copy of the zone's xillver spectrum
-  union {                      // the staged spectrum is read before the prefix sums are formed
-    alignas(16) float xz[kXStage];  // the zone's xillver spectrum (bulk copy)
-    float2 pre[kN / kPre + 1];   // float-float prefix sums of xs at bins 0, kPre, 2 kPre, ...
-  };
+  float bc;                    // scale of the profile
+  uint64_t bar;                // completion of the bulk copy of a zone's xillver spectrum
 };
-static_assert(offsetof(ConvSmem, hr) % 16 == 0, "the profile window is read as float4");
+static_assert(offsetof(ConvSmem, xs) % 16 == 0 && offsetof(ConvSmem, hr) % 16 == 0, "the profile window is read as float4");
 
 // y[k0 + r] = sum_{i in [clo, chi)} hr[i - wlo] * xs[(k0 + r + p - i) mod N]; hr is zero padded
 // past the window, so chi - clo need not be a multiple of kConvD.  Register tile: kConvR outputs x
-// kConvD window bins per step, (kConvR + kConvD) / 4 float4 loads of xs and kConvD/4 float4 loads
-// of hr for kConvR * kConvD FMAs.  k0 + p - clo must be a multiple of 4 (the xs loads are aligned).
+// kConvD window bins per step, two rows of xs and kConvD/4 float4 loads of hr for kConvR * kConvD FMAs.
+// k0 + p - clo is a multiple of 16: the rows' loads have fixed offsets (with tiles aligned to 4 bins the
+// positions of eight loads were as many integer instructions as a quarter of the FMAs).
 __device__ __forceinline__ void conv_tile(const ConvSmem &m, int k0, int p, int wlo, int clo, int chi,
                                           float y[kConvR]) {
+  static_assert(kConvR == 16 && kConvD == 16, "rows of xs");
 #pragma unroll
   for (int r = 0; r < kConvR; r++) y[r] = 0.0f;
-  for (int i0 = clo; i0 < chi; i0 += kConvD) {
-    const int base = k0 + p - i0 - (kConvD - 1) - 1;  // one bin lower: a multiple of 4
+  int row = (k0 + p - clo) >> 4;  // of the step's upper 16 bins
+  for (int i0 = clo; i0 < chi; i0 += kConvD, row--) {
+    const float4 *x0 = reinterpret_cast<const float4 *>(&m.xs[((row - 1) & (kN / 16 - 1)) * 20]);
+    const float4 *x1 = reinterpret_cast<const float4 *>(&m.xs[(row & (kN / 16 - 1)) * 20]);
     float xr[kConvR + kConvD];
 #pragma unroll
     for (int c4 = 0; c4 < (kConvR + kConvD) / 4; c4++) {
-      const float4 v = *reinterpret_cast<const float4 *>(&m.xs[skew((base + 4 * c4) & (kN - 1))]);
+      const float4 v = c4 < 4 ? x0[c4] : x1[c4 - 4];
       xr[4 * c4] = v.x;
       xr[4 * c4 + 1] = v.y;
       xr[4 * c4 + 2] = v.z;
@@ -109,71 +111,63 @@ __device__ __forceinline__ double zone_sum_warp(const RelxSetState &s, const dou
   return zs;
 }
 
-// relline renormalisation factor (renorm_relline_profile, Relprofile.cpp:766-781) in m.bc[0] and the
-// (scaled) profile sum of zone z in m.zsum[z].  Without renormalisation (lamp post) the other zones'
-// sums are not needed.
-__device__ void profile_sums(ConvSmem &m, const RelxSetState &s, const double *tsum, int set, int nblk, int nza,
-                             int z) {
-  const int tid = threadIdx.x, warp = tid >> 5;
-  if (s.relline_norm > 0.0) {
-    for (int q = warp; q < s.nz; q += kConvThreads / 32) {
-      const double zs = zone_sum_warp(s, tsum, set, nblk, nza, q);
-      if ((tid & 31) == 0) m.zsum[q] = zs;
-    }
-    __syncthreads();
-    if (tid == 0) {  // the zones' total in zone order, then the zone scaled
-      double sum = 0.0;
-      for (int q = 0; q < s.nz; q++) sum += m.zsum[q];
-      const double scale = s.relline_norm / sum;
-      m.bc[0] = (float) scale;
-      m.zsum[z] *= scale;
-    }
-  } else if (warp == 0) {
-    const double zs = zone_sum_warp(s, tsum, set, nblk, nza, z);
-    if (tid == 0) {
-      m.zsum[z] = zs;
-      m.bc[0] = 1.0f;
-    }
+// Profile sums of all zones (m.zsum) and the relline renormalisation factor (renorm_relline_profile,
+// Relprofile.cpp:766-781) in m.bc, by the whole block
+__device__ void profile_sums(ConvSmem &m, const RelxSetState &s, const double *tsum, int set, int nblk, int nza) {
+  const int tid = threadIdx.x;
+  for (int q = tid >> 5; q < s.nz; q += kConvWarps) {
+    const double zs = zone_sum_warp(s, tsum, set, nblk, nza, q);
+    if ((tid & 31) == 0) m.zsum[q] = zs;
+  }
+  __syncthreads();
+  if (s.relline_norm <= 0.0) return;
+  double scale = 1.0;
+  if (tid == 0) {  // the zones' total in zone order
+    double sum = 0.0;
+    for (int q = 0; q < s.nz; q++) sum += m.zsum[q];
+    scale = s.relline_norm / sum;
+    m.bc = (float) scale;
+    for (int q = 0; q < s.nz; q++) m.zsum[q] *= scale;
   }
   __syncthreads();
 }
 
-// float-float prefix of xs at bin x (0 <= x <= N)
-__device__ __forceinline__ float2 prefix_at(const ConvSmem &m, int x) {
-  const int q = x / kPre;
-  float2 v = m.pre[q];
-  for (int j = q * kPre; j < x; j++) v = ff_addf(v, m.xs[skew(j)]);
-  return v;
+__device__ __forceinline__ float2 shfl_xor_ff(float2 v, int o) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+__device__ __forceinline__ float2 shfl_ff(float2 v, int l) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
 }
 
-// cost of a split of the window into S segments: rounds of work items times segment length
-__device__ __forceinline__ int split_cost(int nt, int nc, int S) {
-  return ((nt * S + kConvThreads - 1) / kConvThreads) * ((nc + S - 1) / S);
+// steps of the longest thread for 1 << s window segments
+__device__ __forceinline__ int split_cost(int nt, int nc, int s) {
+  return (((nt << s) + kConvThreads - 1) / kConvThreads) * ((nc + (1 << s) - 1) >> s);
 }
 
-// Convolution of xs with hr, normalised as calcFFTNormFactor (Relbase.cpp:199-222), written for the
-// conv bins [olo, ohi] the caller's grid needs.  The 0.01-1000 keV sum of the convolution is
-// sum_i hr_i * (window sum of xs) / cf, from prefix sums of xs, and the band sum of the xillver
-// spectrum is the band's window sum of xs / cf (cf = E/dE is the same in every bin of the log grid
-// up to rounding, and cancels), so bins outside [olo, ohi] are never convolved.  The sums are
-// float-float (about 48 significant bits, on the FP32 pipe).
-__device__ void conv_normalize_store(ConvSmem &m, const RelxTables &tab, int wlo, int whi, int olo, int ohi,
-                                     float2 sr, float *out) {
+// Factor that normalises the convolution of xs with hr as calcFFTNormFactor (Relbase.cpp:199-222):
+// (band sum of the profile) * (band sum of xs) / (band sum of the convolution), over 0.01-1000 keV.  (The
+// xillver spectrum's band sum is that of xs / cf, and cf = E/dE, the same in every bin of the log grid up
+// to rounding, cancels.)  The last is sum_i hr_i W_i with W_i = sum of xs over [a_i, a_i + L), a_i = lo + p - i
+// modulo N for a band of L bins from lo: no bin has to be convolved for it.  W_p is the band sum of xs
+// itself, and W changes by d_j = xs[a_j - 1] - xs[a_j + L - 1] from j to j + 1, so summed by parts
+//   sum_i hr_i W_i = (sum_i hr_i) W_p + sum_{j >= p} d_j (sum_{i > j} hr_i) - sum_{j < p} d_j (sum_{i <= j} hr_i):
+// one sum over xs and prefix sums over the profile's window, a fraction of xs's bins (4096 relxilllp sets of 10
+// zones: with prefix sums over all of xs 1168 us, so and with the stores of conv_bins 930 us, with its aligned
+// tiles 835 us).  The sums are float-float (about 48 significant bits, on
+// the FP32 pipe).  pr: the thread's part of the profile's band sum; xs is zero outside [xlo, xhi).  Starts
+// behind a barrier after xs and hr are complete; two barriers.
+__device__ __forceinline__ float conv_norm(ConvSmem &m, const RelxTables &tab, int wlo, int whi, int xlo, int xhi,
+                                           float2 pr) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  // prefix sums of xs at every kPre-th bin
-  {
-    constexpr int per = kN / kConvThreads;
-    float2 grp[per / kPre];
-    float2 loc = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int g = 0; g < per / kPre; g++) {
-      float2 gs = make_float2(0.0f, 0.0f);
-#pragma unroll
-      for (int q = 0; q < kPre; q++) gs = ff_addf(gs, m.xs[skew(tid * per + g * kPre + q)]);
-      grp[g] = gs;
-      loc = ff_add(loc, gs);
-    }
-    float2 inc = loc;
+  const int p = tab.conv_pos1;
+  const int blo = tab.conv_band_lo, bhi = tab.conv_band_hi, L = bhi - blo + 1;
+  // prefix sums of the profile at the start of the thread's run of bins, over the window and p
+  const int J0 = min(wlo, p), J1 = max(whi, p), R = (J1 - J0 + kConvThreads - 1) / kConvThreads;
+  const int j0 = J0 + tid * R, j1 = min(j0 + R, J1);
+  const bool busy = J0 + w * 32 * R < J1;  // the warp has bins
+  float2 run = make_float2(0.0f, 0.0f), inc = run;
+  if (busy) {
+    for (int j = max(j0, wlo); j < min(j1, whi); j++) inc = ff_addf(inc, m.hr[j - wlo]);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       float2 t;
@@ -181,80 +175,121 @@ __device__ void conv_normalize_store(ConvSmem &m, const RelxTables &tab, int wlo
       t.y = __shfl_up_sync(0xffffffffu, inc.y, o);
       if (lane >= o) inc = ff_add(t, inc);
     }
-    float2 exc;
-    exc.x = __shfl_up_sync(0xffffffffu, inc.x, 1);
-    exc.y = __shfl_up_sync(0xffffffffu, inc.y, 1);
-    if (lane == 0) exc = make_float2(0.0f, 0.0f);
-    if (lane == 31) m.wsum[w] = inc;
-    __syncthreads();
-    float2 run = make_float2(0.0f, 0.0f);
-    for (int q = 0; q < w; q++) run = ff_add(run, m.wsum[q]);
-    run = ff_add(run, exc);
-#pragma unroll
-    for (int g = 0; g < per / kPre; g++) {
-      m.pre[(tid * per) / kPre + g] = run;
-      run = ff_add(run, grp[g]);
-    }
-    if (tid == kConvThreads - 1) m.pre[kN / kPre] = run;
-    __syncthreads();
+    run.x = __shfl_up_sync(0xffffffffu, inc.x, 1);
+    run.y = __shfl_up_sync(0xffffffffu, inc.y, 1);
+    if (lane == 0) run = make_float2(0.0f, 0.0f);
   }
-  const int p = tab.conv_pos1;
-  const int blo = tab.conv_band_lo, L = tab.conv_band_hi - tab.conv_band_lo + 1;
-  if (tid == 32) m.sxw = ff_add(prefix_at(m, blo + L), ff_neg(prefix_at(m, blo)));  // band sum of xs
-  float2 part = make_float2(0.0f, 0.0f);
-  for (int i = wlo + tid; i < whi; i += kConvThreads) {
-    const int a = (blo + p - i) & (kN - 1);
-    float2 ws;
-    if (a + L <= kN) ws = ff_add(prefix_at(m, a + L), ff_neg(prefix_at(m, a)));
-    else ws = ff_add(ff_add(m.pre[kN / kPre], ff_neg(prefix_at(m, a))), prefix_at(m, a + L - kN));
-    part = ff_add(part, ff_mulf(ws, m.hr[i - wlo]));
-  }
-  const float2 scf = block_sum_ff<kConvThreads>(part, m.red);
-  if (tid == 0) m.bc[1] = ff_div_to_float(ff_mul(sr, m.sxw), scf);  // the barrier of block_sum_ff orders m.sxw
+  if (lane == 31) m.wsum[w] = inc;
+  // band sum of xs (a bin below the band that is not finite spoils it, as it does the convolution)
+  float2 sx = make_float2(0.0f, 0.0f);
+  const float *xp = &m.xs[skew(xlo + tid)];
+  for (int j = xlo + tid; j < min(xhi, bhi + 1); j += kConvThreads, xp += conv_skew(kConvThreads))
+    sx = ff_addf(sx, j < blo ? *xp * 0.0f : *xp);
   __syncthreads();
-  const float norm = m.bc[1];
+  // the warps' sums: prefixes within groups of 8 lanes
+  float2 ws = m.wsum[lane & 7];
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    float2 t;
+    t.x = __shfl_up_sync(0xffffffffu, ws.x, o, 8);
+    t.y = __shfl_up_sync(0xffffffffu, ws.y, o, 8);
+    if ((lane & 7) >= o) ws = ff_add(t, ws);
+  }
+  const float2 tot = shfl_ff(ws, 7);
+  ws = shfl_ff(ws, max(w - 1, 0));
+  if (w > 0 && busy) run = ff_add(ws, run);
+  // the change of the windows over the profile
+  float2 part = make_float2(0.0f, 0.0f);
+  for (int j = j0; j < j1; j++) {
+    if (j >= wlo && j < whi) run = ff_addf(run, m.hr[j - wlo]);
+    const int a = blo + p - j;
+    const float2 d = two_sum(m.xs[skew((a - 1) & (kN - 1))], -m.xs[skew((a + L - 1) & (kN - 1))]);
+    const float2 t = j < p ? ff_neg(run) : ff_add(tot, ff_neg(run));
+    part = ff_add(part, ff_mul(t, d));
+  }
+  // the three sums over the block: lanes 0-7 end with the profile's, 8-15 with that of xs, 16-23 with part
+  const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
+  const float2 zero = make_float2(0.0f, 0.0f);
+  const float2 k0 = ff_add(h16 ? part : pr, shfl_xor_ff(h16 ? pr : part, 16));
+  const float2 k1 = ff_add(h16 ? zero : sx, shfl_xor_ff(h16 ? sx : zero, 16));
+  float2 v = ff_add(h8 ? k1 : k0, shfl_xor_ff(h8 ? k0 : k1, 8));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v = ff_add(v, shfl_xor_ff(v, o));
+  if ((lane & 7) == 0) m.wred[lane + w] = v;
+  __syncthreads();
+  v = m.wred[lane];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v = ff_add(v, shfl_xor_ff(v, o));
+  const float2 spr = shfl_ff(v, 0), ssx = shfl_ff(v, 8), spart = shfl_ff(v, 16);
+  return ff_div_to_float(ff_mul(spr, ssx), ff_add(ff_mul(tot, ssx), spart));
+}
+
+// The convolution of xs with hr divided by E/dE and normalised, for the conv bins [olo, ohi] the caller's grid
+// needs; bins outside are never convolved.  It goes to global memory by way of m.y: a thread's 16 bins
+// are 64 bytes, and stored by it they cost a write of every sector for each of its 8 floats.
+__device__ __forceinline__ void conv_bins(ConvSmem &m, const RelxTables &tab, int wlo, int whi, int olo, int ohi,
+                                          float norm, float *__restrict__ out) {
+  const int tid = threadIdx.x, p = tab.conv_pos1;
   if (olo > ohi) return;
-  const int olo_out = olo;
-  olo -= (olo + p - wlo) & 3;  // tiles start where the xs loads of conv_tile are 16-byte aligned
-  // work items: (16-bin output tile, window segment).  The window is split into S (a power of two)
+  // work items: (16-bin output tile, window segment).  The window is split into S = 1 << sh
   // segments so that narrow output ranges still occupy every thread; the S partials of a tile sit
   // in adjacent lanes and are added by a fixed shuffle tree, so the result depends only on this
   // set's own sizes.
-  const int nt = (ohi - olo + 1 + kConvR - 1) / kConvR;
   const int nc = (whi - wlo + kConvD - 1) / kConvD;
-  int S = 1, best = split_cost(nt, nc, 1);
-  for (int c = 2; c <= 32 && c <= nc; c <<= 1) {
-    const int cost = split_cost(nt, nc, c);
-    if (cost < best) { best = cost; S = c; }
+  const int nt4 = (ohi - olo + ((olo + p - wlo) & 3) + kConvR) / kConvR;  // tiles, if aligned to 4 bins
+  int sh = 0, best = split_cost(nt4, nc, 0);
+  for (int c = 1; c <= 5 && (1 << c) <= nc; c++) {
+    const int cost = split_cost(nt4, nc, c);
+    if (cost < best) { best = cost; sh = c; }
   }
-  const int seg = ((nc + S - 1) / S) * kConvD;  // window bins per segment
-  const int nitems = nt * S;
+  const int seg = ((nc + (1 << sh) - 1) >> sh) * kConvD;  // window bins per segment
+  const int k0 = olo - ((olo + p - wlo) & 15);  // tiles start on rows of xs
+  const int nitems = ((ohi - k0) / kConvR + 1) << sh;
   for (int q0 = 0; q0 < nitems; q0 += kConvThreads) {
     const int q = q0 + tid;
-    const int t = q / S, sg = q % S;
+    const int t = q >> sh, sg = q & ((1 << sh) - 1);
     float y[kConvR];
     if (q < nitems) {
       const int clo = wlo + sg * seg, chi = min(whi, clo + seg);
-      conv_tile(m, olo + t * kConvR, p, wlo, clo, chi, y);
+      conv_tile(m, k0 + t * kConvR, p, wlo, clo, chi, y);
     } else {
 #pragma unroll
       for (int r = 0; r < kConvR; r++) y[r] = 0.0f;
     }
-    for (int o = S >> 1; o > 0; o >>= 1) {
+    for (int o = (1 << sh) >> 1; o > 0; o >>= 1) {
 #pragma unroll
       for (int r = 0; r < kConvR; r++) y[r] += __shfl_xor_sync(0xffffffffu, y[r], o);
     }
     if (q < nitems && sg == 0) {
 #pragma unroll
-      for (int r = 0; r < kConvR; r++) {
-        const int k = olo + t * kConvR + r;
-        if (k >= olo_out && k <= ohi) out[k] = y[r] * __frcp_rn(tab.conv_cf[k]) * norm;
-      }
+      for (int r = 0; r < kConvR; r++) m.y[t * (kConvR + 1) + r] = y[r];
     }
+  }
+  __syncthreads();
+  for (int k = olo + tid; k <= ohi; k += kConvThreads) {
+    const int i = k - k0;
+    out[k] = m.y[i + (i >> 4)] * __frcp_rn(tab.conv_cf[k]) * norm;
   }
 }
 
-__global__ void __launch_bounds__(kConvThreads) conv_zone_kernel(RelxTables tab, const RelxSetState *__restrict__ sst,
+// The profile pz over its window weighted by E/dE, in hr; returns the thread's part of its band sum
+__device__ __forceinline__ float2 profile_window(ConvSmem &m, const RelxTables &tab, const float *__restrict__ pz, int wlo,
+                                                 int whi, float fscale) {
+  float2 pr = make_float2(0.0f, 0.0f);
+  for (int i = threadIdx.x; i < whi - wlo + kConvR; i += kConvThreads) {
+    const int j = wlo + i;
+    float v = 0.0f;
+    if (j < whi) {
+      const float fr = pz[j] * fscale;
+      v = fr * tab.conv_cf[j];
+      if (j >= tab.conv_band_lo && j <= tab.conv_band_hi) pr = ff_addf(pr, fr);
+    }
+    m.hr[i] = v;
+  }
+  return pr;
+}
+
+__global__ void __launch_bounds__(kConvThreads, 4) conv_zone_kernel(RelxTables tab, const RelxSetState *__restrict__ sst,
                                                                  const float *__restrict__ prof,
                                                                  const double *__restrict__ tsum, int nblk,
                                                                  const float *__restrict__ xill, int nza,
@@ -265,61 +300,46 @@ __global__ void __launch_bounds__(kConvThreads) conv_zone_kernel(RelxTables tab,
   const RelxSetState &s = sst[set];
   if (s.status != RELX_OK || s.model < RELX_RELXILL || z >= s.nz) return;
   float *out = cout + ((size_t) set * nza + z) * kN;
-  profile_sums(m, s, tsum, set, nblk, nza, z);
+  // the zone's xillver spectrum on the conv grid (x E/dE) in the layout of xs: one bulk copy into place,
+  // overlapped with the profile loads
+  const int clo = tab.x_clo, chi = tab.x_clo + tab.x_cpad;
+  const uint32_t xbytes = (uint32_t) conv_skew(tab.x_cpad) * 4u;
+  if (tid == 0) {
+    mbar_init(&m.bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(&m.bar, xbytes);
+    bulk_g2s(&m.xs[skew(clo)], xill + ((size_t) set * nza + z) * conv_skew(tab.x_cpad), xbytes, &m.bar);
+  }
+  float fscale = 1.0f;
+  if (s.relline_norm > 0.0) {
+    profile_sums(m, s, tsum, set, nblk, nza);
+    fscale = m.bc;
+  } else if (tid < 32) {  // without renormalisation (lamp post) the zone's own sum
+    const double zs = zone_sum_warp(s, tsum, set, nblk, nza, z);
+    if (tid == 0) m.zsum[z] = zs;
+  }
+  const int wlo = s.zw_lo[z], whi = s.zw_hi[z];  // the zone's profile is zero outside
+  const float2 pr = profile_window(m, tab, prof + ((size_t) set * nza + z) * kN, wlo, whi, fscale);
+  // bins the table does not reach are zero
+  for (int j = tid; j < skew(clo) / 4; j += kConvThreads)
+    reinterpret_cast<float4 *>(m.xs)[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int j = skew(chi) / 4 + tid; j < skew(kN) / 4; j += kConvThreads)
+    reinterpret_cast<float4 *>(m.xs)[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  __syncthreads();  // the mbarrier is initialised, hr and the zone's sum are complete
+  if (__syncthreads_or(!mbar_wait_bounded(&m.bar, 0))) {
+    if (tid == 0) {
+      (void) mbar_wait_bounded(&m.bar, 0);  // give the copy in flight another bounded wait
+      atomicExch(err, RELX_ERR_TIMEOUT);
+    }
+    return;
+  }
   // relxill_convolution_multizone skips zones without flux (Relxill.cpp:455-457)
   if (m.zsum[z] < 1e-12) {
     for (int k = s.out_lo + tid; k <= s.out_hi; k += kConvThreads) out[k] = 0.0f;
     return;
   }
-  const int wlo = s.zw_lo[z], whi = s.zw_hi[z];  // the zone's profile is zero outside
-  const float fscale = m.bc[0];
-  const float *pz = prof + ((size_t) set * nza + z) * kN;
-  // the zone's xillver spectrum on the conv grid (x E/dE): one bulk copy into shared memory,
-  // overlapped with the profile loads
-  const float *xz = xill + ((size_t) set * nza + z) * tab.x_cpad;
-  // bulk copies need 16-byte aligned rows of a 16-byte multiple (rows are padded to 4 floats)
-  const bool staged = tab.x_cpad <= kXStage && (tab.x_cpad & 3) == 0 && (((uintptr_t) xz) & 15) == 0;
-  if (staged && tid == 0) {
-    m.abort_flag = 0;
-    mbar_init(&m.bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(&m.bar, (uint32_t) tab.x_cpad * 4u);
-    bulk_g2s(m.xz, xz, (uint32_t) tab.x_cpad * 4u, &m.bar);
-  }
-  // relline profile weighted by E/dE over its window; band sum of the profile
-  float2 pr = make_float2(0.0f, 0.0f);
-  for (int i = tid; i < whi - wlo + kConvR; i += kConvThreads) {
-    const int j = wlo + i;
-    float v = 0.0f;
-    if (j < whi) {
-      const float fr = pz[j] * fscale;
-      v = fr * tab.conv_cf[j];
-      if (j >= tab.conv_band_lo && j <= tab.conv_band_hi) pr = ff_addf(pr, fr);
-    }
-    m.hr[i] = v;
-  }
-  if (staged) {
-    __syncthreads();  // the barrier is initialised
-    if (!mbar_wait_bounded(&m.bar, 0)) atomicExch(&m.abort_flag, 1);
-    __syncthreads();
-    if (m.abort_flag) {
-      if (tid == 0) {
-        (void) mbar_wait_bounded(&m.bar, 0);  // give the copy in flight another bounded wait
-        atomicExch(err, RELX_ERR_TIMEOUT);
-      }
-      return;
-    }
-  }
-  const float *xs_src = staged ? m.xz : xz;
-  // the zone's spectrum, already rebinned onto the conv grid and weighted by E/dE (the table rows
-  // are, and the zone spectrum is linear in them): bins outside the table's reach are zero
-  const int clo = tab.x_clo, cn = tab.x_cn;
-  for (int j = tid; j < kN; j += kConvThreads) {
-    const int q = j - clo;
-    m.xs[skew(j)] = (q >= 0 && q < cn) ? xs_src[q] : 0.0f;
-  }
-  const float2 sr = block_sum_ff<kConvThreads>(pr, m.red);
-  conv_normalize_store(m, tab, wlo, whi, s.out_lo, s.out_hi, sr, out);
+  const float norm = conv_norm(m, tab, wlo, whi, clo, chi, pr);
+  conv_bins(m, tab, wlo, whi, s.out_lo, s.out_hi, norm, out);
 }
 
 // relconv (relconv_kernel, Relbase.cpp:257-289): the caller's spectrum is
@@ -350,10 +370,13 @@ __global__ void __launch_bounds__(kConvThreads) relconv_conv_kernel(RelxTables t
     if (tid == 0) sflag[set] = RELX_ERR_INPUT;
     return;
   }
-  profile_sums(m, s, tsum, set, nblk, nza, 0);
+  float fscale = 1.0f;
+  if (s.relline_norm > 0.0) {
+    profile_sums(m, s, tsum, set, nblk, nza);
+    fscale = m.bc;
+  }
   const int wlo = s.win_lo, whi = s.win_hi;
   const int zlo = s.zw_lo[0], zhi = s.zw_hi[0];  // the convolved zone's profile is zero outside
-  const float fscale = m.bc[0];
   const float *pz = prof + (size_t) set * nza * kN;
   float2 pr = make_float2(0.0f, 0.0f);
   for (int i = tid; i < whi - wlo + kConvR; i += kConvThreads) {
@@ -397,8 +420,9 @@ __global__ void __launch_bounds__(kConvThreads) relconv_conv_kernel(RelxTables t
     }
     m.xs[skew(j)] = v * tab.conv_cf[j];
   }
-  const float2 sr = block_sum_ff<kConvThreads>(pr, m.red);
-  conv_normalize_store(m, tab, wlo, whi, s.out_lo, s.out_hi, sr, out);
+  __syncthreads();
+  const float norm = conv_norm(m, tab, wlo, whi, 0, kN, pr);
+  conv_bins(m, tab, wlo, whi, s.out_lo, s.out_hi, norm, out);
 }
 
 // _rebin_spectrum (relutility.c:549-601) of one output bin from the conv grid; the bin indices
@@ -569,7 +593,7 @@ __global__ void __launch_bounds__(kFinThreads) finalize_relline_kernel(const Rel
 }
 
 size_t conv_smem_bytes() { return sizeof(ConvSmem); }
-size_t fin_smem_bytes() { return sizeof(FinSmem); }
+static_assert(4 * (sizeof(ConvSmem) + 1024) <= 228 * 1024, "four CTAs per SM");
 
 // wide: 512 threads per set (few sets: one set's bins spread over more threads); otherwise 128.
 // Every output is computed by one thread with the same arithmetic, so both give the same numbers.

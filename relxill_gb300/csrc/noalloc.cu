@@ -65,14 +65,14 @@ constexpr size_t kScratchBytes =
                                                                                : kMaxLineBins)) +  // profile
     align_up(sizeof(float) * RELX_NZMAX * RELX_MAX_INCL) +                                   // angle histogram
     align_up(sizeof(double) * (size_t) ((kMaxLineBins + kSumBinsH - 1) / kSumBinsH) * RELX_NZMAX) +  // block sums
-    align_up(sizeof(float) * (size_t) RELX_NZMAX * kMaxXillBins) +                           // xillver spectra
+    align_up(sizeof(float) * (size_t) RELX_NZMAX * (kMaxXillBins + kMaxXillBins / 4)) +      // xillver spectra
     align_up(sizeof(float) * (size_t) RELX_NZMAX * RELX_NCONV) +                             // convolved spectra
     align_up(sizeof(double) * (RELX_NZMAX + 1)) + align_up(sizeof(NthTable)) +               // nthcomp (Cp)
     align_up(sizeof(float4) * (size_t) (RELX_NZMAX + 1) * 900) +                             // nthcomp solve
     align_up(sizeof(float4) * (size_t) RELX_MAX_NRTAB * RELX_MAX_NG) +                      // interpolated table
     3 * kAlign;                                                                              // flags
 
-// the scratch of this entry point (about 3.8 MB)
+// the scratch of this entry point (about 4.0 MB)
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 struct NoallocPtrs {
@@ -107,7 +107,7 @@ static size_t carve(unsigned char *base, int model, int nza, int nbins, int nblk
   p->prof = (float *) take(sizeof(float) * (line ? (size_t) nbins : (size_t) nza * RELX_NCONV));
   p->dist = (float *) take(sizeof(float) * nza * RELX_MAX_INCL);
   p->tsum = (double *) take(sizeof(double) * nblk * nza);
-  p->xill = (float *) take(sizeof(float) * (size_t) nza * x_pad);
+  p->xill = (float *) take(sizeof(float) * (size_t) nza * conv_skew(x_pad));
   p->cout = (float *) take(sizeof(float) * (size_t) nza * RELX_NCONV);
   const bool cp = relx_is_cp(model);
   p->nthq = (double *) take(cp ? sizeof(double) * (RELX_NZMAX + 1) : 0);

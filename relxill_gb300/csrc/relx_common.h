@@ -108,7 +108,8 @@ struct RelxTables {
   const float *x_spec;       // [rows][x_nener_pad], each row divided by 10^logXi of its grid point
   int64_t x_rows;
   // the same rows rebinned onto the conv grid and weighted by E/dE of the conv bin (the form the
-  // convolution reads): conv bins [x_clo, x_clo + x_cn), rows of x_cpad floats (a multiple of 4)
+  // convolution reads): conv bins [x_clo, x_clo + x_cn), rows of x_cpad floats; x_clo and x_cpad are
+  // multiples of 16, the rows of conv_skew
   const float *x_cspec;
   int x_clo, x_cn, x_cpad;
   // conv grid and precomputed maps
@@ -143,6 +144,10 @@ struct RelxTables {
   // nthcomp photon grid of the Cp models (nthcomp.cu)
   const NthGrid *nth_grid;
 };
+
+// Position of conv bin m in the layout of the zone spectra and of the convolution's shared memory: rows of
+// 16 bins, each followed by 4 floats of padding (no bank conflicts between threads 16 bins apart)
+RELX_HD inline int conv_skew(int m) { return m + ((m >> 4) << 2); }
 
 // per-set inputs
 struct RelxSetIn {

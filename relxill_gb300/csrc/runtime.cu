@@ -734,9 +734,9 @@ static int load_tables(const std::string &dir, Tables &T) {
       g_errmsg = "xillver table: its energy grid does not overlap the convolution grid";
       return RELX_ERR_TABLE;
     }
-    d.x_clo = clo;
-    d.x_cn = chi + 1 - clo;
-    d.x_cpad = (d.x_cn + 3) & ~3;
+    d.x_clo = clo & ~15;  // whole rows of conv_skew (bins the table does not reach hold zeros)
+    d.x_cn = chi + 1 - d.x_clo;
+    d.x_cpad = (d.x_cn + 15) & ~15;
     return 0;
   };
   if ((st = rebin_tables(xe, T.x, T.d)) || (has_cp && (st = rebin_tables(xe_cp, T.xcp, T.dcp)))) return st;
@@ -1140,7 +1140,7 @@ static int reserve_workspace(const Tables &T, Workspace &W, const BatchShape &b,
   }
   if (relx_is_relxill(kind)) {
     if ((st = W.corners.reserve(S * sizeof(RelxCorners))) || (st = W.order.reserve(S * sizeof(int))) ||
-        (st = W.xill.reserve(S * nza * (size_t) std::max(T.d.x_cpad, T.dcp.x_cpad) * sizeof(float))))
+        (st = W.xill.reserve(S * nza * (size_t) conv_skew(std::max(T.d.x_cpad, T.dcp.x_cpad)) * sizeof(float))))
       return st;
     if (need_zone_corners && (st = W.zcorners.reserve(S * sizeof(RelxZoneCorners)))) return st;
   }
@@ -1185,7 +1185,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   float *prof = conv_grid ? W.prof.as<float>() + (size_t) base * nza * RELX_NCONV : W.prof.as<float>();
   float *dist = W.dist.as<float>() + (size_t) base * nza * RELX_MAX_INCL;
   double *tsum = W.tsum.as<double>() + (size_t) base * b.nblk * nza;
-  float *xill = W.xill.p ? W.xill.as<float>() + (size_t) base * nza * tab.x_cpad : nullptr;
+  float *xill = W.xill.p ? W.xill.as<float>() + (size_t) base * nza * conv_skew(tab.x_cpad) : nullptr;
   float *cout = W.cout.p ? W.cout.as<float>() + (size_t) base * nza * RELX_NCONV : nullptr;
   int *sflag = W.sflag.as<int>() + base;
   double *flux = W.flux.as<double>() - base;  // kernels address set i at e_off(i) - i
@@ -1785,7 +1785,7 @@ size_t batch_device_bytes(int model, int n_sets, int64_t n_edges, int max_bins, 
   else per_edge += (kind == RELX_RELCONV) ? sizeof(double) : 0;              // relconv input
   if (kind != RELX_RELLINE) per_set += 2 * sizeof(float) * (size_t) nza * RELX_NCONV;
   if (relx_is_relxill(kind))
-    per_set += sizeof(RelxCorners) + sizeof(float) * (size_t) nza * 4096;
+    per_set += sizeof(RelxCorners) + sizeof(float) * (size_t) nza * conv_skew(RELX_NCONV);
   if (relx_is_cp(model) || nza > RELX_ZDENSE) per_set += sizeof(RelxZoneCorners);
   return staged + cp + per_set * S + per_edge * E + err_bytes(S) +
          line_list_entries(n_sets, nza, (int) nblk) * sizeof(uint2) +

@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) xillver_dense_kernel(R
 #pragma unroll
     for (int z = 0; z < NZ; z++) {
       if (z < nz) {
-        float4 *o = reinterpret_cast<float4 *>(xout + ((size_t) set * nza + z) * pitch + e0) + q;
-        *o = acc[z];
+        float *o = xout + ((size_t) set * nza + z) * conv_skew(pitch) + conv_skew(e0 + 4 * q);
+        *reinterpret_cast<float4 *>(o) = acc[z];
       }
     }
   }
@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(kXillThreads) xillver_zone_kernel(RelxTables t
     }
   }
   for (int z = 0; z < nz; z++)
-    reinterpret_cast<float4 *>(xout + ((size_t) set * nza + z) * pitch + e0)[q] = acc[z * kXillThreads + q];
+    *reinterpret_cast<float4 *>(xout + ((size_t) set * nza + z) * conv_skew(pitch) + conv_skew(e0 + 4 * q)) =
+        acc[z * kXillThreads + q];
 }
 
 #define RELX_XILL_INSTANCES(X) X(1, 10) X(10, 10) X(16, 10) X(1, 0) X(10, 0) X(16, 0)
