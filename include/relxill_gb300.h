@@ -113,6 +113,13 @@ int relx_eval_batch(int model, int n_sets, const double *params, const double *e
                     const int64_t *energy_offsets, const double *flux_in, double *flux, int *status,
                     const int *ion_grad_type, const double *iongrad_index);
 
+/* Same with every set's grid and input spectrum where the caller has them: energy[i] points at the
+ * energy_offsets[i+1] - energy_offsets[i] edges of set i, flux_in[i] at its input spectrum (relconv /
+ * relconv_lp; NULL otherwise).  flux is laid out as above. */
+int relx_eval_batch_sets(int model, int n_sets, const double *params, const double *const *energy,
+                         const int64_t *energy_offsets, const double *const *flux_in, double *flux, int *status,
+                         const int *ion_grad_type, const double *iongrad_index);
+
 /* Same with device buffers, asynchronous on `stream` (a cudaStream_t; NULL:
  * the library's stream).  flux_in (relconv) uses the energy-edge layout
  * (set i at energy_offsets[i]).  h_energy_offsets and h_ion_grad_type are host

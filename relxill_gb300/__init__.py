@@ -13,7 +13,10 @@ present, calls raise.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
+import sysconfig
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -21,6 +24,7 @@ import numpy as np
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_lib", "librelxill_gb300.so")
+HOST_EXT_PATH = os.path.join(_HERE, "_lib", "_relx_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 MODELS: Dict[str, int] = {"relline": 0, "relconv": 1, "relxill": 2, "relxilllp": 3, "relline_lp": 4,
                           "relconv_lp": 5, "xillver": 6, "xillverCp": 7, "relxillCp": 8, "relxilllpCp": 9}
@@ -71,6 +75,7 @@ class RelxillError(RuntimeError):
 
 
 _lib: Optional[ctypes.CDLL] = None
+_host_ext = None
 
 _dp = ctypes.POINTER(ctypes.c_double)
 _ip = ctypes.POINTER(ctypes.c_int)
@@ -91,6 +96,9 @@ def lib() -> ctypes.CDLL:
     L.relx_last_status.restype = ctypes.c_int
     L.relx_eval_batch.argtypes = [ctypes.c_int, ctypes.c_int, _dp, _dp, _lp, _dp, _dp, _ip, _ip, _dp]
     L.relx_eval_batch.restype = ctypes.c_int
+    L.relx_eval_batch_sets.argtypes = [ctypes.c_int, ctypes.c_int, _dp, ctypes.c_char_p, _lp, ctypes.c_char_p, _dp, _ip,
+                                       _ip, _dp]
+    L.relx_eval_batch_sets.restype = ctypes.c_int
     L.relx_eval_batch_device.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                          _lp, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, _ip,
                                          ctypes.c_void_p, ctypes.c_void_p]
@@ -128,6 +136,19 @@ def lib() -> ctypes.CDLL:
         fn.restype = None
     _lib = L
     return L
+
+
+def _host():
+    """The extension that reads arrays' addresses (csrc/pyhost.c)."""
+    global _host_ext
+    if _host_ext is None:
+        if not os.path.exists(HOST_EXT_PATH):
+            raise RuntimeError(f"{HOST_EXT_PATH} is missing: build it with `python -m relxill_gb300.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_relx_host", HOST_EXT_PATH)
+        ext = importlib.util.module_from_spec(importlib.util.spec_from_loader("_relx_host", loader))
+        loader.exec_module(ext)
+        _host_ext = ext
+    return _host_ext
 
 
 def _ptr(a: np.ndarray, t=_dp):
@@ -175,7 +196,20 @@ def eval_batch(model: str, params, energies: Sequence[np.ndarray], flux_in: Opti
     n = p.shape[0]
     if len(energies) != n:
         raise ValueError("one energy grid per parameter set")
-    edges, offs = pack_grids(energies)
+    energies = list(energies)  # the arrays stay alive and in place while their addresses are in use
+    plain = _host().arrays(energies)
+    if plain is not None and model in CONV_MODELS and flux_in is not None:
+        flux_in = list(flux_in)
+        spectra = _host().arrays(flux_in)
+        # as many values as bins in each, or they are joined as they come
+        if spectra is None or not np.array_equal(np.frombuffer(spectra[1], np.int64) + 1,
+                                                 np.frombuffer(plain[1], np.int64)):
+            plain = None
+    if plain is None:
+        edges, offs = pack_grids(energies)
+    else:
+        offs = np.zeros(n + 1, dtype=np.int64)
+        np.cumsum(np.frombuffer(plain[1], np.int64), out=offs[1:])
     nflux = int(offs[-1]) - n
     flux = np.zeros(nflux, dtype=np.float64)
     status = np.zeros(n, dtype=np.int32)
@@ -183,16 +217,22 @@ def eval_batch(model: str, params, energies: Sequence[np.ndarray], flux_in: Opti
     if model in CONV_MODELS:
         if flux_in is None:
             raise ValueError(f"{model} needs the input spectra")
-        fin = np.concatenate([np.asarray(f, dtype=np.float64) for f in flux_in])
+        if plain is None:
+            fin = np.concatenate([np.asarray(f, dtype=np.float64) for f in flux_in])
     igt = None if ion_grad_type is None else np.ascontiguousarray(ion_grad_type, dtype=np.int32)
     igi = None if iongrad_index is None else np.ascontiguousarray(iongrad_index, dtype=np.float64)
-    st = L.relx_eval_batch(MODELS[model], n, _ptr(p), _ptr(edges), _ptr(offs, _lp),
-                           _ptr(fin) if fin is not None else None, _ptr(flux), _ptr(status, _ip),
-                           _ptr(igt, _ip) if igt is not None else None, _ptr(igi) if igi is not None else None)
+    tail = (_ptr(flux), _ptr(status, _ip), _ptr(igt, _ip) if igt is not None else None,
+            _ptr(igi) if igi is not None else None)
+    if plain is not None:
+        st = L.relx_eval_batch_sets(MODELS[model], n, _ptr(p), plain[0], _ptr(offs, _lp),
+                                    spectra[0] if model in CONV_MODELS else None, *tail)
+    else:
+        st = L.relx_eval_batch(MODELS[model], n, _ptr(p), _ptr(edges), _ptr(offs, _lp),
+                               _ptr(fin) if fin is not None else None, *tail)
     if check and st and not np.any(status):
         raise RelxillError(st, L.relx_last_error().decode())
-    out = [flux[offs[i] - i: offs[i + 1] - i - 1] for i in range(n)]
-    return out, status
+    at = (offs - np.arange(n + 1)).tolist()
+    return [flux[a:b] for a, b in zip(at, at[1:])], status
 
 
 def _lmod(model: str, energy, params, flux_in=None) -> np.ndarray:
@@ -327,28 +367,36 @@ class Server:
         if not self._h:
             raise RelxillError(last_status_or(6), last_error())
         self._keep: Dict[int, tuple] = {}
+        self._submit = _host().submit
+        self._submit_fn = ctypes.cast(L.relx_serve_submit, ctypes.c_void_p).value
 
     def submit(self, model: str, params, energy: np.ndarray, out: np.ndarray, flux_in: Optional[np.ndarray] = None,
                ion_grad_type: int = 0, iongrad_index: float = 0.0) -> int:
+        rid = self._submit(self._submit_fn, self._h, MODELS[model], len(PARAMS[model]), params, energy, out, flux_in,
+                           ion_grad_type, iongrad_index)
+        if rid is None:  # arrays that need a conversion, or a refusal
+            rid = self._submit_any(model, params, energy, out, flux_in, ion_grad_type, iongrad_index)
+        if rid < 0:
+            raise RelxillError(int(-rid), last_error())
+        self._keep[rid] = (energy, out, flux_in)
+        return rid
+
+    def _submit_any(self, model, params, energy, out, flux_in, ion_grad_type, iongrad_index) -> int:
         p = np.ascontiguousarray(params, dtype=np.float64)
         if energy.dtype != np.float64 or not energy.flags.c_contiguous:
             raise ValueError("energy must be a contiguous float64 array")
         if out.dtype != np.float64 or not out.flags.c_contiguous or len(out) != len(energy) - 1:
             raise ValueError("out must be a contiguous float64 array of len(energy) - 1")
-        rid = lib().relx_serve_submit(self._h, MODELS[model], _ptr(p), _ptr(energy), len(energy) - 1,
-                                      _ptr(flux_in) if flux_in is not None else None, _ptr(out),
-                                      int(ion_grad_type), float(iongrad_index))
-        if rid < 0:
-            raise RelxillError(int(-rid), last_error())
-        self._keep[rid] = (p, energy, out, flux_in)
-        return int(rid)
+        return int(lib().relx_serve_submit(self._h, MODELS[model], _ptr(p), _ptr(energy), len(energy) - 1,
+                                           _ptr(flux_in) if flux_in is not None else None, _ptr(out),
+                                           int(ion_grad_type), float(iongrad_index)))
 
     def poll(self, max_n: int = 4096) -> List[Tuple[int, int, float]]:
         ids = np.zeros(max_n, dtype=np.int64)
         sts = np.zeros(max_n, dtype=np.int32)
         lat = np.zeros(max_n, dtype=np.float64)
         n = lib().relx_serve_poll(self._h, _ptr(ids, _lp), _ptr(sts, _ip), _ptr(lat), max_n)
-        res = [(int(ids[i]), int(sts[i]), float(lat[i])) for i in range(n)]
+        res = list(zip(ids[:n].tolist(), sts[:n].tolist(), lat[:n].tolist())) if n > 0 else []
         for rid, _, _ in res:
             self._keep.pop(rid, None)
         return res

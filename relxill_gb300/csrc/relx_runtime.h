@@ -25,9 +25,11 @@ void runtime_set_error(int status, const char *msg);
 struct HostBatch {
   int model = 0, n_sets = 0;
   const double *params = nullptr;   // n_sets x npar
-  const double *energy = nullptr;   // concatenated edges
+  const double *energy = nullptr;   // concatenated edges, or
+  const double *const *energies = nullptr;   // each set's edges
   const int64_t *eoff = nullptr;    // n_sets + 1 edge offsets
-  const double *flux_in = nullptr;  // relconv inputs (flux layout) or null
+  const double *flux_in = nullptr;  // relconv inputs (flux layout) or null, or
+  const double *const *spectra = nullptr;    // each set's (with energies)
   const int *igt = nullptr;         // ionisation-gradient type per set or null
   const double *igi = nullptr;      // ionisation-gradient index per set or null
 };

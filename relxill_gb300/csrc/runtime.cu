@@ -1513,9 +1513,12 @@ static int batch_shape(int model, int n_sets, const int64_t *eoff_host, const in
 static int enqueue_host_batch(Context &C, Workspace &W, Pinned &P, cudaStream_t s, const HostBatch &hb,
                               bool use_cache, size_t *o_flux, size_t *o_status, bool allow_tune = true) {
   const int model = hb.model, n_sets = hb.n_sets;
-  if (model < 0 || model >= RELX_NMODELS || n_sets <= 0 || !hb.params || !hb.energy || !hb.eoff) return RELX_ERR_ARG;
+  if (model < 0 || model >= RELX_NMODELS || n_sets <= 0 || !hb.params || (!hb.energy && !hb.energies) || !hb.eoff)
+    return RELX_ERR_ARG;
   const bool conv = relx_kind(model) == RELX_RELCONV;
-  if (conv && !hb.flux_in) return RELX_ERR_ARG;
+  if (conv && !(hb.energies ? (const void *) hb.spectra : hb.flux_in)) return RELX_ERR_ARG;
+  for (int i = 0; hb.energies && i < n_sets; i++)
+    if (!hb.energies[i] || (conv && !hb.spectra[i])) return RELX_ERR_ARG;
   if (relx_is_cp(model) && !C.T.has_cp) {
     g_errmsg = "xillverCp_v3.4.fits not found: the Cp models need the nthcomp xillver table";
     return RELX_ERR_NOTABLE;
@@ -1544,6 +1547,9 @@ static int enqueue_host_batch(Context &C, Workspace &W, Pinned &P, cudaStream_t 
     return o;
   };
   size_t o_p = put(hb.params, pb), o_e = put(hb.energy, eb), o_o = put(hb.eoff, ob);
+  for (int i = 0; hb.energies && i < n_sets; i++)
+    jobs.push_back({(double *) (h + o_e) + hb.eoff[i], hb.energies[i],
+                    sizeof(double) * (size_t) (hb.eoff[i + 1] - hb.eoff[i])});
   size_t o_g = hb.igt ? put(hb.igt, gb) : 0, o_i = hb.igi ? put(hb.igi, ib) : 0;
   size_t o_f = 0;
   if (conv) {
@@ -1552,7 +1558,7 @@ static int enqueue_host_batch(Context &C, Workspace &W, Pinned &P, cudaStream_t 
     double *fi = (double *) (h + o_f);
     for (int i = 0; i < n_sets; i++) {
       int n = (int) (hb.eoff[i + 1] - hb.eoff[i] - 1);
-      jobs.push_back({fi + hb.eoff[i], hb.flux_in + (hb.eoff[i] - i), sizeof(double) * n});
+      jobs.push_back({fi + hb.eoff[i], hb.spectra ? hb.spectra[i] : hb.flux_in + (hb.eoff[i] - i), sizeof(double) * n});
     }
   }
   CopyPool::get().run(jobs);
@@ -1616,7 +1622,7 @@ static int eval_host(const HostBatch &hb, double *flux, int *status) {
   int st = ensure_init(C, nullptr);
   if (st) return st;
   const int n = hb.n_sets;
-  if (hb.model < 0 || hb.model >= RELX_NMODELS || n <= 0 || !hb.params || !hb.energy || !hb.eoff)
+  if (hb.model < 0 || hb.model >= RELX_NMODELS || n <= 0 || !hb.params || (!hb.energy && !hb.energies) || !hb.eoff)
     return RELX_ERR_ARG;
   const std::vector<int> s0 = host_groups(n);
   const int ng = (int) s0.size() - 1;
@@ -1633,7 +1639,9 @@ static int eval_host(const HostBatch &hb, double *flux, int *status) {
     b = hb;
     b.n_sets = m;
     b.params = hb.params + (size_t) a * npar;
-    b.energy = hb.energy + e0;
+    b.energy = hb.energy ? hb.energy + e0 : nullptr;
+    b.energies = hb.energies ? hb.energies + a : nullptr;
+    b.spectra = hb.spectra ? hb.spectra + a : nullptr;
     b.eoff = offs[g].data();
     b.flux_in = (conv && hb.flux_in) ? hb.flux_in + (e0 - a) : hb.flux_in;
     b.igt = hb.igt ? hb.igt + a : nullptr;
@@ -1855,6 +1863,23 @@ int relx_eval_batch(int model, int n_sets, const double *params, const double *e
   hb.energy = energy;
   hb.eoff = energy_offsets;
   hb.flux_in = flux_in;
+  hb.igt = ion_grad_type;
+  hb.igi = iongrad_index;
+  int st = eval_host(hb, flux, status);
+  g_last_status = st;
+  return st;
+}
+
+int relx_eval_batch_sets(int model, int n_sets, const double *params, const double *const *energy,
+                         const int64_t *energy_offsets, const double *const *flux_in, double *flux, int *status,
+                         const int *ion_grad_type, const double *iongrad_index) {
+  HostBatch hb;
+  hb.model = model;
+  hb.n_sets = n_sets;
+  hb.params = params;
+  hb.energies = energy;
+  hb.eoff = energy_offsets;
+  hb.spectra = flux_in;
   hb.igt = ion_grad_type;
   hb.igi = iongrad_index;
   int st = eval_host(hb, flux, status);

@@ -57,7 +57,8 @@ struct Completed {
 struct SlotState {
   BatchSlot *slot = nullptr;
   std::vector<Request> reqs;  // requests of the batch in flight
-  std::vector<double> params, energy, flux_in, igi;
+  std::vector<double> params, igi;
+  std::vector<const double *> energies, spectra;  // the clients' buffers
   std::vector<int64_t> eoff;
   std::vector<int> igt;
   bool busy = false;
@@ -118,22 +119,22 @@ void Server::scheduler() {
     }
     S.busy = true;
     lk.unlock();
-    // pack the host batch
+    // describe the host batch; it is staged from the clients' buffers
     const int n = (int) S.reqs.size(), npar = model_npar(model);
     S.params.resize((size_t) n * npar);
     S.eoff.assign(n + 1, 0);
     S.igt.resize(n);
     S.igi.resize(n);
     for (int i = 0; i < n; i++) S.eoff[i + 1] = S.eoff[i] + S.reqs[i].n_bins + 1;
-    S.energy.resize((size_t) S.eoff[n]);
     const bool conv = relx_kind(model) == RELX_RELCONV;
-    if (conv) S.flux_in.resize((size_t) (S.eoff[n] - n));
+    S.energies.resize(n);
+    S.spectra.resize(n);
     bool any_ig = false;
     for (int i = 0; i < n; i++) {
       const Request &r = S.reqs[i];
       std::memcpy(&S.params[(size_t) i * npar], r.params, sizeof(double) * npar);
-      std::memcpy(&S.energy[(size_t) S.eoff[i]], r.energy, sizeof(double) * (r.n_bins + 1));
-      if (conv) std::memcpy(&S.flux_in[(size_t) (S.eoff[i] - i)], r.flux_in, sizeof(double) * r.n_bins);
+      S.energies[i] = r.energy;
+      S.spectra[i] = r.flux_in;
       S.igt[i] = r.igt;
       S.igi[i] = r.igi;
       any_ig = any_ig || r.igt != 0;
@@ -142,9 +143,9 @@ void Server::scheduler() {
     hb.model = model;
     hb.n_sets = n;
     hb.params = S.params.data();
-    hb.energy = S.energy.data();
+    hb.energies = S.energies.data();
     hb.eoff = S.eoff.data();
-    hb.flux_in = conv ? S.flux_in.data() : nullptr;
+    hb.spectra = conv ? S.spectra.data() : nullptr;
     hb.igt = any_ig ? S.igt.data() : nullptr;
     hb.igi = any_ig ? S.igi.data() : nullptr;
     S.status = slot_enqueue(S.slot, hb, use_cache);
