@@ -240,7 +240,7 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
                                        nzones_env, flags, nza, p.sin, p.sflag, p.err);
   if (kind == RELX_XILLVER) {
     if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, 1, true, p.nthq, p.nth, nullptr, nullptr, p.nthscr, 1, 0));
-    NOALLOC_CUDA(launch_xillver_model(s, tab, 1, p.sin, d_energy, p.sst, d_flux, cp ? p.nthq : nullptr,
+    NOALLOC_CUDA(launch_xillver_model(s, tab, 1, n_bins, p.sin, d_energy, p.sst, d_flux, cp ? p.nthq : nullptr,
                                       cp ? p.nth : nullptr));
     noalloc_status_kernel<<<1, 32, 0, s>>>(p.sst, p.sflag, p.err, p.status, d_status);
     NOALLOC_CUDA(cudaGetLastError());
@@ -258,12 +258,12 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
                                 p.err, nullptr));
     conv_zone_kernel<<<dim3(nza, 1), kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sst, p.prof, p.tsum, nblk, p.xill, nza, p.cout,
                                                                             p.err);
-    NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, tab, p.sin, p.sst, p.cout, nza, d_energy, d_flux,
+    NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, n_bins, tab, p.sin, p.sst, p.cout, nza, d_energy, d_flux,
                                          cp ? p.nth : nullptr));
   } else if (kind == RELX_RELCONV) {
     relconv_conv_kernel<<<1, kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sin, p.sst, p.prof, p.tsum, nblk, nza, d_energy, d_flux_in, p.cout,
                                                                     p.sflag);
-    finalize_relconv_kernel<<<1, kFinThreadsH, 0, s>>>(tab, p.sin, p.sst, p.cout, nza, d_energy, p.sflag, d_flux);
+    finalize_relconv_kernel<<<dim3(1, out_parts(1, n_bins, kFinThreadsH, 608)), kFinThreadsH, 0, s>>>(tab, p.sin, p.sst, p.cout, nza, d_energy, p.sflag, d_flux);
   } else {
     finalize_relline_kernel<<<1, kFinThreadsH, 0, s>>>(p.sin, p.sst, p.prof, p.tsum, nblk, nza,
                                                         d_flux);

@@ -317,18 +317,19 @@ __device__ __forceinline__ int block_max_i(int v, int *scratch) {
   return r;
 }
 
-// Sum over the coarse normalisation grid of the cut-off power law times the bin centre, scaled to
-// the xillver table normalisation (calcNormWrtXillverTableSpec with spec_cutoffpl,
-// Xillspec.cpp:179-233): FP32 terms summed as float-float by one warp, every lane returns the
-// total.  cpow: E^-Gamma per coarse bin, or null to compute it here.
-__device__ __forceinline__ double primary_qsum_warp(const RelxTables &tab, float gam, float ecut, const float *cpow) {
+// Term of the sum over the coarse normalisation grid (bin centre, width, centre as float-float, 0 outside the
+// band) of the cut-off power law times the bin centre, scaled to the xillver table normalisation
+// (calcNormWrtXillverTableSpec with spec_cutoffpl, Xillspec.cpp:179-233), and the sum of the FP32 terms
+// as float-float by one warp; every lane returns it
+__device__ __forceinline__ float primary_term(float4 t, float gam, float ecut) {
+  return expf(1.0f / ecut) * powf(t.x, -gam) * expf(-t.x / ecut) * t.y;
+}
+__device__ __forceinline__ double primary_qsum_terms(const RelxTables &tab, const float *term) {
   const int lane = threadIdx.x & 31;
   float2 part = make_float2(0.0f, 0.0f);
   for (int b = lane; b < RELX_NCOARSE; b += 32) {
-    const float4 t = tab.coarse_t[b];  // bin centre, width, centre as float-float (0 outside the band)
-    const float pw = cpow ? cpow[b] : powf(t.x, -gam);
-    const float term = expf(1.0f / ecut) * pw * expf(-t.x / ecut) * t.y;
-    part = ff_add(part, ff_mulf(make_float2(t.z, t.w), term));
+    const float4 t = tab.coarse_t[b];
+    part = ff_add(part, ff_mulf(make_float2(t.z, t.w), term[b]));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -356,13 +357,23 @@ __device__ __forceinline__ double nth_prim_at(const double *x, const double *sp,
   return sp[jl] + (e / 511. * zp1 - x[jl]) * (sp[jl + 1] - sp[jl]) / (x[jl + 1] - x[jl]);
 }
 
-// 1 / f_spp(1 / xn): the table's E F_E at xn = (1 + z) / 511 (donthcomp.c:617-638, 754-758)
-__device__ __forceinline__ double nth_normfac(const double *x, const double *sp, int nth, double zp1) {
+// 1 / f_spp(1 / xn): the table's E F_E at xn = (1 + z) / 511 (donthcomp.c:617-638, 754-758), by a warp (every
+// lane returns it): the first point from the second on that is not below, 32 points per round instead
+// of the reference's walk
+__device__ __forceinline__ double nth_normfac_warp(const double *x, const double *sp, int nth, double zp1) {
   const double xn = zp1 / 511.;
   const double xx = 1 / (1 / xn);
-  int ih = 2;
-  while (ih < nth && xx > x[ih]) ++ih;
-  const int il = ih - 1;
+  const int lane = threadIdx.x & 31;
+  int lo = 2, hi = max(nth, 2);  // the point is in [lo, hi]
+  while (lo < hi) {
+    const int step = (hi - lo + 31) / 32;
+    const int i = min(lo + lane * step, hi);
+    const int n = __popc(__ballot_sync(0xffffffffu, i < hi && xx > x[i]));  // probes below, a prefix (x ascends)
+    const int l = lo;
+    lo = n ? min(l + (n - 1) * step, hi) + 1 : l;
+    hi = n < 32 ? min(l + n * step, hi) : hi;
+  }
+  const int ih = lo, il = ih - 1;
   return 1 / (sp[il] + (sp[ih] - sp[il]) * (xx - x[il]) / (x[ih] - x[il]));
 }
 

@@ -1,6 +1,7 @@
 // relx_kernels.h -- declarations of the sm_103a kernels and their launch
 // geometry, used by the host runtime (runtime.cu).
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include <vector>
@@ -14,7 +15,6 @@ constexpr int kSumBinsH = 32;    // bins per profile-sum block (tsum)
 constexpr int kLineTileH = 128;   // bins per task of the line profile of many sets
 constexpr int kConvThreadsH = 256;
 constexpr int kFinThreadsH = 128;
-constexpr int kXmodThreadsH = 256;  // xillver model kernel
 
 size_t hist_smem_bytes(int nr, int ng);
 size_t conv_smem_bytes();
@@ -97,7 +97,8 @@ cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetI
 size_t xillver_model_smem_bytes(int n_ener, int n_ener_pad);
 cudaError_t xillver_model_set_smem(int n_ener, int n_ener_pad);
 // xillverCp: nthq / nth from launch_nthcomp (params mode); null for xillver
-cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_sets, const RelxSetIn *sin,
+// n_bins: the output bins of all sets
+cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
                                  const double *user_e, RelxSetState *sst, double *flux, const double *nthq,
                                  const NthTable *nth);
 
@@ -107,10 +108,23 @@ __global__ void relconv_conv_kernel(RelxTables tab, const RelxSetIn *sin, const 
                                     const double *tsum, int nblk, int nza, const double *user_e,
                                     const double *user_f, float *cout, int *sflag);
 // nth: the nthcomp tables of the sets (Cp models), or null
-// zone sum, primary continuum and rebin to the caller's grid; wide: 512 threads per set (for few sets)
-cudaError_t launch_finalize_relxill(cudaStream_t s, bool wide, int n_sets, const RelxTables &tab,
+// zone sum, primary continuum and rebin to the caller's grid; few: 512 threads per CTA and few_parts CTAs per set
+cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_t n_bins, const RelxTables &tab,
                                     const RelxSetIn *sin, const RelxSetState *sst, const float *cout, int nza,
                                     const double *user_e, double *flux, const NthTable *nth);
+// CTAs per set for the output bins of few sets: about `per` bins of a mean set each, and at most `ctas` in all (as
+// many as run at once: 64 xillver sets in 256 CTAs of 1024 threads 31 us, in 128 CTAs 25 us).
+// Every bin is computed by one thread with the same arithmetic, so any split gives the same numbers.
+inline int out_parts(int n_sets, int64_t n_bins, int per, int ctas) {
+  const int64_t mean = n_bins / n_sets;
+  return (int) std::max<int64_t>(1, std::min<int64_t>((mean + per - 1) / per, ctas / n_sets));
+}
+// the part blockIdx.y of gridDim.y of bins 0..n-1
+#ifdef __CUDACC__
+__device__ __forceinline__ int2 out_range(int n) {
+  return make_int2((int) ((int64_t) n * blockIdx.y / gridDim.y), (int) ((int64_t) n * (blockIdx.y + 1) / gridDim.y));
+}
+#endif
 __global__ void finalize_relconv_kernel(RelxTables tab, const RelxSetIn *sin, const RelxSetState *sst,
                                         const float *cout, int nza, const double *user_e, const int *sflag,
                                         double *flux);

@@ -1198,7 +1198,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
     {
       ProfScope ps(PK_XILL, s);
-      RELX_CUDA(launch_xillver_model(s, tab, n, sin, user_e, sst, flux, nthq, ntab));
+      RELX_CUDA(launch_xillver_model(s, tab, n, b.n_edges - b.n_sets, sin, user_e, sst, flux, nthq, ntab));
     }
     ProfScope ps(PK_STATUS, s);
     status_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, sst, sflag, W.err.as<int>(), W.status.as<int>() + base);
@@ -1279,13 +1279,13 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
     {
       ProfScope ps(PK_FIN, s);
-      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, tab, sin, sst, cout, b.nza, user_e, flux, ntab));
+      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, cout, b.nza, user_e, flux, ntab));
     }
   } else if (kind == RELX_RELCONV) {
     ProfScope ps(PK_CONV, s, 2);  // convolution and finalize
     relconv_conv_kernel<<<n, kConvThreadsH, conv_smem_bytes(), s>>>(tab, sin, sst, prof, tsum, b.nblk, b.nza, user_e, W.user_f.as<double>(),
                                                                     cout, sflag);
-    finalize_relconv_kernel<<<n, kFinThreadsH, 0, s>>>(tab, sin, sst, cout, b.nza, user_e, sflag, flux);
+    finalize_relconv_kernel<<<dim3(n, out_parts(b.n_sets, b.n_edges - b.n_sets, kFinThreadsH, 608)), kFinThreadsH, 0, s>>>(tab, sin, sst, cout, b.nza, user_e, sflag, flux);
   } else {
     ProfScope ps(PK_FIN, s);
     finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, b.nza, flux);
