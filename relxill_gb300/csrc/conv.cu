@@ -27,6 +27,7 @@ constexpr int kConvR = 16;         // output bins per thread and work item
 constexpr int kConvD = 16;         // window bins per step of the register tile
 constexpr int kN = RELX_NCONV;
 constexpr int kConvWarps = kConvThreads / 32;
+static_assert(kN % kConvThreads == 0, "a thread per conv bin in the rebin");
 static_assert(kConvWarps == 8, "the warps' sums are added by groups of 8 lanes");
 
 // xs is stored in rows of 16 bins, each followed by 4 padding floats (conv_skew): the 16-byte loads of
@@ -342,34 +343,87 @@ __global__ void __launch_bounds__(kConvThreads, 4) conv_zone_kernel(RelxTables t
   conv_bins(m, tab, wlo, whi, s.out_lo, s.out_hi, norm, out);
 }
 
-// relconv (relconv_kernel, Relbase.cpp:257-289): the caller's spectrum is
-// rebinned onto the conv grid, convolved with the single-zone profile and
+// relconv (relconv_kernel, Relbase.cpp:257-289): the caller's spectrum is rebinned onto the conv grid
+// (relconv_rebin_kernel, in the layout of the zone spectra), convolved with the single-zone profile and
 // rebinned back; output bins outside 0.01-1000 keV are zero.
-__global__ void __launch_bounds__(kConvThreads) relconv_conv_kernel(RelxTables tab, const RelxSetIn *__restrict__ sin,
-                                                                    const RelxSetState *__restrict__ sst,
-                                                                    const float *__restrict__ prof,
-                                                                    const double *__restrict__ tsum, int nblk, int nza,
-                                                                    const double *__restrict__ user_e,
-                                                                    const double *__restrict__ user_f, float *__restrict__ cout,
-                                                                    int *__restrict__ sflag) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ConvSmem &m = *reinterpret_cast<ConvSmem *>(smem_raw);
-  const int set = blockIdx.x, tid = threadIdx.x;
+
+// Largest index with a[m] <= v (0 if none) of the n ascending positive edges
+__device__ __forceinline__ int last_le(const double *a, int n, double v) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int k = (lo + hi) >> 1;
+    if (dge(v, a[k])) lo = k + 1; else hi = k;
+  }
+  return max(lo - 1, 0);
+}
+
+// _rebin_spectrum (relutility.c:549-601), conv grid <- caller's grid: a thread per conv bin, times E/dE.  Each
+// edge is searched once for the two bins that share it, by comparisons of bit patterns on the integer
+// pipe, and by many CTAs: within the convolution's CTA the FP64 comparisons of two searches per bin held
+// one SM's FP64 pipe for two thirds of the kernel (with the rebin back, 11 to 16 sets 70 us, so 45 us;
+// 152 sets 79 us and 73 us).
+__global__ void __launch_bounds__(kConvThreads) relconv_rebin_kernel(RelxTables tab, const RelxSetIn *__restrict__ sin,
+                                                                     const RelxSetState *__restrict__ sst,
+                                                                     const double *__restrict__ user_e,
+                                                                     const double *__restrict__ user_f,
+                                                                     float *__restrict__ xs) {
+  __shared__ int at[kConvThreads + 1];  // last caller's edge at or below each conv edge
+  const int set = blockIdx.x, tid = threadIdx.x, j = blockIdx.y * kConvThreads + tid;
   const RelxSetState &s = sst[set];
   if (s.status != RELX_OK || s.model != RELX_RELCONV) return;
   const RelxSetIn &in = sin[set];
   const double *ue = user_e + in.e_off;
   const double *uf = user_f + in.e_off;
   const int nu = in.n_ener;
+  const double elo0 = tab.conv_e[j], ehi0 = tab.conv_e[j + 1];
+  at[tid] = last_le(ue, nu + 1, elo0);
+  if (tid == kConvThreads - 1) at[kConvThreads] = last_le(ue, nu + 1, ehi0);
+  __syncthreads();
+  float v = 0.0f;
+  if (dge(ehi0, ue[0]) && dge(ue[nu], elo0)) {
+    const int imin = at[tid], imax = min(at[tid + 1], nu - 1);
+    const double elo = dgt(ue[imin], elo0) ? ue[imin] : elo0;
+    const double ehi = dgt(ehi0, ue[imax + 1]) ? ue[imax + 1] : ehi0;
+    if (imax == imin) {
+      v = (float) ((ehi - elo) / (ue[imin + 1] - ue[imin]) * uf[imin]);
+    } else {
+      const double dmin = (ue[imin + 1] - elo) / (ue[imin + 1] - ue[imin]);
+      const double dmax = (ehi - ue[imax]) / (ue[imax + 1] - ue[imax]);
+      double acc = uf[imin] * dmin + uf[imax] * dmax;
+      for (int q = imin + 1; q <= imax - 1; q++) acc += uf[q];
+      v = (float) acc;
+    }
+  }
+  xs[(size_t) set * conv_skew(kN) + conv_skew(j)] = v * tab.conv_cf[j];
+}
+
+__global__ void __launch_bounds__(kConvThreads, 4) relconv_conv_kernel(RelxTables tab, const RelxSetIn *__restrict__ sin,
+                                                                       const RelxSetState *__restrict__ sst,
+                                                                       const float *__restrict__ prof,
+                                                                       const double *__restrict__ tsum, int nblk, int nza,
+                                                                       const double *__restrict__ user_f,
+                                                                       const float *__restrict__ xs, float *__restrict__ cout,
+                                                                       int *__restrict__ sflag, int *__restrict__ err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ConvSmem &m = *reinterpret_cast<ConvSmem *>(smem_raw);
+  const int set = blockIdx.x, tid = threadIdx.x;
+  const RelxSetState &s = sst[set];
+  if (s.status != RELX_OK || s.model != RELX_RELCONV) return;
+  const RelxSetIn &in = sin[set];
+  const double *uf = user_f + in.e_off;
+  const int nu = in.n_ener;
   float *out = cout + (size_t) set * nza * kN;
+  const uint32_t xbytes = (uint32_t) conv_skew(kN) * 4u;
+  if (tid == 0) {
+    mbar_init(&m.bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(&m.bar, xbytes);
+    bulk_g2s(m.xs, xs + (size_t) set * conv_skew(kN), xbytes, &m.bar);
+  }
   // conv_model requires a positive input sum (LocalModel.cpp:84-86)
   double ps = 0.0;
   for (int i = tid; i < nu; i += kConvThreads) ps += uf[i];
   const double usum = block_sum_d<kConvThreads>(ps, m.dred);
-  if (!(usum > 0.0)) {
-    if (tid == 0) sflag[set] = RELX_ERR_INPUT;
-    return;
-  }
   float fscale = 1.0f;
   if (s.relline_norm > 0.0) {
     profile_sums(m, s, tsum, set, nblk, nza);
@@ -389,38 +443,18 @@ __global__ void __launch_bounds__(kConvThreads) relconv_conv_kernel(RelxTables t
     }
     m.hr[i] = v;
   }
-  // _rebin_spectrum(conv grid <- user grid)
-  const double *ce = tab.conv_e;
-  for (int j = tid; j < kN; j += kConvThreads) {
-    const double elo0 = ce[j], ehi0 = ce[j + 1];
-    float v = 0.0f;
-    if (ue[0] <= ehi0 && ue[nu] >= elo0) {
-      int imin = 0, imax = 0;
-      {  // largest index with ue[m] <= elo0 (0 if none), capped at nu
-        int lo = 0, hi = nu + 1;
-        while (lo < hi) { int k = (lo + hi) >> 1; if (ue[k] <= elo0) lo = k + 1; else hi = k; }
-        imin = lo > 0 ? lo - 1 : 0;
-      }
-      {  // largest index <= nu-1 with ue[m] <= ehi0 (0 if none)
-        int lo = 0, hi = nu;
-        while (lo < hi) { int k = (lo + hi) >> 1; if (ue[k] <= ehi0) lo = k + 1; else hi = k; }
-        imax = lo > 0 ? lo - 1 : 0;
-      }
-      double elo = elo0 < ue[imin] ? ue[imin] : elo0;
-      double ehi = ehi0 > ue[imax + 1] ? ue[imax + 1] : ehi0;
-      if (imax == imin) {
-        v = (float) ((ehi - elo) / (ue[imin + 1] - ue[imin]) * uf[imin]);
-      } else {
-        double dmin = (ue[imin + 1] - elo) / (ue[imin + 1] - ue[imin]);
-        double dmax = (ehi - ue[imax]) / (ue[imax + 1] - ue[imax]);
-        double acc = uf[imin] * dmin + uf[imax] * dmax;
-        for (int q = imin + 1; q <= imax - 1; q++) acc += uf[q];
-        v = (float) acc;
-      }
+  // the copy is complete before the CTA may end
+  if (__syncthreads_or(!mbar_wait_bounded(&m.bar, 0))) {
+    if (tid == 0) {
+      (void) mbar_wait_bounded(&m.bar, 0);
+      atomicExch(err, RELX_ERR_TIMEOUT);
     }
-    m.xs[skew(j)] = v * tab.conv_cf[j];
+    return;
   }
-  __syncthreads();
+  if (!(usum > 0.0)) {
+    if (tid == 0) sflag[set] = RELX_ERR_INPUT;
+    return;
+  }
   const float norm = conv_norm(m, tab, wlo, whi, 0, kN, pr);
   conv_bins(m, tab, wlo, whi, s.out_lo, s.out_hi, norm, out);
 }
@@ -604,6 +638,21 @@ __global__ void __launch_bounds__(kFinThreads) finalize_relline_kernel(const Rel
   // as here
   const int lo = s.zw_lo[s.nz - 1], hi = s.zw_hi[s.nz - 1];
   for (int i = tid; i < nu; i += kFinThreads) fo[i] = ((i >= lo && i < hi) ? (double) p[i] : 0.0) * scale;
+}
+
+cudaError_t relconv_set_smem() {
+  return cudaFuncSetAttribute(relconv_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(ConvSmem));
+}
+cudaError_t launch_relconv(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
+                           const RelxSetState *sst, const float *prof, const double *tsum, int nblk, int nza,
+                           const double *user_e, const double *user_f, float *xs, float *cout, int *sflag, int *err,
+                           double *flux) {
+  relconv_rebin_kernel<<<dim3(n_sets, kN / kConvThreads), kConvThreads, 0, s>>>(tab, sin, sst, user_e, user_f, xs);
+  relconv_conv_kernel<<<n_sets, kConvThreads, sizeof(ConvSmem), s>>>(tab, sin, sst, prof, tsum, nblk, nza, user_f, xs,
+                                                                     cout, sflag, err);
+  finalize_relconv_kernel<<<dim3(n_sets, out_parts(n_sets, n_bins, kFinThreads, 608)), kFinThreads, 0, s>>>(
+      tab, sin, sst, cout, nza, user_e, sflag, flux);
+  return cudaGetLastError();
 }
 
 size_t conv_smem_bytes() { return sizeof(ConvSmem); }

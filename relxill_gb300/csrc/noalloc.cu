@@ -107,7 +107,7 @@ static size_t carve(unsigned char *base, int model, int nza, int nbins, int nblk
   p->prof = (float *) take(sizeof(float) * (line ? (size_t) nbins : (size_t) nza * RELX_NCONV));
   p->dist = (float *) take(sizeof(float) * nza * RELX_MAX_INCL);
   p->tsum = (double *) take(sizeof(double) * nblk * nza);
-  p->xill = (float *) take(sizeof(float) * (size_t) nza * conv_skew(x_pad));
+  p->xill = (float *) take(sizeof(float) * (size_t) nza * conv_skew(relx_kind(model) == RELX_RELCONV ? RELX_NCONV : x_pad));
   p->cout = (float *) take(sizeof(float) * (size_t) nza * RELX_NCONV);
   const bool cp = relx_is_cp(model);
   p->nthq = (double *) take(cp ? sizeof(double) * (RELX_NZMAX + 1) : 0);
@@ -261,9 +261,8 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
     NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, n_bins, tab, p.sin, p.sst, p.cout, nza, d_energy, d_flux,
                                          cp ? p.nth : nullptr));
   } else if (kind == RELX_RELCONV) {
-    relconv_conv_kernel<<<1, kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sin, p.sst, p.prof, p.tsum, nblk, nza, d_energy, d_flux_in, p.cout,
-                                                                    p.sflag);
-    finalize_relconv_kernel<<<dim3(1, out_parts(1, n_bins, kFinThreadsH, 608)), kFinThreadsH, 0, s>>>(tab, p.sin, p.sst, p.cout, nza, d_energy, p.sflag, d_flux);
+    NOALLOC_CUDA(launch_relconv(s, tab, 1, n_bins, p.sin, p.sst, p.prof, p.tsum, nblk, nza, d_energy, d_flux_in, p.xill,
+                                p.cout, p.sflag, p.err, d_flux));
   } else {
     finalize_relline_kernel<<<1, kFinThreadsH, 0, s>>>(p.sin, p.sst, p.prof, p.tsum, nblk, nza,
                                                         d_flux);

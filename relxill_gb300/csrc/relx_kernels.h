@@ -104,9 +104,13 @@ cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_se
 
 __global__ void conv_zone_kernel(RelxTables tab, const RelxSetState *sst, const float *prof, const double *tsum,
                                  int nblk, const float *xill, int nza, float *cout, int *err);
-__global__ void relconv_conv_kernel(RelxTables tab, const RelxSetIn *sin, const RelxSetState *sst, const float *prof,
-                                    const double *tsum, int nblk, int nza, const double *user_e,
-                                    const double *user_f, float *cout, int *sflag);
+// relconv of n_sets sets with n_bins output bins in all: three kernels; xs: conv_skew(RELX_NCONV) floats per set
+constexpr int kRelconvKernels = 3;
+cudaError_t relconv_set_smem();
+cudaError_t launch_relconv(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
+                           const RelxSetState *sst, const float *prof, const double *tsum, int nblk, int nza,
+                           const double *user_e, const double *user_f, float *xs, float *cout, int *sflag, int *err,
+                           double *flux);
 // nth: the nthcomp tables of the sets (Cp models), or null
 // zone sum, primary continuum and rebin to the caller's grid; few: 512 threads per CTA and few_parts CTAs per set
 cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_t n_bins, const RelxTables &tab,
@@ -125,9 +129,6 @@ __device__ __forceinline__ int2 out_range(int n) {
   return make_int2((int) ((int64_t) n * blockIdx.y / gridDim.y), (int) ((int64_t) n * (blockIdx.y + 1) / gridDim.y));
 }
 #endif
-__global__ void finalize_relconv_kernel(RelxTables tab, const RelxSetIn *sin, const RelxSetState *sst,
-                                        const float *cout, int nza, const double *user_e, const int *sflag,
-                                        double *flux);
 __global__ void finalize_relline_kernel(const RelxSetIn *sin, const RelxSetState *sst, const float *prof,
                                         const double *tsum, int nblk, int nza, double *flux);
 

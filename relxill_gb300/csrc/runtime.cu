@@ -990,7 +990,7 @@ static int set_kernel_attrs(const Tables &T) {
     RELX_CUDA(xillver_model_set_smem(ne, nep));
   }
   RELX_CUDA(cudaFuncSetAttribute(conv_zone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) conv_smem_bytes()));
-  RELX_CUDA(cudaFuncSetAttribute(relconv_conv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) conv_smem_bytes()));
+  RELX_CUDA(relconv_set_smem());
   return 0;
 }
 
@@ -1136,7 +1136,9 @@ static int reserve_workspace(const Tables &T, Workspace &W, const BatchShape &b,
     if ((st = W.prof.reserve(S * nza * RELX_NCONV * sizeof(float))) ||
         (st = W.cout.reserve(S * nza * RELX_NCONV * sizeof(float))))
       return st;
-    if (kind == RELX_RELCONV && (st = W.user_f.reserve(b.n_edges * sizeof(double)))) return st;
+    if (kind == RELX_RELCONV && ((st = W.user_f.reserve(b.n_edges * sizeof(double))) ||
+                                 (st = W.xill.reserve(S * conv_skew(RELX_NCONV) * sizeof(float)))))
+      return st;
   }
   if (relx_is_relxill(kind)) {
     if ((st = W.corners.reserve(S * sizeof(RelxCorners))) || (st = W.order.reserve(S * sizeof(int))) ||
@@ -1185,7 +1187,9 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   float *prof = conv_grid ? W.prof.as<float>() + (size_t) base * nza * RELX_NCONV : W.prof.as<float>();
   float *dist = W.dist.as<float>() + (size_t) base * nza * RELX_MAX_INCL;
   double *tsum = W.tsum.as<double>() + (size_t) base * b.nblk * nza;
-  float *xill = W.xill.p ? W.xill.as<float>() + (size_t) base * nza * conv_skew(tab.x_cpad) : nullptr;
+  // relconv: one spectrum per set on the whole conv grid
+  const size_t xset = kind == RELX_RELCONV ? conv_skew(RELX_NCONV) : nza * conv_skew(tab.x_cpad);
+  float *xill = W.xill.p ? W.xill.as<float>() + (size_t) base * xset : nullptr;
   float *cout = W.cout.p ? W.cout.as<float>() + (size_t) base * nza * RELX_NCONV : nullptr;
   int *sflag = W.sflag.as<int>() + base;
   double *flux = W.flux.as<double>() - base;  // kernels address set i at e_off(i) - i
@@ -1282,10 +1286,9 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
       RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, cout, b.nza, user_e, flux, ntab));
     }
   } else if (kind == RELX_RELCONV) {
-    ProfScope ps(PK_CONV, s, 2);  // convolution and finalize
-    relconv_conv_kernel<<<n, kConvThreadsH, conv_smem_bytes(), s>>>(tab, sin, sst, prof, tsum, b.nblk, b.nza, user_e, W.user_f.as<double>(),
-                                                                    cout, sflag);
-    finalize_relconv_kernel<<<dim3(n, out_parts(b.n_sets, b.n_edges - b.n_sets, kFinThreadsH, 608)), kFinThreadsH, 0, s>>>(tab, sin, sst, cout, b.nza, user_e, sflag, flux);
+    ProfScope ps(PK_CONV, s, kRelconvKernels);
+    RELX_CUDA(launch_relconv(s, tab, n, b.n_edges - b.n_sets, sin, sst, prof, tsum, b.nblk, b.nza, user_e,
+                             W.user_f.as<double>(), xill, cout, sflag, W.err.as<int>(), flux));
   } else {
     ProfScope ps(PK_FIN, s);
     finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, b.nza, flux);
@@ -1792,6 +1795,7 @@ size_t batch_device_bytes(int model, int n_sets, int64_t n_edges, int max_bins, 
   if (kind == RELX_RELLINE) per_edge += sizeof(double) + sizeof(float);     // line grid, profile
   else per_edge += (kind == RELX_RELCONV) ? sizeof(double) : 0;              // relconv input
   if (kind != RELX_RELLINE) per_set += 2 * sizeof(float) * (size_t) nza * RELX_NCONV;
+  if (kind == RELX_RELCONV) per_set += sizeof(float) * (size_t) conv_skew(RELX_NCONV);
   if (relx_is_relxill(kind))
     per_set += sizeof(RelxCorners) + sizeof(float) * (size_t) nza * conv_skew(RELX_NCONV);
   if (relx_is_cp(model) || nza > RELX_ZDENSE) per_set += sizeof(RelxZoneCorners);
