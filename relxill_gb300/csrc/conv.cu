@@ -497,6 +497,7 @@ struct FinSmem {
 template <int NT>
 __global__ void __launch_bounds__(NT) finalize_relxill_kernel(RelxTables tab, const RelxSetIn *__restrict__ sin,
                                                                         const RelxSetState *__restrict__ sst,
+                                                                        const int *__restrict__ sflag,
                                                                         const float *__restrict__ cout, int nza,
                                                                         const double *__restrict__ user_e,
                                                                         double *__restrict__ flux,
@@ -509,8 +510,9 @@ __global__ void __launch_bounds__(NT) finalize_relxill_kernel(RelxTables tab, co
   const int nu = in.n_ener;
   double *fo = flux + in.e_off - set;  // flux offsets: e_off counts n+1 edges per set
   const int2 part = out_range(nu);
-  if (s.status != RELX_OK || s.model < RELX_RELXILL) {
-    if (s.model != RELX_RELCONV || s.status != RELX_OK)
+  const bool bad = s.status != RELX_OK || sflag[set] != RELX_OK;
+  if (bad || s.model < RELX_RELXILL) {
+    if (s.model != RELX_RELCONV || bad)
       for (int i = part.x + tid; i < part.y; i += NT) fo[i] = 0.0;
     return;
   }
@@ -662,13 +664,14 @@ static_assert(4 * (sizeof(ConvSmem) + 1024) <= 228 * 1024, "four CTAs per SM");
 // 12 us); otherwise a CTA of 128 per set.
 // Every output is computed by one thread with the same arithmetic, so both give the same numbers.
 cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_t n_bins, const RelxTables &tab,
-                                    const RelxSetIn *sin, const RelxSetState *sst, const float *cout, int nza,
+                                    const RelxSetIn *sin, const RelxSetState *sst, const int *sflag,
+                                    const float *cout, int nza,
                                     const double *user_e, double *flux, const NthTable *nth) {
   if (n_sets <= 0) return cudaSuccess;
   if (few)
-    finalize_relxill_kernel<512><<<dim3(n_sets, out_parts(n_sets, n_bins, 512, 304)), 512, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e, flux, nth);
+    finalize_relxill_kernel<512><<<dim3(n_sets, out_parts(n_sets, n_bins, 512, 304)), 512, sizeof(FinSmem), s>>>(tab, sin, sst, sflag, cout, nza, user_e, flux, nth);
   else
-    finalize_relxill_kernel<kFinThreads><<<n_sets, kFinThreads, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e,
+    finalize_relxill_kernel<kFinThreads><<<n_sets, kFinThreads, sizeof(FinSmem), s>>>(tab, sin, sst, sflag, cout, nza, user_e,
                                                                                      flux, nth);
   return cudaGetLastError();
 }

@@ -239,7 +239,7 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
   noalloc_pack_kernel<<<1, 32, 0, s>>>(runtime_nparams(model), d_params, n_bins, ion_grad_type, iongrad_index,
                                        nzones_env, flags, nza, p.sin, p.sflag, p.err);
   if (kind == RELX_XILLVER) {
-    if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, 1, true, p.nthq, p.nth, nullptr, nullptr, p.nthscr, 1, 0));
+    if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, 1, true, p.nthq, p.nth, nullptr, nullptr, nullptr, p.nthscr, 1, 0));
     NOALLOC_CUDA(launch_xillver_model(s, tab, 1, n_bins, p.sin, d_energy, p.sst, d_flux, cp ? p.nthq : nullptr,
                                       cp ? p.nth : nullptr));
     noalloc_status_kernel<<<1, 32, 0, s>>>(p.sst, p.sflag, p.err, p.status, d_status);
@@ -248,7 +248,7 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
     return RELX_OK;
   }
   NOALLOC_CUDA(launch_setup(s, 1, tab, model, p.sin, d_energy, p.line_e, p.sst, p.rad, p.cor, p.zcor));
-  if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, nza, false, p.nthq, p.nth, p.cor, p.zcor, p.nthscr, nza + 1, 0));
+  if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, nza, false, p.nthq, p.nth, p.cor, p.zcor, p.sflag, p.nthscr, nza + 1, 0));
   NOALLOC_CUDA(launch_line_table(1, nza, s, tab, p.sst, p.htab, p.rad, nullptr, nullptr));
   NOALLOC_CUDA(launch_relline(1, nblk, s, tab, p.sin, p.sst, p.rad, p.line_e, nza, p.prof, p.tsum,
                               kind == RELX_RELLINE || kind == RELX_RELCONV, p.htab, nullptr, nullptr));
@@ -258,7 +258,7 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
                                 p.err, nullptr));
     conv_zone_kernel<<<dim3(nza, 1), kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sst, p.prof, p.tsum, nblk, p.xill, nza, p.cout,
                                                                             p.err);
-    NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, n_bins, tab, p.sin, p.sst, p.cout, nza, d_energy, d_flux,
+    NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, n_bins, tab, p.sin, p.sst, p.sflag, p.cout, nza, d_energy, d_flux,
                                          cp ? p.nth : nullptr));
   } else if (kind == RELX_RELCONV) {
     NOALLOC_CUDA(launch_relconv(s, tab, 1, n_bins, p.sin, p.sst, p.prof, p.tsum, nblk, nza, d_energy, d_flux_in, p.xill,

@@ -544,7 +544,9 @@ __global__ void __launch_bounds__(kNthCoopThreads) nthcomp_coop_kernel(const Nth
 
 // normalisation changes of the zones on their corner weights (the de-duplicated list or the per-zone
 // lists), source normalisation of the primary
-__global__ void nthcomp_apply_kernel(RelxSetState *__restrict__ sst, const double *__restrict__ q, int nq,
+// sflag: marks a set without a spectrum; the set-up's status is left alone, as the line profile's kernels may be
+// reading it on another stream
+__global__ void nthcomp_apply_kernel(RelxSetState *__restrict__ sst, int *__restrict__ sflag, const double *__restrict__ q, int nq,
                                      RelxCorners *__restrict__ cor, RelxZoneCorners *__restrict__ zcor) {
   const int set = blockIdx.x, tid = threadIdx.x;
   RelxSetState &s = sst[set];
@@ -554,7 +556,7 @@ __global__ void nthcomp_apply_kernel(RelxSetState *__restrict__ sst, const doubl
   for (int z = 0; z < s.nz && !bad; z++)
     if (s.zshift[z] != 1.0 && !isfinite(q[(size_t) set * nq + z + 1])) bad = true;
   if (bad) {  // no nthcomp spectrum for the set's kTe (every thread sees the same)
-    if (tid == 0) s.status = RELX_ERR_PARAM;
+    if (tid == 0) sflag[set] = RELX_ERR_PARAM;
     return;
   }
   const int nz = s.nz;
@@ -590,7 +592,7 @@ size_t nthcomp_scratch_bytes(int n_sets, int nza, bool params) {
 
 cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetIn *sin, RelxSetState *sst, int n_sets,
                            int nza, bool params, double *q, NthTable *tabs, RelxCorners *cor, RelxZoneCorners *zcor,
-                           float4 *scr, int64_t ncont_all, int64_t c_off) {
+                           int *sflag, float4 *scr, int64_t ncont_all, int64_t c_off) {
   if (n_sets <= 0) return cudaSuccess;
   const int nq = RELX_NZMAX + 1;
   const int per = params ? 1 : nza + 1;
@@ -603,7 +605,7 @@ cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetI
                      sizeof(NthPoint) * (RELX_NTH_N + 1), s>>>(tab.nth_grid, sin, sst, params, per, n_sets, nq, q,
                                                               tabs, scr, ncont_all, c_off);
   }
-  if (!params) nthcomp_apply_kernel<<<n_sets, 128, 0, s>>>(sst, q, nq, cor, zcor);
+  if (!params) nthcomp_apply_kernel<<<n_sets, 128, 0, s>>>(sst, sflag, q, nq, cor, zcor);
   return cudaGetLastError();
 }
 

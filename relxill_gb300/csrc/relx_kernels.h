@@ -90,7 +90,7 @@ size_t nthcomp_scratch_bytes(int n_sets, int nza, bool params);
 // scr: scratch of nthcomp_scratch_bytes for the whole batch, ncont_all continua per grid point,
 // this launch's continua starting at c_off.
 cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetIn *sin, RelxSetState *sst, int n_sets,
-                           int nza, bool params, double *q, NthTable *tabs, RelxCorners *cor, RelxZoneCorners *zcor,
+                           int nza, bool params, double *q, NthTable *tabs, RelxCorners *cor, RelxZoneCorners *zcor, int *sflag,
                            float4 *scr, int64_t ncont_all, int64_t c_off);
 
 // the xillver model: one CTA per set, writes the flux and the status fields of the set state
@@ -114,7 +114,8 @@ cudaError_t launch_relconv(cudaStream_t s, const RelxTables &tab, int n_sets, in
 // nth: the nthcomp tables of the sets (Cp models), or null
 // zone sum, primary continuum and rebin to the caller's grid; few: 512 threads per CTA and few_parts CTAs per set
 cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_t n_bins, const RelxTables &tab,
-                                    const RelxSetIn *sin, const RelxSetState *sst, const float *cout, int nza,
+                                    const RelxSetIn *sin, const RelxSetState *sst, const int *sflag,
+                                    const float *cout, int nza,
                                     const double *user_e, double *flux, const NthTable *nth);
 // CTAs per set for the output bins of few sets: about `per` bins of a mean set each, and at most `ctas` in all (as
 // many as run at once: 64 xillver sets in 256 CTAs of 1024 threads 31 us, in 128 CTAs 25 us).

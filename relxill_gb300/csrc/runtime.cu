@@ -941,8 +941,8 @@ struct Context {
   // per launching stream, a side stream for the emission-angle histograms and the xillver stage,
   // which depend on the set-up only and run beside the line profile (fork and join events)
   struct Side {
-    cudaStream_t main, side;
-    cudaEvent_t fork, join;
+    cudaStream_t main, side, nth;  // nth: the nthcomp continua
+    cudaEvent_t fork, join, nfork, njoin;
   };
   std::vector<Side> sides;
   cudaEvent_t aux_ev[2] = {nullptr, nullptr}, fork_ev = nullptr;
@@ -1154,13 +1154,17 @@ static Context::Side *side_of(Context &C, cudaStream_t s) {
   for (auto &x : C.sides)
     if (x.main == s) return &x;
   if (C.sides.size() >= 16) return nullptr;
-  Context::Side x{s, nullptr, nullptr, nullptr};
-  if (cudaStreamCreateWithFlags(&x.side, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming) != cudaSuccess) {
+  Context::Side x{s, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  bool ok = true;
+  for (cudaStream_t *t : {&x.side, &x.nth}) ok = ok && cudaStreamCreateWithFlags(t, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t *e : {&x.fork, &x.join, &x.nfork, &x.njoin})
+    ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
     cudaGetLastError();
-    if (x.side) cudaStreamDestroy(x.side);
-    if (x.fork) cudaEventDestroy(x.fork);
+    for (cudaStream_t t : {x.side, x.nth})
+      if (t) cudaStreamDestroy(t);
+    for (cudaEvent_t e : {x.fork, x.join, x.nfork, x.njoin})
+      if (e) cudaEventDestroy(e);
     return nullptr;
   }
   C.sides.push_back(x);
@@ -1197,7 +1201,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   if (kind == RELX_XILLVER) {
     if (cp) {
       ProfScope ps(PK_NTH, s);
-      RELX_CUDA(launch_nthcomp(s, tab, sin, sst, n, 1, true, nthq, ntab, nullptr, nullptr, W.nthscr.as<float4>(),
+      RELX_CUDA(launch_nthcomp(s, tab, sin, sst, n, 1, true, nthq, ntab, nullptr, nullptr, nullptr, W.nthscr.as<float4>(),
                                (int64_t) b.n_sets, (int64_t) base));
     }
     {
@@ -1213,10 +1217,23 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     ProfScope ps(PK_SETUP, s);
     RELX_CUDA(launch_setup(s, n, tab, b.model, sin, user_e, W.line_e.as<double>(), sst, rad, cor, zcor));
   }
+  // relxill models: the emission-angle histograms and the xillver zone spectra depend on the set-up
+  // only; they run on a side stream while the line profile runs on s, and s waits for them.  The nthcomp continua
+  // run on a third one from the set-up on: the xillver spectra are the first to need them (all on
+  // s while per-kernel timing is on, so that the kernels' intervals do not overlap)
+  const bool relxill = relx_is_relxill(kind);
+  Context::Side *sd = (relxill && !g_prof.on) ? side_of(C, s) : nullptr;
+  cudaStream_t xs = sd ? sd->side : s;
   if (cp) {  // the nthcomp continua of the source and the zones, their normalisations on the corner weights
     ProfScope ps(PK_NTH, s, 2);
-    RELX_CUDA(launch_nthcomp(s, tab, sin, sst, n, b.nza, false, nthq, ntab, cor, zcor, W.nthscr.as<float4>(),
+    cudaStream_t ns = sd ? sd->nth : s;
+    if (sd) {
+      RELX_CUDA(cudaEventRecord(sd->nfork, s));
+      RELX_CUDA(cudaStreamWaitEvent(ns, sd->nfork, 0));
+    }
+    RELX_CUDA(launch_nthcomp(ns, tab, sin, sst, n, b.nza, false, nthq, ntab, cor, zcor, sflag, W.nthscr.as<float4>(),
                              (int64_t) b.n_sets * (b.nza + 1), (int64_t) base * (b.nza + 1)));
+    if (sd) RELX_CUDA(cudaEventRecord(sd->njoin, ns));
   }
   if (cached) {
     ProfScope ps(PK_SETUP, s, 2);
@@ -1225,15 +1242,9 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     RELX_CUDA(cache_fill(C.cache, s, sst, W.cslot.as<int>() + base, n, b.nza, b.nblk, prof, tsum,
                          dist));
   }
-  // relxill models: the emission-angle histograms and the xillver zone spectra depend on the set-up
-  // only; they run on a side stream while the line profile runs on s, and s waits for them (all on
-  // s while per-kernel timing is on, so that the kernels' intervals do not overlap)
   // the sets' interpolated transfer-function tables (line_table_kernel), then the line profile on
   // s; the histograms and the xillver zone spectra on the side stream after the tables
   float4 *htab = W.htab.as<float4>() + (size_t) base * tab.rel_nr * tab.rel_ng;
-  const bool relxill = relx_is_relxill(kind);
-  Context::Side *sd = (relxill && !g_prof.on) ? side_of(C, s) : nullptr;
-  cudaStream_t xs = sd ? sd->side : s;
   uint2 *list = W.list.as<uint2>() ? W.list.as<uint2>() + line_list_entries(base, b.nza, b.nblk) : nullptr;
   int *cnt = W.err.as<int>() + 4 + 2 * base;  // the range's task counters
   {
@@ -1259,6 +1270,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
       const bool sort = dense && xill_sorted(n);
       ProfScope ps(PK_XILL, xs, (zone ? 1 : 0) + (dense ? 1 : 0) + (sort ? 1 : 0));
       int *order = sort ? W.order.as<int>() + base : nullptr;
+      if (sd && cp) RELX_CUDA(cudaStreamWaitEvent(xs, sd->njoin, 0));
       if (sort) launch_xill_order(xs, sst, cor, zcor, n, order);
       RELX_CUDA(launch_xillver(xs, tab, n, b.nza, zone, dense, sst, cor, zcor, dist, xill, W.err.as<int>(), order));
     }
@@ -1283,7 +1295,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
     {
       ProfScope ps(PK_FIN, s);
-      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, cout, b.nza, user_e, flux, ntab));
+      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, sflag, cout, b.nza, user_e, flux, ntab));
     }
   } else if (kind == RELX_RELCONV) {
     ProfScope ps(PK_CONV, s, kRelconvKernels);
