@@ -1014,33 +1014,69 @@ static int ensure_init(Context &C, const char *path) {
   return 0;
 }
 
-// pack (params, energy offsets) into RelxSetIn on the device
-__global__ void pack_kernel(int n_sets, int npar, const double *__restrict__ params, const int64_t *__restrict__ eoff,
-                            const int *__restrict__ igt, const double *__restrict__ igi, int nzones_env, int flags,
-                            int nza, RelxSetIn *__restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_sets) return;
-  RelxSetIn s;
-  for (int q = 0; q < RELX_NPARAM_MAX; q++) s.p[q] = q < npar ? params[(size_t) i * npar + q] : 0.0;
-  s.e_off = eoff[i];
-  s.n_ener = (int) (eoff[i + 1] - eoff[i] - 1);
-  s.ion_grad_type = igt ? igt[i] : 0;
-  s.iongrad_index = igi ? igi[i] : 0.0;
-  s.nzones_env = nzones_env;
-  s.flags = flags;
-  s.nza = nza;
-  out[i] = s;
+// Takes a batch's inputs from the caller's device buffers or from pinned staging: packs (params, energy offsets)
+// into RelxSetIn, copies the grids (e_src) and relconv's spectra (f_src) where given, and clears the
+// flags and counters.  One kernel for what were three or four copies, a pack kernel and two memsets, each
+// with its own latency on the stream (one xillver set, host buffers: 40 us per call against 54).
+struct StageArgs {
+  int n_sets, npar, nzones_env, flags, nza, n_err;
+  int64_t n_edges;
+  const double *params, *igi, *e_src, *f_src;
+  const int64_t *eoff;
+  const int *igt;
+  RelxSetIn *out;
+  double *e_dst, *f_dst;
+  int *sflag, *err;
+};
+constexpr int kStageThreads = 256;
+__global__ void __launch_bounds__(kStageThreads) stage_kernel(StageArgs a) {
+  const int64_t t = (int64_t) blockIdx.x * kStageThreads + threadIdx.x, stride = (int64_t) gridDim.x * kStageThreads;
+  for (int64_t i = t; i < a.n_sets; i += stride) {
+    RelxSetIn s;
+    for (int q = 0; q < RELX_NPARAM_MAX; q++) s.p[q] = q < a.npar ? a.params[(size_t) i * a.npar + q] : 0.0;
+    s.e_off = a.eoff[i];
+    s.n_ener = (int) (a.eoff[i + 1] - a.eoff[i] - 1);
+    s.ion_grad_type = a.igt ? a.igt[i] : 0;
+    s.iongrad_index = a.igi ? a.igi[i] : 0.0;
+    s.nzones_env = a.nzones_env;
+    s.flags = a.flags;
+    s.nza = a.nza;
+    a.out[i] = s;
+    a.sflag[i] = 0;
+  }
+  for (int64_t i = t; i < a.n_err; i += stride) a.err[i] = 0;
+  if (a.e_src)
+    for (int64_t i = t; i < a.n_edges; i += stride) a.e_dst[i] = a.e_src[i];
+  if (a.f_src)
+    for (int64_t i = t; i < a.n_edges; i += stride) a.f_dst[i] = a.f_src[i];
 }
 
+// a set's status from the set-up, its flag and the batch's error flag; and, where hflux is given, the fluxes and
+// statuses out to (pinned or the caller's) buffers
 __global__ void status_kernel(int n_sets, const RelxSetState *__restrict__ st, const int *__restrict__ sflag,
-                              const int *__restrict__ err, int *__restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_sets) return;
-  int s = st[i].status;
-  if (s == RELX_OK && sflag[i] != RELX_OK) s = sflag[i];
-  if (s == RELX_OK && *err != RELX_OK) s = *err;
-  out[i] = s;
+                              const int *__restrict__ err, int *__restrict__ out, int64_t n_flux,
+                              const double *__restrict__ flux, double *__restrict__ hflux, int *__restrict__ hstatus) {
+  const int64_t t = (int64_t) blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t) gridDim.x * blockDim.x;
+  for (int64_t i = t; i < n_sets; i += stride) {
+    int s = st[i].status;
+    if (s == RELX_OK && sflag[i] != RELX_OK) s = sflag[i];
+    if (s == RELX_OK && *err != RELX_OK) s = *err;
+    out[i] = s;
+    if (hstatus) hstatus[i] = s;
+  }
+  if (hflux)
+    for (int64_t i = t; i < n_flux; i += stride) hflux[i] = flux[i];
 }
+// results to the caller's device buffers
+__global__ void __launch_bounds__(kStageThreads) out_kernel(int64_t n_flux, const double *__restrict__ flux, double *__restrict__ dflux,
+                                                            int n_sets, const int *__restrict__ status, int *__restrict__ dstatus) {
+  const int64_t t = (int64_t) blockIdx.x * kStageThreads + threadIdx.x, stride = (int64_t) gridDim.x * kStageThreads;
+  for (int64_t i = t; i < n_flux; i += stride) dflux[i] = flux[i];
+  if (dstatus)
+    for (int64_t i = t; i < n_sets; i += stride) dstatus[i] = status[i];
+}
+// CTAs for n grid-stride items
+static int stage_ctas(int64_t n) { return (int) std::max<int64_t>(1, std::min<int64_t>((n + kStageThreads - 1) / kStageThreads, 8 * 152)); }
 
 // ---- optional per-kernel timing with CUDA events on the launching stream ----
 enum ProfKernel { PK_PACK, PK_SETUP, PK_LINE, PK_XILL, PK_CONV, PK_FIN, PK_STATUS, PK_NTH, PK_HIST, PK_N };
@@ -1104,6 +1140,9 @@ struct BatchShape {
   int chunk = 0;      // sets per pipelined chunk (0: one range)
   bool any_limb = false;  // some set uses a limb-darkening law (relline / relconv limb parameter)
   int64_t n_edges;  // total energy edges
+  bool cleared = false;       // stage_kernel has cleared the flags and counters for this launch
+  double *hflux = nullptr;    // pinned memory for the results of a small host batch (status_kernel), or null
+  int *hstatus = nullptr;
 };
 
 // the error flag, then the two task counters of the range of sets that starts at a set
@@ -1171,6 +1210,16 @@ static Context::Side *side_of(Context &C, cudaStream_t s) {
   return &C.sides.back();
 }
 
+// the statuses of the sets [base, base + n), and the results of a whole batch to pinned memory (b.hflux)
+static void launch_status(Workspace &W, const BatchShape &b, cudaStream_t s, int base, int n) {
+  ProfScope ps(PK_STATUS, s);
+  const int64_t nflux = b.n_edges - b.n_sets;
+  double *hf = n == b.n_sets ? b.hflux : nullptr;
+  status_kernel<<<stage_ctas(hf ? std::max<int64_t>(n, nflux) : n), kStageThreads, 0, s>>>(
+      n, W.st.as<RelxSetState>() + base, W.sflag.as<int>() + base, W.err.as<int>(), W.status.as<int>() + base, nflux,
+      W.flux.as<double>(), hf, hf ? b.hstatus : nullptr);
+}
+
 // the kernel sequence for one batch; all pointers are device pointers, asynchronous on `s`
 // The kernel sequence for the sets [base, base + n) of a batch, asynchronous on s.  Per-set
 // arrays are addressed from the range's first set; energy grids and fluxes keep the batch's
@@ -1208,8 +1257,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
       ProfScope ps(PK_XILL, s);
       RELX_CUDA(launch_xillver_model(s, tab, n, b.n_edges - b.n_sets, sin, user_e, sst, flux, nthq, ntab));
     }
-    ProfScope ps(PK_STATUS, s);
-    status_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, sst, sflag, W.err.as<int>(), W.status.as<int>() + base);
+    launch_status(W, b, s, base, n);
     RELX_CUDA(cudaGetLastError());
     return 0;
   }
@@ -1306,8 +1354,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, b.nza, flux);
   }
   {
-    ProfScope ps(PK_STATUS, s);
-    status_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, sst, sflag, W.err.as<int>(), W.status.as<int>() + base);
+    launch_status(W, b, s, base, n);
   }
   RELX_CUDA(cudaGetLastError());
   return 0;
@@ -1324,8 +1371,10 @@ static int chunk_sets() {
 // the batch as launched, without graphs
 static int launch_direct(Context &C, Workspace &W, const BatchShape &b, cudaStream_t s, bool cached) {
   const int S = b.n_sets;
-  RELX_CUDA(cudaMemsetAsync(W.sflag.p, 0, S * sizeof(int), s));
-  RELX_CUDA(cudaMemsetAsync(W.err.p, 0, err_bytes(S), s));  // the error flag and the line tasks' counters
+  if (!b.cleared) {
+    RELX_CUDA(cudaMemsetAsync(W.sflag.p, 0, S * sizeof(int), s));
+    RELX_CUDA(cudaMemsetAsync(W.err.p, 0, err_bytes(S), s));  // the error flag and the line tasks' counters
+  }
   const int chunk = b.chunk;
   if (cached || chunk <= 0 || S < 2 * chunk) return launch_range(C, W, b, s, 0, S, cached);
   for (int k = 0; k < 2; k++) {
@@ -1349,7 +1398,8 @@ static int launch_direct(Context &C, Workspace &W, const BatchShape &b, cudaStre
 static std::vector<uintptr_t> graph_key(const Workspace &W, const BatchShape &b) {
   std::vector<uintptr_t> k = {(uintptr_t) b.model, (uintptr_t) b.n_sets, (uintptr_t) b.nza, (uintptr_t) b.nz_min,
                               (uintptr_t) b.nblk, (uintptr_t) b.chunk,
-                              (uintptr_t) b.any_limb, (uintptr_t) b.n_edges};
+                              (uintptr_t) b.any_limb, (uintptr_t) b.n_edges, (uintptr_t) b.cleared,
+                              (uintptr_t) b.hflux, (uintptr_t) b.hstatus};
   for (const DevBuf *d : {&W.setin, &W.st, &W.rad, &W.corners, &W.zcorners, &W.line_e, &W.prof, &W.dist, &W.tsum,
                           &W.xill, &W.cout, &W.user_e, &W.user_f, &W.flux, &W.sflag, &W.status, &W.err, &W.order,
                           &W.htab, &W.list, &W.nthq, &W.nthtab, &W.nthscr})
@@ -1460,6 +1510,7 @@ static int tuned_launch(Context &C, Workspace &W, BatchShape &b, cudaStream_t s,
     C.tune.push_back(Context::TuneEntry{b.model, sclass, b.nza, kLineTileH, 0, {0, 0, 0, 0}});
     return launch_batch(C, W, b, s, use_cache);
   }
+  b.cleared = false;  // the trials launch more than once
   const std::vector<int> cands = {0, 1024};
   cudaEvent_t e0, e1;
   RELX_CUDA(cudaEventCreate(&e0));
@@ -1522,6 +1573,29 @@ static int batch_shape(int model, int n_sets, const int64_t *eoff_host, const in
   return 0;
 }
 
+// bytes of input and results up to which a host batch is small (64 sets of 2000 bins, 2 MB: 214 us against 230 us
+// with copies; above, where the copies of one group run under the kernels of another, no difference was seen)
+constexpr size_t kSmallBatch = 2 << 20;
+
+// the inputs of a (sources and optional ones in a, the rest filled in here); the flags and counters are clear after it
+static void launch_stage(Workspace &W, BatchShape &b, const EnvOpts &env, cudaStream_t s, StageArgs &a) {
+  a.n_sets = b.n_sets;
+  a.npar = model_nparams(b.model);
+  a.nzones_env = env.nzones_env;
+  a.flags = env.flags;
+  a.nza = b.nza;
+  a.n_err = (int) (err_bytes(b.n_sets) / sizeof(int));
+  a.n_edges = b.n_edges;
+  a.out = W.setin.as<RelxSetIn>();
+  a.e_dst = W.user_e.as<double>();
+  a.f_dst = a.f_src ? W.user_f.as<double>() : nullptr;
+  a.sflag = W.sflag.as<int>();
+  a.err = W.err.as<int>();
+  b.cleared = true;
+  ProfScope ps(PK_PACK, s);
+  stage_kernel<<<stage_ctas(a.e_src ? a.n_edges : a.n_err), kStageThreads, 0, s>>>(a);
+}
+
 // Stages the inputs of a host batch through pinned memory, launches the batch and queues the
 // copies of the results (flux, then per-set statuses) back into pinned memory, all asynchronous on
 // s.  *o_flux / *o_status: their offsets in P.  Caller holds C.mu.
@@ -1579,25 +1653,41 @@ static int enqueue_host_batch(Context &C, Workspace &W, Pinned &P, cudaStream_t 
   CopyPool::get().run(jobs);
   *o_flux = put(nullptr, nflux * sizeof(double));
   *o_status = put(nullptr, sizeof(int) * n_sets);
-  if ((st = W.params.reserve(pb)) || (st = W.eoff.reserve(ob)) || (hb.igt && (st = W.igt.reserve(gb))) ||
-      (hb.igi && (st = W.igi.reserve(ib))))
-    return st;
-  RELX_CUDA(cudaMemcpyAsync(W.params.p, h + o_p, pb, cudaMemcpyHostToDevice, s));
-  RELX_CUDA(cudaMemcpyAsync(W.user_e.p, h + o_e, eb, cudaMemcpyHostToDevice, s));
-  RELX_CUDA(cudaMemcpyAsync(W.eoff.p, h + o_o, ob, cudaMemcpyHostToDevice, s));
-  if (hb.igt) RELX_CUDA(cudaMemcpyAsync(W.igt.p, h + o_g, gb, cudaMemcpyHostToDevice, s));
-  if (hb.igi) RELX_CUDA(cudaMemcpyAsync(W.igi.p, h + o_i, ib, cudaMemcpyHostToDevice, s));
-  if (conv) RELX_CUDA(cudaMemcpyAsync(W.user_f.p, h + o_f, fb, cudaMemcpyHostToDevice, s));
-  {
-    ProfScope ps(PK_PACK, s);
-    pack_kernel<<<(n_sets + 127) / 128, 128, 0, s>>>(n_sets, npar, W.params.as<double>(), W.eoff.as<int64_t>(),
-                                                     hb.igt ? W.igt.as<int>() : nullptr,
-                                                     hb.igi ? W.igi.as<double>() : nullptr, env.nzones_env, env.flags,
-                                                     b.nza, W.setin.as<RelxSetIn>());
+  // a small batch's kernels read and write the pinned staging themselves; a large one's inputs and results are
+  // moved by the copy engines
+  const bool small = off <= kSmallBatch && n_sets < 2048 && b.chunk <= 0;  // never split into chunks
+  StageArgs a;
+  a.e_src = a.f_src = nullptr;
+  if (small) {
+    a.params = (const double *) (h + o_p);
+    a.eoff = (const int64_t *) (h + o_o);
+    a.igt = hb.igt ? (const int *) (h + o_g) : nullptr;
+    a.igi = hb.igi ? (const double *) (h + o_i) : nullptr;
+    a.e_src = (const double *) (h + o_e);
+    if (conv) a.f_src = (const double *) (h + o_f);
+    b.hflux = (double *) (h + *o_flux);
+    b.hstatus = (int *) (h + *o_status);
+  } else {
+    if ((st = W.params.reserve(pb)) || (st = W.eoff.reserve(ob)) || (hb.igt && (st = W.igt.reserve(gb))) ||
+        (hb.igi && (st = W.igi.reserve(ib))))
+      return st;
+    RELX_CUDA(cudaMemcpyAsync(W.params.p, h + o_p, pb, cudaMemcpyHostToDevice, s));
+    RELX_CUDA(cudaMemcpyAsync(W.user_e.p, h + o_e, eb, cudaMemcpyHostToDevice, s));
+    RELX_CUDA(cudaMemcpyAsync(W.eoff.p, h + o_o, ob, cudaMemcpyHostToDevice, s));
+    if (hb.igt) RELX_CUDA(cudaMemcpyAsync(W.igt.p, h + o_g, gb, cudaMemcpyHostToDevice, s));
+    if (hb.igi) RELX_CUDA(cudaMemcpyAsync(W.igi.p, h + o_i, ib, cudaMemcpyHostToDevice, s));
+    if (conv) RELX_CUDA(cudaMemcpyAsync(W.user_f.p, h + o_f, fb, cudaMemcpyHostToDevice, s));
+    a.params = W.params.as<double>();
+    a.eoff = W.eoff.as<int64_t>();
+    a.igt = hb.igt ? W.igt.as<int>() : nullptr;
+    a.igi = hb.igi ? W.igi.as<double>() : nullptr;
   }
+  launch_stage(W, b, env, s, a);
   if ((st = tuned_launch(C, W, b, s, use_cache, allow_tune))) return st;
-  RELX_CUDA(cudaMemcpyAsync(h + *o_flux, W.flux.p, nflux * sizeof(double), cudaMemcpyDeviceToHost, s));
-  RELX_CUDA(cudaMemcpyAsync(h + *o_status, W.status.p, sizeof(int) * n_sets, cudaMemcpyDeviceToHost, s));
+  if (!small) {
+    RELX_CUDA(cudaMemcpyAsync(h + *o_flux, W.flux.p, nflux * sizeof(double), cudaMemcpyDeviceToHost, s));
+    RELX_CUDA(cudaMemcpyAsync(h + *o_status, W.status.p, sizeof(int) * n_sets, cudaMemcpyDeviceToHost, s));
+  }
   return 0;
 }
 
@@ -1925,20 +2015,21 @@ int relx_eval_batch_device(int model, int n_sets, const double *d_params, const 
   if ((st = reserve_workspace(C.T, C.W, b, need_zc))) return st;
   cudaStream_t s = stream ? (cudaStream_t) stream : C.stream;
   Workspace &W = C.W;
-  RELX_CUDA(cudaMemcpyAsync(W.user_e.p, d_energy, sizeof(double) * b.n_edges, cudaMemcpyDeviceToDevice, s));
-  if (relx_kind(model) == RELX_RELCONV) {
-    if (!d_flux_in) return RELX_ERR_ARG;
-    RELX_CUDA(cudaMemcpyAsync(W.user_f.p, d_flux_in, sizeof(double) * b.n_edges, cudaMemcpyDeviceToDevice, s));
-  }
-  {
-    ProfScope ps(PK_PACK, s);
-    pack_kernel<<<(n_sets + 127) / 128, 128, 0, s>>>(n_sets, model_nparams(model), d_params, d_energy_offsets,
-                                                     d_ion_grad_type, d_iongrad_index, env.nzones_env, env.flags,
-                                                     b.nza, W.setin.as<RelxSetIn>());
-  }
+  const bool conv = relx_kind(model) == RELX_RELCONV;
+  if (conv && !d_flux_in) return RELX_ERR_ARG;
+  StageArgs a;
+  a.params = d_params;
+  a.eoff = d_energy_offsets;
+  a.igt = d_ion_grad_type;
+  a.igi = d_iongrad_index;
+  a.e_src = d_energy;
+  a.f_src = conv ? d_flux_in : nullptr;
+  launch_stage(W, b, env, s, a);
   if ((st = tuned_launch(C, W, b, s, true))) return st;
-  RELX_CUDA(cudaMemcpyAsync(d_flux, W.flux.p, sizeof(double) * (b.n_edges - n_sets), cudaMemcpyDeviceToDevice, s));
-  if (d_status) RELX_CUDA(cudaMemcpyAsync(d_status, W.status.p, sizeof(int) * n_sets, cudaMemcpyDeviceToDevice, s));
+  const int64_t nflux = b.n_edges - n_sets;
+  out_kernel<<<stage_ctas(nflux), kStageThreads, 0, s>>>(nflux, W.flux.as<double>(), d_flux, n_sets, W.status.as<int>(),
+                                                         d_status);
+  RELX_CUDA(cudaGetLastError());
   return 0;
 }
 
