@@ -252,7 +252,7 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
   NOALLOC_CUDA(launch_line_table(1, nza, s, tab, p.sst, p.htab, p.rad, nullptr, nullptr));
   NOALLOC_CUDA(launch_relline(1, nblk, s, tab, p.sin, p.sst, p.rad, p.line_e, nza, p.prof, p.tsum,
                               kind == RELX_RELLINE || kind == RELX_RELCONV, p.htab, nullptr, nullptr));
-  if (relx_is_relxill(kind)) NOALLOC_CUDA(launch_hist(1, s, tab, p.sst, p.rad, nza, p.dist, nza > 1, p.htab));
+  if (relx_is_relxill(kind)) NOALLOC_CUDA(launch_hist(1, s, tab, p.sst, p.rad, nza, p.dist, p.htab));
   if (relx_is_relxill(kind)) {
     NOALLOC_CUDA(launch_xillver(s, tab, 1, nza, nza > RELX_ZDENSE || cp, true, p.sst, p.cor, p.zcor, p.dist, p.xill,
                                 p.err, nullptr));

@@ -48,7 +48,6 @@ constexpr float kSideBand = 2e-5f;  // grid units within which the side of a g* 
 constexpr float kConvBand = 2e-6f;
 constexpr int kGroup = 8;         // consecutive radii of a zone that a warp integrates side by side
 constexpr int kRadLanes = 32 / kGroup;  // lanes per radius, each with a quarter of the radius's bins
-constexpr int kChunk = 128;       // radius records staged per chunk of the histogram kernel
 static_assert(kSumBinsH == 32, "a profile-sum block is the bins of one warp's sum");
 
 constexpr float kMagic = 12582912.0f;   // 1.5 2^23: x + kMagic holds x rounded to an integer in its low bits
@@ -1193,20 +1192,12 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW) relline_team_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// emission-angle distribution per zone (Relprofile.cpp:908-938), one CTA per set.  The set's
+// emission-angle distribution per zone (Relprofile.cpp:908-938), one CTA per set (few sets: per zone).  The set's
 // (a, mu0)-interpolated transfer functions and emission-angle cosines on all table radii are
 // written once per set by line_table_kernel (which the line profile reads as well) and read
-// through the read-only cache, so that the histogram CTA's shared memory stays small; five CTAs
-// per SM (48 registers: 0.82 -> 0.77 ms per 4096-set step against four; six spill).
+// through the read-only cache.
 // ---------------------------------------------------------------------------
-struct HistSmem {
-  RelxRadRec rec[kChunk];    // radius records of the current chunk
-  float re[kChunk];
-  float lh[kLineWarps][RELX_MAX_INCL][32];  // per-lane histograms, lane fastest (no bank conflicts)
-  float hist[kLineWarps][RELX_MAX_INCL];
-  float gfac[RELX_MAX_NG];   // d_gstar / sqrt(g*(1-g*))
-  float gsf[RELX_MAX_NG];
-};
+constexpr int kHistWarps = 8;  // classes of radii of a zone, each summed by itself
 
 // interpol_a_mu0 (Relprofile.cpp:39-80) of (trff1, trff2, cosne1, cosne2) at every (table radius,
 // g*) of a set, for the line profile and the histogram: grid (chunks of kLineThreads entries, sets).
@@ -1270,7 +1261,6 @@ __global__ void __launch_bounds__(kLineThreads) line_table_kernel(RelxTables tab
   ht[nr * ng + q] =
       make_float2(w00 * a.z + w10 * b.z + w01 * c.z + w11 * d.z, w00 * a.w + w10 * b.w + w01 * c.w + w11 * d.w);
 }
-static_assert(offsetof(HistSmem, rec) % 16 == 0, "radius records are staged as int4 rows");
 
 // FP64 emission-angle cosine of one fine radius, table point g, branch k
 // (interp_lin_2d_float then interp_lin_1d as Relprofile.cpp:67-77, 287-290)
@@ -1289,121 +1279,195 @@ __device__ double cosne_fp64(const RelxTables &tab, const RelxSetState &s, int i
   return lerp1(ifac, v[0], v[1]);
 }
 
-__global__ void __launch_bounds__(kLineThreads, 5) hist_kernel(RelxTables tab, const RelxSetState *__restrict__ sst,
-                                                            const RelxRadial *__restrict__ srad, int nza,
-                                                            const float4 *__restrict__ htab, float *__restrict__ dist) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  HistSmem &m = *reinterpret_cast<HistSmem *>(smem_raw);
-  const int set = blockIdx.x;
-  const RelxSetState &s = sst[set];
-  if (s.status != RELX_OK || s.model < RELX_RELXILL || s.cached || (int) blockIdx.y >= s.nz) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const RelxRadial &R = srad[set];
+// the bin of a cosine so near a bin's edge that FP32 does not decide it (get_cosne_bin, Relprofile.cpp:799-801)
+__device__ __noinline__ int cosne_bin_fp64(const RelxTables &tab, const RelxSetState &s, int itab, double ifac, int g, int k) {
+  const double mud = cosne_fp64(tab, s, itab, ifac, g, k);
+  return ((int) (tab.x_nincl * (1 - mud) + 1)) - 1;
+}
+
+// A zone's radii fall into kHistWarps classes: class w the radii 4 w to 4 w + 3 of every 32 from the zone's start.  A
+// warp takes four radii at a time, 8 lanes per radius, each lane a block of at most GP consecutive table
+// points (gper = (ng + 7) / 8 of them) with both branches.  Consecutive points mostly fall into the same
+// angle bin: a lane adds runs and flushes a run on a change of bin into its private histogram.  At the end of
+// a class the lanes are added by a shuffle tree, and the classes in order.
+// A CTA of kHistWarps warps per zone, a class each (a warp per zone without barriers, eight classes one after
+// the other: 771 us against 681 us for 4096 relxilllp sets).  Bound by issue and the latency of the loads.
+// 4096 sets took 762 us, 1000 relxilllpCp sets 249 us and 64 relxill sets 72 us by a CTA per set with a loop over the
+// points (addresses, integer conversions and a dependent load each, divergent flushes) and records staged in
+// shared memory with two barriers per 128 radii; with the points unrolled, a radius's loads in flight together, the
+// next radius's record fetched ahead and flushes without branches 681 us, 177 us and 35 us.
+constexpr int kHistFull = 5;  // the 40 points of the relline tables, 5 for each of 8 lanes
+
+template <int GP>
+struct HistLane {
+  int g0, np;  // the lane's points
+  float gsf[GP], gfac[GP];
+};
+
+// class w of zone [i0, i1]; the lane's sums end in lh
+template <int GP>
+__device__ __forceinline__ void hist_class(const RelxTables &tab, const RelxSetState &s, const RelxRadial &R,
+                                           const float2 *__restrict__ T, const HistLane<GP> &L, int i0, int i1, int w,
+                                           float *lh) {
+  const int lane = threadIdx.x & 31, grp = lane >> 3;
   const int nr = tab.rel_nr, ng = tab.rel_ng, n_incl = tab.x_nincl;
-  // the set's interpolated table: (trff1, trff2) plane, then (cosne1, cosne2)
-  const float2 *__restrict__ T = reinterpret_cast<const float2 *>(htab + (size_t) set * nr * ng);
-  const float2 *__restrict__ C = T + nr * ng;
-  {
-    for (int g = tid; g < ng; g += kLineThreads) {
-      double gs = 5e-3 + (1.0 - 2 * 5e-3) / (ng - 1) * ((float) g);
-      double gs1 = 5e-3 + (1.0 - 2 * 5e-3) / (ng - 1) * ((float) 1);
-      double dgs = (g == 0 || g == ng - 1) ? 0.5 * (gs1 - 5e-3) + 5e-3 : gs1 - 5e-3;
-      m.gfac[g] = (float) (dgs / sqrt(gs - gs * gs));
-      m.gsf[g] = (float) gs;
-    }
-  }
-  __syncthreads();
-  // Each lane owns (g*, branch) pairs q = lane, lane + 32, ... and keeps a private histogram in
-  // shared memory; at the end of a zone the lanes are added by a shuffle tree and the warps in order.
-  float(*lh)[32] = m.lh[warp];
-  for (int j = 0; j < RELX_MAX_INCL; j++) lh[j][lane] = 0.0f;
   const float c4pi2 = (float) (4.0 * kPi * kPi);
-  const int zb = gridDim.y > 1 ? (int) blockIdx.y : 0, ze = gridDim.y > 1 ? min((int) blockIdx.y + 1, s.nz) : s.nz;
-  for (int z = zb; z < ze; z++) {
-    const int i0 = s.zi0[z], i1 = s.zi1[z];
-    for (int c0 = i0; c0 <= i1; c0 += kChunk) {
-      const int cn = min(kChunk, i1 + 1 - c0);
-      {
-        const int4 *src = reinterpret_cast<const int4 *>(&R.rec[c0]);
-        int4 *dst = reinterpret_cast<int4 *>(m.rec);
-        for (int q = tid; q < cn * 4; q += kLineThreads) dst[q] = src[q];
-        for (int q = tid; q < cn; q += kLineThreads) m.re[q] = (float) R.re[c0 + q];
-      }
-      __syncthreads();
-      // four radii per warp: 8 lanes per radius, each lane takes a block of consecutive table points
-      const int grp = lane >> 3, sub = lane & 7;
-      for (int cb = warp * 4; cb < cn; cb += kLineWarps * 4) {
-        const int ci = cb + grp;
-        if (ci >= cn) continue;
-        const RelxRadRec &rr = m.rec[ci];
-        if (rr.ielo < 0) continue;  // radius outside the line-profile grid (Relprofile.cpp:863)
-        const int it = rr.itab;
-        const float fr = rr.ifac;
-        const float re = m.re[ci];
-        const float c = re * re * re * c4pi2 * rr.ew;
-        const float dg = rr.dg.x, gmn = rr.gmin.x;
-        // consecutive table points mostly fall into the same angle bin: each lane takes a block of
-        // consecutive points, adds runs and flushes a run on a change of bin
-        int cur0 = -1, cur1 = -1;
-        float run0 = 0.0f, run1 = 0.0f;
-        const int gper = (ng + 7) >> 3, g_end = min(ng, (sub + 1) * gper);
-        for (int g = sub * gper; g < g_end; g++) {
-          // trf(g*) and cosne(g*) at this radius: interp_lin_1d(ifac_r, T[ind+1], T[ind]) (Relprofile.cpp:280-293)
-          const float2 lo = __ldg(&T[(it + 1) * ng + g]), hi = __ldg(&T[it * ng + g]);
-          const float2 clo = __ldg(&C[(it + 1) * ng + g]), chi = __ldg(&C[it * ng + g]);
-          const float ge_ = m.gsf[g] * dg + gmn;
-          const float cg = c * ge_ * ge_ * m.gfac[g];
+  const float fn = (float) n_incl;
+  int r = i0 + w * 4 + grp;
+  int4 q3 = make_int4(0, -1, -1, 0);  // ifac, ielo, iehi, itab
+  float gmn = 0.0f, dg = 0.0f, ew = 0.0f, re = 0.0f;
+  const auto fetch = [&](int k) {
+    const RelxRadRec *rp = &R.rec[k];
+    q3 = __ldg(reinterpret_cast<const int4 *>(rp) + 3);
+    gmn = __ldg(&rp->gmin.x);
+    dg = __ldg(&rp->dg.x);
+    ew = __ldg(&rp->ew);
+    re = __ldg(&R.re[k]);
+  };
+  if (r <= i1) fetch(r);
+  for (; i0 + w * 4 <= i1 && __any_sync(0xffffffffu, r <= i1); r += kHistWarps * 4) {
+    const bool on = r <= i1 && q3.y >= 0 && L.np > 0;  // radius inside the line-profile grid (Relprofile.cpp:863)
+    const float fr = __int_as_float(q3.x), fl = 1.0f - fr;
+    const int it = (short) (q3.w & 0xffff);
+    const float c = re * re * re * c4pi2 * ew, dgr = dg, gmr = gmn;
+    const float2 *hi = T + it * ng, *lo = hi + ng, *chi = hi + nr * ng, *clo = lo + nr * ng;
+    // the cosines first, then the transfer functions: half the registers
+    float2 wh[GP], wl[GP];
 #pragma unroll
-          for (int k = 0; k < 2; k++) {
-            const float trf = k ? fr * hi.y + (1.0f - fr) * lo.y : fr * hi.x + (1.0f - fr) * lo.x;
-            const float mu = k ? fr * chi.y + (1.0f - fr) * clo.y : fr * chi.x + (1.0f - fr) * clo.x;
-            const float xb = (float) n_incl * (1.0f - mu);
-            int b;
-            if (fabsf(xb - rintf(xb)) < 1e-5f) {
-              const double mud = cosne_fp64(tab, s, it, R.ifac[c0 + ci], g, k);
-              b = ((int) (n_incl * (1 - mud) + 1)) - 1;  // get_cosne_bin, Relprofile.cpp:799-801
-            } else {
-              b = ((int) (xb + 1.0f)) - 1;
-            }
-            b = max(0, min(b, n_incl - 1));
-            const float term = cg * trf;
-            int &cur = k ? cur1 : cur0;
-            float &run = k ? run1 : run0;
-            if (b != cur) {
-              if (cur >= 0) lh[cur][lane] += run;
-              cur = b;
-              run = 0.0f;
-            }
-            run += term;
-          }
+    for (int e = 0; e < GP; e++) {
+      wh[e] = wl[e] = make_float2(0.0f, 0.0f);
+      if (on && e < L.np) {
+        wh[e] = __ldg(chi + e);
+        wl[e] = __ldg(clo + e);
+      }
+    }
+    if (r + kHistWarps * 4 <= i1) fetch(r + kHistWarps * 4);
+    // trf(g*) and cosne(g*) at this radius: interp_lin_1d(ifac_r, T[ind+1], T[ind]) (Relprofile.cpp:280-293).  The
+    // angle bin is floor(n_incl (1 - cosne)), from the nearest integer to that minus 1/2, by a magic sum whose
+    // low bits hold the integer; FP32 decides it unless the fraction is within 1e-5 of an edge
+    const float wl_ = -fn * fl, wh_ = -fn * fr;
+    int b[GP][2];
+    float edge = 0.0f;
+#pragma unroll
+    for (int e = 0; e < GP; e++) {
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const float x = __fmaf_rn(wh_, k ? wh[e].y : wh[e].x, __fmaf_rn(wl_, k ? wl[e].y : wl[e].x, fn - 0.5f));
+        const float q = __fadd_rn(x, kMagic);
+        edge = fmaxf(edge, fabsf(__fadd_rn(x, -__fadd_rn(q, -kMagic))));
+        b[e][k] = max(kMagicBits, min(__float_as_int(q), kMagicBits + n_incl - 1));
+      }
+    }
+    if (on && edge > 0.5f - 1e-5f) {
+#pragma unroll 1
+      for (int q = 0; q < 2 * L.np; q++) {
+        const int e_ = q >> 1;
+        const float2 h = __ldg(chi + e_), l = __ldg(clo + e_);
+        const float x = __fmaf_rn(wh_, q & 1 ? h.y : h.x, __fmaf_rn(wl_, q & 1 ? l.y : l.x, fn - 0.5f));
+        if (!(fabsf(x - rintf(x)) > 0.5f - 1e-5f)) continue;
+        const int v = kMagicBits + max(0, min(cosne_bin_fp64(tab, s, it, R.ifac[r], L.g0 + e_, q & 1), n_incl - 1));
+#pragma unroll
+        for (int e = 0; e < GP; e++) {
+          if (2 * e == q) b[e][0] = v;
+          if (2 * e + 1 == q) b[e][1] = v;
         }
-        if (cur0 >= 0) lh[cur0][lane] += run0;
-        if (cur1 >= 0) lh[cur1][lane] += run1;
       }
-      __syncthreads();
     }
-    // zone end: lanes by a shuffle tree, warps in order
-    for (int j = 0; j < n_incl; j++) {
-      float v = lh[j][lane];
+    float2 vh[GP], vl[GP];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) m.hist[warp][j] = v;
-      lh[j][lane] = 0.0f;
+    for (int e = 0; e < GP; e++) {
+      vh[e] = vl[e] = make_float2(0.0f, 0.0f);
+      if (on && e < L.np) {
+        vh[e] = __ldg(hi + e);
+        vl[e] = __ldg(lo + e);
+      }
     }
-    __syncthreads();
-    if (tid < n_incl) {
-      float h = 0.0f;
-      for (int w = 0; w < kLineWarps; w++) h += m.hist[w][tid];
-      dist[((size_t) set * nza + z) * RELX_MAX_INCL + tid] = h;
+    // the runs; a lane that has none to flush adds to the row for nothing, which costs less than a branch.  (The
+    // second branch's products are rounded before they are added: the sums are those of the kernel before
+    // this one.)
+    int cur[2] = {b[0][0], b[0][1]};
+    float run[2] = {0.0f, 0.0f};
+    const auto flush = [&](bool f0, bool f1) {
+      float *a0 = lh + (f0 ? cur[0] - kMagicBits : RELX_MAX_INCL) * 32, *a1 = lh + (f1 ? cur[1] - kMagicBits : RELX_MAX_INCL) * 32;
+      const float v0 = *a0 + run[0];
+      float v1 = a1 == a0 ? v0 : *a1;
+      v1 += run[1];
+      *a0 = v0;
+      *a1 = v1;
+    };
+#pragma unroll
+    for (int e = 0; e < GP; e++) {
+      const float ge_ = __fmaf_rn(L.gsf[e], dgr, gmr);
+      const float cg = c * ge_ * ge_ * L.gfac[e];
+      const float t0 = __fmaf_rn(fl, vl[e].x, __fmul_rn(fr, vh[e].x)), t1 = __fmaf_rn(fl, vl[e].y, __fmul_rn(fr, vh[e].y));
+      if (e == 0) {
+        run[0] = __fmul_rn(cg, t0);
+        run[1] = __fmul_rn(cg, t1);
+      } else {
+        const bool in = on && e < L.np;
+        const bool f0 = in && b[e][0] != cur[0], f1 = in && b[e][1] != cur[1];
+        flush(f0, f1);
+        if (GP != kHistFull && !in) continue;
+        run[0] = __fmaf_rn(cg, t0, f0 ? 0.0f : run[0]);
+        run[1] = __fadd_rn(f1 ? 0.0f : run[1], __fmul_rn(cg, t1));
+      }
+      cur[0] = b[e][0];
+      cur[1] = b[e][1];
     }
-    __syncthreads();
+    flush(on, on);
   }
 }
 
-size_t hist_smem_bytes(int nr, int ng) {
-  (void) nr;
-  (void) ng;
-  return sizeof(HistSmem);
+// sums of the lanes' histograms, two bins at a time, one in each half of the warp: lane j returns bin j's
+__device__ __forceinline__ float hist_lanes(float (*lh)[32], int n_incl) {
+  const int lane = threadIdx.x & 31;
+  float h = 0.0f;
+  for (int j = 0; j < n_incl; j += 2) {
+    const float v0 = lh[j][lane], v1 = lh[j + 1][lane];
+    float v = lane < 16 ? v0 : v1;
+    v += __shfl_xor_sync(0xffffffffu, lane < 16 ? v1 : v0, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const float u = __shfl_xor_sync(0xffffffffu, v, 16);
+    if (lane == j) h = lane < 16 ? v : u;
+    if (lane == j + 1) h = lane < 16 ? u : v;
+  }
+  return h;
+}
+
+template <int GP>
+__global__ void __launch_bounds__(kHistWarps * 32, GP == kHistFull ? 3 : 1)
+    hist_kernel(RelxTables tab, const RelxSetState *__restrict__ sst, const RelxRadial *__restrict__ srad, int nza,
+                const float4 *__restrict__ htab, float *__restrict__ dist) {
+  __shared__ float lhs[kHistWarps][RELX_MAX_INCL + 1][32];  // per-lane histograms, lane fastest (no bank conflicts), and a row for nothing
+  __shared__ float hw[kHistWarps][RELX_MAX_INCL];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, z = blockIdx.x, set = blockIdx.y;
+  const RelxSetState &s = sst[set];
+  if (s.status != RELX_OK || s.model < RELX_RELXILL || s.cached || z >= s.nz) return;
+  const int ng = tab.rel_ng, n_incl = tab.x_nincl;
+  HistLane<GP> L;
+  const int gper = GP == kHistFull ? kHistFull : (ng + 7) >> 3;
+  L.g0 = (lane & 7) * gper;
+  L.np = GP == kHistFull ? kHistFull : max(0, min(gper, ng - L.g0));
+#pragma unroll
+  for (int e = 0; e < GP; e++) {
+    const float2 g = __ldg(&tab.rel_gs[min(L.g0 + e, ng - 1)]);
+    L.gsf[e] = g.x;
+    L.gfac[e] = g.y;
+  }
+  // the set's interpolated table: (trff1, trff2) plane, then (cosne1, cosne2)
+  const float2 *__restrict__ T = reinterpret_cast<const float2 *>(htab + (size_t) set * tab.rel_nr * ng) + min(L.g0, ng - 1);
+  float(*lh)[32] = lhs[warp];
+  for (int j = 0; j <= RELX_MAX_INCL; j++) lh[j][lane] = 0.0f;
+  hist_class<GP>(tab, s, srad[set], T, L, s.zi0[z], s.zi1[z], warp, &lh[0][lane]);
+  const float h = hist_lanes(lh, n_incl);
+  if (lane < n_incl) hw[warp][lane] = h;
+  __syncthreads();
+  if (tid < n_incl) {
+    float v = 0.0f;
+    for (int w = 0; w < kHistWarps; w++) v += hw[w][tid];
+    dist[((size_t) set * nza + z) * RELX_MAX_INCL + tid] = v;
+  }
 }
 
 constexpr int kSoloTile = kLineTileH;
@@ -1431,7 +1495,6 @@ cudaError_t relline_set_smem(int nr, int ng) {
   SET((relline_team_kernel<false, kSumBinsH, 16>), line_team_smem<false>(ng, 16))
   SET((relline_team_kernel<true, kSumBinsH, 16>), line_team_smem<true>(ng, 16))
   SET((relline_team_kernel<false, kSumBinsH, 32>), line_team_smem<false>(ng, 32))
-  SET(hist_kernel, hist_smem_bytes(nr, ng))
 #undef SET
   return cudaSuccess;
 }
@@ -1495,9 +1558,12 @@ cudaError_t launch_relline(int n_sets, int nblk, cudaStream_t s, const RelxTable
 }
 
 cudaError_t launch_hist(int n_sets, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
-                        const RelxRadial *srad, int nza, float *dist, bool zsplit, const float4 *htab) {
-  hist_kernel<<<dim3(n_sets, zsplit ? nza : 1), kLineThreads, hist_smem_bytes(tab.rel_nr, tab.rel_ng), s>>>(
-      tab, sst, srad, nza, htab, dist);
+                        const RelxRadial *srad, int nza, float *dist, const float4 *htab) {
+  const dim3 grid(nza, n_sets);
+  if (tab.rel_ng == 8 * kHistFull)
+    hist_kernel<kHistFull><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
+  else
+    hist_kernel<RELX_MAX_NG / 8><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
   return cudaGetLastError();
 }
 

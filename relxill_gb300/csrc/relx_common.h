@@ -95,6 +95,7 @@ struct RelxTables {
   const float *rel_a, *rel_mu0;
   const float *rel_r, *rel_gmin, *rel_gmax;
   const float4 *rel_tc;
+  const float2 *rel_gs;  // per table point: g*, and d_gstar / sqrt(g* (1 - g*)) (Relprofile.cpp:908-938)
   // lamp-post table (reltable.h:51-69): [a][h], [a][rad], [a][h][rad]; del, del_inc stored as |x|
   int lp_na, lp_nh, lp_nrad;
   const float *lp_a, *lp_h, *lp_rad, *lp_intens, *lp_del, *lp_delinc;
@@ -227,7 +228,7 @@ static_assert(sizeof(RelxRadRec) == 64, "radius record is four int4 rows");
 // per-set radial data [RELX_NFRAD] (written by setup, read by the line-profile kernels)
 struct RelxRadial {
   RelxRadRec rec[RELX_NFRAD];
-  double re[RELX_NFRAD];
+  float re[RELX_NFRAD];
   double ifac[RELX_NFRAD];    // FP64 radial factor (emission-angle bin decisions near bin edges)
   float  wt[RELX_NFRAD];      // trapez weight / 2
   // lowest and highest line-profile bin that each group of eight consecutive radii of a zone reaches

@@ -39,7 +39,7 @@ cudaError_t launch_relline(int n_sets, int nblk, cudaStream_t s, const RelxTable
                            double *tsum, bool any_limb, const float4 *htab, const uint2 *list, int *cnt);
 // the emission-angle histograms alone (relxill models), for a launch on its own stream
 cudaError_t launch_hist(int n_sets, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
-                        const RelxRadial *srad, int nza, float *dist, bool zsplit, const float4 *htab);
+                        const RelxRadial *srad, int nza, float *dist, const float4 *htab);
 
 cudaError_t xillver_set_smem(int n_incl);
 // bounded-wait self-test: writes the status of a wait that cannot complete (RELX_ERR_TIMEOUT)

@@ -220,7 +220,7 @@ static int upload(DevBuf &b, const std::vector<T> &v) {
 // ---------------------------------------------------------------------------
 struct Tables {
   RelxTables d{};
-  DevBuf rel_a, rel_mu0, rel_r, rel_gmin, rel_gmax, rel_tc;
+  DevBuf rel_a, rel_mu0, rel_r, rel_gmin, rel_gmax, rel_tc, rel_gs;
   DevBuf lp_a, lp_h, lp_rad, lp_intens, lp_del, lp_delinc;
   // one xillver table: the standard one (x) and the nthcomp one of the Cp models (xcp)
   struct XillBufs {
@@ -237,7 +237,7 @@ struct Tables {
   size_t bytes_total = 0;
   bool loaded = false;
   void release() {
-    for (DevBuf *b : {&rel_a, &rel_mu0, &rel_r, &rel_gmin, &rel_gmax, &rel_tc, &lp_a, &lp_h, &lp_rad, &lp_intens,
+    for (DevBuf *b : {&rel_a, &rel_mu0, &rel_r, &rel_gmin, &rel_gmax, &rel_tc, &rel_gs, &lp_a, &lp_h, &lp_rad, &lp_intens,
                       &lp_del, &lp_delinc, &rr_spin, &rr_rlo, &rr_rhi, &rr_tfr, &rr_g, &conv_e, &conv_eff, &conv_inv_emid, &conv_cf,
                       &conv_cw, &coarse_e, &coarse_t, &nth_grid})
       b->release();
@@ -293,13 +293,21 @@ static int load_relline(const std::string &dir, Tables &T) {
     }
   }
   int st;
+  std::vector<float2> gsv(ng);
+  for (int g = 0; g < ng; g++) {
+    const double step = (1.0 - 2 * 5e-3) / (ng - 1);
+    const double gs = std::fma(step, (double) g, 5e-3), gs1 = step + 5e-3;
+    const double dgs = (g == 0 || g == ng - 1) ? 0.5 * (gs1 - 5e-3) + 5e-3 : gs1 - 5e-3;
+    gsv[g] = make_float2((float) gs, (float) (dgs / std::sqrt(std::fma(-gs, gs, gs))));
+  }
   if ((st = upload(T.rel_a, a)) || (st = upload(T.rel_mu0, mu0)) || (st = upload(T.rel_r, r)) ||
-      (st = upload(T.rel_gmin, gmin)) || (st = upload(T.rel_gmax, gmax)) || (st = upload(T.rel_tc, tc)))
+      (st = upload(T.rel_gmin, gmin)) || (st = upload(T.rel_gmax, gmax)) || (st = upload(T.rel_tc, tc)) || (st = upload(T.rel_gs, gsv)))
     return st;
   T.d.rel_na = na; T.d.rel_nmu0 = nm; T.d.rel_nr = nr; T.d.rel_ng = ng;
   T.d.rel_a = T.rel_a.as<float>(); T.d.rel_mu0 = T.rel_mu0.as<float>();
   T.d.rel_r = T.rel_r.as<float>(); T.d.rel_gmin = T.rel_gmin.as<float>(); T.d.rel_gmax = T.rel_gmax.as<float>();
   T.d.rel_tc = T.rel_tc.as<float4>();
+  T.d.rel_gs = T.rel_gs.as<float2>();
   T.bytes_total += r.size() * 12 + tc.size() * 16;
   return 0;
 }
@@ -1308,7 +1316,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   if (relxill) {
     {
       ProfScope ps(PK_HIST, xs);
-      RELX_CUDA(launch_hist(n, xs, tab, sst, rad, b.nza, dist, b.nza > 1 && n < 2 * 152, htab));
+      RELX_CUDA(launch_hist(n, xs, tab, sst, rad, b.nza, dist, htab));
     }
     {
       // the zone kernel for sets with more than RELX_ZDENSE zones and for 6-parameter sets whose

@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
     const double gmn = fma(ifac, m.dgmin_t[ind], m.gmin_t[ind + 1]);
     const double gmx = fma(ifac, m.dgmax_t[ind], m.gmax_t[ind + 1]);
     const double dg = gmx - gmn;
-    R.re[ii] = r;
+    R.re[ii] = d2f(r);
     R.ifac[ii] = ifac;
     RelxRadRec rr;
     rr.gmin = ff_split(gmn);
