@@ -379,15 +379,27 @@ __global__ void __launch_bounds__(kXillThreads) xillver_zone_kernel(RelxTables t
   if (q * 4 >= len) return;
   const float *src0 = tab.x_cspec + e0 + 4 * q;
   const int nlive = live_s;
-  for (int u = 0; u < U; u++) {
+  // a row's inclinations are fetched while the row before is summed (3 CTAs of 128 threads per SM leave 170 registers
+  // a thread): 500 sets of 25 zones 556 us one row at a time, 480 us so
+  float4 v[NIU], vn[NIU];
+  auto fetch = [&](int u, float4 *x) {
     const float *src = src0 + (size_t) rows[u] * pitch;
-    float4 v[NIU];
 #pragma unroll
     for (int i = 0; i < NIU; i++)
-      if (i < ni) v[i] = __ldg(reinterpret_cast<const float4 *>(src + (size_t) i * pitch));
-    for (int e = first[u + 1]; e < (u + 1 < U ? first[u + 2] : nlive); e++) {
+      if (i < ni) x[i] = __ldg(reinterpret_cast<const float4 *>(src + (size_t) i * pitch));
+  };
+  if (U > 0) fetch(0, vn);
+  for (int u = 0; u < U; u++) {
+#pragma unroll
+    for (int i = 0; i < NIU; i++) v[i] = vn[i];
+    if (u + 1 < U) fetch(u + 1, vn);
+    const int last = u + 1 < U ? first[u + 2] : nlive;
+    for (int e = first[u + 1]; e < last; e++) {
       const int2 en = ent[e];
-      const float *d = &dist[en.x * RELX_MAX_INCL];
+      float d[(NIU + 3) & ~3];
+#pragma unroll
+      for (int i = 0; i < NIU; i += 4)
+        *reinterpret_cast<float4 *>(&d[i]) = *reinterpret_cast<const float4 *>(&dist[en.x * RELX_MAX_INCL + i]);
       const float wz = __int_as_float(en.y);
       float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
