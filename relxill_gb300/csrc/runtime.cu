@@ -1037,6 +1037,19 @@ struct StageArgs {
   int *sflag, *err;
 };
 constexpr int kStageThreads = 256;
+// n doubles, four loads of a thread in flight (8-byte accesses: the callers' arrays need no more alignment)
+__device__ __forceinline__ void copy_doubles(double *__restrict__ dst, const double *__restrict__ src, int64_t n, int64_t t,
+                                             int64_t stride) {
+  int64_t i = t;
+  for (; i + 3 * stride < n; i += 4 * stride) {
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = src[i + k * stride];
+#pragma unroll
+    for (int k = 0; k < 4; k++) dst[i + k * stride] = v[k];
+  }
+  for (; i < n; i += stride) dst[i] = src[i];
+}
 __global__ void __launch_bounds__(kStageThreads) stage_kernel(StageArgs a) {
   const int64_t t = (int64_t) blockIdx.x * kStageThreads + threadIdx.x, stride = (int64_t) gridDim.x * kStageThreads;
   for (int64_t i = t; i < a.n_sets; i += stride) {
@@ -1053,10 +1066,8 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(StageArgs a) {
     a.sflag[i] = 0;
   }
   for (int64_t i = t; i < a.n_err; i += stride) a.err[i] = 0;
-  if (a.e_src)
-    for (int64_t i = t; i < a.n_edges; i += stride) a.e_dst[i] = a.e_src[i];
-  if (a.f_src)
-    for (int64_t i = t; i < a.n_edges; i += stride) a.f_dst[i] = a.f_src[i];
+  if (a.e_src) copy_doubles(a.e_dst, a.e_src, a.n_edges, t, stride);
+  if (a.f_src) copy_doubles(a.f_dst, a.f_src, a.n_edges, t, stride);
 }
 
 // a set's status from the set-up, its flag and the batch's error flag; and, where hflux is given, the fluxes and
@@ -1072,14 +1083,13 @@ __global__ void status_kernel(int n_sets, const RelxSetState *__restrict__ st, c
     out[i] = s;
     if (hstatus) hstatus[i] = s;
   }
-  if (hflux)
-    for (int64_t i = t; i < n_flux; i += stride) hflux[i] = flux[i];
+  if (hflux) copy_doubles(hflux, flux, n_flux, t, stride);
 }
 // results to the caller's device buffers
 __global__ void __launch_bounds__(kStageThreads) out_kernel(int64_t n_flux, const double *__restrict__ flux, double *__restrict__ dflux,
                                                             int n_sets, const int *__restrict__ status, int *__restrict__ dstatus) {
   const int64_t t = (int64_t) blockIdx.x * kStageThreads + threadIdx.x, stride = (int64_t) gridDim.x * kStageThreads;
-  for (int64_t i = t; i < n_flux; i += stride) dflux[i] = flux[i];
+  copy_doubles(dflux, flux, n_flux, t, stride);
   if (dstatus)
     for (int64_t i = t; i < n_sets; i += stride) dstatus[i] = status[i];
 }
