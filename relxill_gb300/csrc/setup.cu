@@ -379,23 +379,18 @@ __device__ __forceinline__ float2 rrad_corr_coef(float cg) {
   return make_float2(al, 1.0f - al);
 }
 
-// corrected_gshift_fluxboost_factor / g (Relreturn_Corona.cpp:37-86), FP32; ab from rrad_corr_coef(cg)
-__device__ __forceinline__ float rrad_corrected_boost_over_g(float cg, float2 ab, float g, float lg, float gamma) {
-  float gc;
-  if (cg < 1.0f) {
-    if (g >= 1.0f) {
-      const float ig = 1.0f / g;
-      gc = ig * (ig * ab.x + ab.y);
-    } else {
-      gc = g * (g * ab.x + ab.y);
-    }
-  } else {
-    gc = (g >= 1.0f) ? (1.0f / g * ab.x + ab.y) : (g * ab.x + ab.y);
-  }
+// corrected_gshift_fluxboost_factor / g (Relreturn_Corona.cpp:37-86), FP32; ab from rrad_corr_coef(cg), ig = 1 / g
+// rounded to nearest.  The quotient by g from ig and one exact remainder, which rounds correctly (Markstein,
+// IBM J. Res. Dev. 34, 1990): the divisions by g were most of the pass
+__device__ __forceinline__ float rrad_corrected_boost_over_g(float cg, float2 ab, float g, float lg, float ig, float gamma) {
+  const float x = g >= 1.0f ? ig : g;
+  const float lin = __fmaf_rn(x, ab.x, ab.y);
+  const float gc = cg < 1.0f ? x * lin : lin;
   float fb = exp2f(gamma * lg) * gc;
   if (g < 1.0f && fb > 1.0f) fb = 1.0f;
   if (fb < 0.0f) fb = 0.0f;
-  return fb / g;
+  const float q = __fmul_rn(fb, ig);
+  return __fmaf_rn(__fmaf_rn(-q, g, fb), ig, q);
 }
 
 // calc_rrad_emis_corona (Relreturn_Corona.cpp:125-160) on the table bins: er[i] = sum_j
@@ -405,7 +400,7 @@ __device__ __forceinline__ float rrad_corrected_boost_over_g(float cg, float2 ab
 // the emitting bins, FP32, a fixed reduction order.
 template <int NT>
 __device__ void rrad_pass(const RelxTables &tab, RradSmem &q, float gamma, bool corr) {
-  const int NR = RELX_RR_NR, NG = RELX_RR_NG;
+  constexpr int NR = RELX_RR_NR, NG = RELX_RR_NG;
   const int n = q.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double *tfr = tab.rr_tfr + (size_t) q.spin * NR * NR;
   const float4 *gt = tab.rr_g + (size_t) q.spin * NR * NR * NG;
@@ -422,13 +417,29 @@ __device__ void rrad_pass(const RelxTables &tab, RradSmem &q, float gamma, bool 
       const float cg = corr ? q.cg_f[j] : 1.0f;
       const float2 ab = rrad_corr_coef(cg);
       float h = 0.0f;
-#pragma unroll 5
-      for (int k = 0; k < NG; k++) {
-        const float4 v = __ldg(g + (size_t) k * NR);  // frac_g, g, log2 g, |g - 1| > 1e-3
-        float e = v.x;
-        if (use_corr) e *= rrad_corrected_boost_over_g(cg, ab, v.y, v.z, gamma);
-        else if (v.w != 0.0f) e *= exp2f((gamma - 1.0f) * v.z);
-        h += e;
+      // five samples summed while the next five are fetched
+      constexpr int kBatch = 5;
+      static_assert(NG % kBatch == 0, "samples of a pair of bins");
+      float4 nx[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; k++) nx[k] = __ldg(g + (size_t) k * NR);
+#pragma unroll 1
+      for (int k0 = 0; k0 < NG; k0 += kBatch) {
+        float4 cu[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) cu[k] = nx[k];
+        if (k0 + kBatch < NG) {
+#pragma unroll
+          for (int k = 0; k < kBatch; k++) nx[k] = __ldg(g + (size_t) (k0 + kBatch + k) * NR);
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) {
+          const float4 v = cu[k];  // frac_g, g, log2 g, 1 / g (negative where |g - 1| <= 1e-3)
+          float e = v.x;
+          if (use_corr) e *= rrad_corrected_boost_over_g(cg, ab, v.y, v.z, fabsf(v.w), gamma);
+          else if (v.w > 0.0f) e *= exp2f((gamma - 1.0f) * v.z);
+          h += e;
+        }
       }
       acc += h * d2f(t) * q.emis_in[j];
     }
