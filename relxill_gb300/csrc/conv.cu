@@ -497,11 +497,10 @@ struct FinSmem {
 template <int NT>
 __global__ void __launch_bounds__(NT) finalize_relxill_kernel(RelxTables tab, const RelxSetIn *__restrict__ sin,
                                                                         const RelxSetState *__restrict__ sst,
-                                                                        const int *__restrict__ sflag,
                                                                         const float *__restrict__ cout, int nza,
                                                                         const double *__restrict__ user_e,
                                                                         double *__restrict__ flux,
-                                                                        const NthTable *__restrict__ nth) {
+                                                                        const NthTable *__restrict__ nth, StatusOut so) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FinSmem &m = *reinterpret_cast<FinSmem *>(smem_raw);
   const int set = blockIdx.x, tid = threadIdx.x;
@@ -510,7 +509,8 @@ __global__ void __launch_bounds__(NT) finalize_relxill_kernel(RelxTables tab, co
   const int nu = in.n_ener;
   double *fo = flux + in.e_off - set;  // flux offsets: e_off counts n+1 edges per set
   const int2 part = out_range(nu);
-  const bool bad = s.status != RELX_OK || sflag[set] != RELX_OK;
+  if (tid == 0 && blockIdx.y == 0) put_status(so, set, s.status);
+  const bool bad = s.status != RELX_OK || so.sflag[set] != RELX_OK;
   if (bad || s.model < RELX_RELXILL) {
     if (s.model != RELX_RELCONV || bad)
       for (int i = part.x + tid; i < part.y; i += NT) fo[i] = 0.0;
@@ -583,16 +583,16 @@ __global__ void __launch_bounds__(kFinThreads) finalize_relconv_kernel(RelxTable
                                                                         const RelxSetState *__restrict__ sst,
                                                                         const float *__restrict__ cout, int nza,
                                                                         const double *__restrict__ user_e,
-                                                                        const int *__restrict__ sflag,
-                                                                        double *__restrict__ flux) {
+                                                                        double *__restrict__ flux, StatusOut so) {
   const int set = blockIdx.x, tid = threadIdx.x;
   const RelxSetState &s = sst[set];
   const RelxSetIn &in = sin[set];
+  if (tid == 0 && blockIdx.y == 0) put_status(so, set, s.status);
   if (s.model != RELX_RELCONV) return;
   const int nu = in.n_ener;
   double *fo = flux + in.e_off - set;
   const int2 part = out_range(nu);
-  if (s.status != RELX_OK || sflag[set] != RELX_OK) {
+  if (s.status != RELX_OK || so.sflag[set] != RELX_OK) {
     for (int i = part.x + tid; i < part.y; i += kFinThreads) fo[i] = 0.0;
     return;
   }
@@ -610,10 +610,11 @@ __global__ void __launch_bounds__(kFinThreads) finalize_relline_kernel(const Rel
                                                                         const RelxSetState *__restrict__ sst,
                                                                         const float *__restrict__ prof,
                                                                         const double *__restrict__ tsum, int nblk, int nza,
-                                                                        double *__restrict__ flux) {
+                                                                        double *__restrict__ flux, StatusOut so) {
   const int set = blockIdx.x, tid = threadIdx.x;
   const RelxSetState &s = sst[set];
   const RelxSetIn &in = sin[set];
+  if (tid == 0) put_status(so, set, s.status);
   if (s.model != RELX_RELLINE) return;
   const int nu = in.n_ener;
   double *fo = flux + in.e_off - set;
@@ -648,12 +649,12 @@ cudaError_t relconv_set_smem() {
 cudaError_t launch_relconv(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
                            const RelxSetState *sst, const float *prof, const double *tsum, int nblk, int nza,
                            const double *user_e, const double *user_f, float *xs, float *cout, int *sflag, int *err,
-                           double *flux) {
+                           double *flux, const StatusOut &so) {
   relconv_rebin_kernel<<<dim3(n_sets, kN / kConvThreads), kConvThreads, 0, s>>>(tab, sin, sst, user_e, user_f, xs);
   relconv_conv_kernel<<<n_sets, kConvThreads, sizeof(ConvSmem), s>>>(tab, sin, sst, prof, tsum, nblk, nza, user_f, xs,
                                                                      cout, sflag, err);
   finalize_relconv_kernel<<<dim3(n_sets, out_parts(n_sets, n_bins, kFinThreads, 608)), kFinThreads, 0, s>>>(
-      tab, sin, sst, cout, nza, user_e, sflag, flux);
+      tab, sin, sst, cout, nza, user_e, flux, so);
   return cudaGetLastError();
 }
 
@@ -664,15 +665,13 @@ static_assert(4 * (sizeof(ConvSmem) + 1024) <= 228 * 1024, "four CTAs per SM");
 // 12 us); otherwise a CTA of 128 per set.
 // Every output is computed by one thread with the same arithmetic, so both give the same numbers.
 cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_t n_bins, const RelxTables &tab,
-                                    const RelxSetIn *sin, const RelxSetState *sst, const int *sflag,
-                                    const float *cout, int nza,
-                                    const double *user_e, double *flux, const NthTable *nth) {
+                                    const RelxSetIn *sin, const RelxSetState *sst, const float *cout, int nza,
+                                    const double *user_e, double *flux, const NthTable *nth, const StatusOut &so) {
   if (n_sets <= 0) return cudaSuccess;
   if (few)
-    finalize_relxill_kernel<512><<<dim3(n_sets, out_parts(n_sets, n_bins, 512, 304)), 512, sizeof(FinSmem), s>>>(tab, sin, sst, sflag, cout, nza, user_e, flux, nth);
+    finalize_relxill_kernel<512><<<dim3(n_sets, out_parts(n_sets, n_bins, 512, 304)), 512, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e, flux, nth, so);
   else
-    finalize_relxill_kernel<kFinThreads><<<n_sets, kFinThreads, sizeof(FinSmem), s>>>(tab, sin, sst, sflag, cout, nza, user_e,
-                                                                                     flux, nth);
+    finalize_relxill_kernel<kFinThreads><<<n_sets, kFinThreads, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e, flux, nth, so);
   return cudaGetLastError();
 }
 

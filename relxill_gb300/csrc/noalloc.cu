@@ -238,10 +238,11 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
 
   noalloc_pack_kernel<<<1, 32, 0, s>>>(runtime_nparams(model), d_params, n_bins, ion_grad_type, iongrad_index,
                                        nzones_env, flags, nza, p.sin, p.sflag, p.err);
+  const StatusOut so{p.sflag, p.err, nullptr, nullptr};  // noalloc_status_kernel writes it
   if (kind == RELX_XILLVER) {
     if (cp) NOALLOC_CUDA(launch_nthcomp(s, tab, p.sin, p.sst, 1, 1, true, p.nthq, p.nth, nullptr, nullptr, nullptr, p.nthscr, 1, 0));
     NOALLOC_CUDA(launch_xillver_model(s, tab, 1, n_bins, p.sin, d_energy, p.sst, d_flux, cp ? p.nthq : nullptr,
-                                      cp ? p.nth : nullptr));
+                                      cp ? p.nth : nullptr, so));
     noalloc_status_kernel<<<1, 32, 0, s>>>(p.sst, p.sflag, p.err, p.status, d_status);
     NOALLOC_CUDA(cudaGetLastError());
     runtime_set_error(RELX_OK, "");
@@ -258,14 +259,14 @@ static int eval_one_noalloc(int model, const double *d_params, const double *d_e
                                 p.err, nullptr));
     conv_zone_kernel<<<dim3(nza, 1), kConvThreadsH, conv_smem_bytes(), s>>>(tab, p.sst, p.prof, p.tsum, nblk, p.xill, nza, p.cout,
                                                                             p.err);
-    NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, n_bins, tab, p.sin, p.sst, p.sflag, p.cout, nza, d_energy, d_flux,
-                                         cp ? p.nth : nullptr));
+    NOALLOC_CUDA(launch_finalize_relxill(s, true, 1, n_bins, tab, p.sin, p.sst, p.cout, nza, d_energy, d_flux,
+                                         cp ? p.nth : nullptr, so));
   } else if (kind == RELX_RELCONV) {
     NOALLOC_CUDA(launch_relconv(s, tab, 1, n_bins, p.sin, p.sst, p.prof, p.tsum, nblk, nza, d_energy, d_flux_in, p.xill,
-                                p.cout, p.sflag, p.err, d_flux));
+                                p.cout, p.sflag, p.err, d_flux, so));
   } else {
     finalize_relline_kernel<<<1, kFinThreadsH, 0, s>>>(p.sin, p.sst, p.prof, p.tsum, nblk, nza,
-                                                        d_flux);
+                                                        d_flux, so);
   }
   noalloc_status_kernel<<<1, 32, 0, s>>>(p.sst, p.sflag, p.err, p.status, d_status);
   NOALLOC_CUDA(cudaGetLastError());

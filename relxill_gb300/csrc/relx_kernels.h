@@ -93,6 +93,22 @@ cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetI
                            int nza, bool params, double *q, NthTable *tabs, RelxCorners *cor, RelxZoneCorners *zcor, int *sflag,
                            float4 *scr, int64_t ncont_all, int64_t c_off);
 
+// A set's status, from the set-up, its flag and the batch's error flag: written by the last kernel of a set, to
+// status and, where given, to pinned memory (host).  A kernel of its own for it was 3 us of every call.
+struct StatusOut {
+  const int *sflag, *err;
+  int *status, *host;  // status null: not here
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void put_status(const StatusOut &o, int set, int st) {
+  if (!o.status) return;
+  if (st == RELX_OK && o.sflag[set] != RELX_OK) st = o.sflag[set];
+  if (st == RELX_OK && *o.err != RELX_OK) st = *o.err;
+  o.status[set] = st;
+  if (o.host) o.host[set] = st;
+}
+#endif
+
 // the xillver model: one CTA per set, writes the flux and the status fields of the set state
 size_t xillver_model_smem_bytes(int n_ener, int n_ener_pad);
 cudaError_t xillver_model_set_smem(int n_ener, int n_ener_pad);
@@ -100,7 +116,7 @@ cudaError_t xillver_model_set_smem(int n_ener, int n_ener_pad);
 // n_bins: the output bins of all sets
 cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
                                  const double *user_e, RelxSetState *sst, double *flux, const double *nthq,
-                                 const NthTable *nth);
+                                 const NthTable *nth, const StatusOut &so);
 
 __global__ void conv_zone_kernel(RelxTables tab, const RelxSetState *sst, const float *prof, const double *tsum,
                                  int nblk, const float *xill, int nza, float *cout, int *err);
@@ -110,13 +126,12 @@ cudaError_t relconv_set_smem();
 cudaError_t launch_relconv(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
                            const RelxSetState *sst, const float *prof, const double *tsum, int nblk, int nza,
                            const double *user_e, const double *user_f, float *xs, float *cout, int *sflag, int *err,
-                           double *flux);
+                           double *flux, const StatusOut &so);
 // nth: the nthcomp tables of the sets (Cp models), or null
-// zone sum, primary continuum and rebin to the caller's grid; few: 512 threads per CTA and few_parts CTAs per set
+// zone sum, primary continuum and rebin to the caller's grid; few: 512 threads per CTA and out_parts CTAs per set
 cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_t n_bins, const RelxTables &tab,
-                                    const RelxSetIn *sin, const RelxSetState *sst, const int *sflag,
-                                    const float *cout, int nza,
-                                    const double *user_e, double *flux, const NthTable *nth);
+                                    const RelxSetIn *sin, const RelxSetState *sst, const float *cout, int nza,
+                                    const double *user_e, double *flux, const NthTable *nth, const StatusOut &so);
 // CTAs per set for the output bins of few sets: about `per` bins of a mean set each, and at most `ctas` in all (as
 // many as run at once: 64 xillver sets in 256 CTAs of 1024 threads 31 us, in 128 CTAs 25 us).
 // Every bin is computed by one thread with the same arithmetic, so any split gives the same numbers.
@@ -131,6 +146,6 @@ __device__ __forceinline__ int2 out_range(int n) {
 }
 #endif
 __global__ void finalize_relline_kernel(const RelxSetIn *sin, const RelxSetState *sst, const float *prof,
-                                        const double *tsum, int nblk, int nza, double *flux);
+                                        const double *tsum, int nblk, int nza, double *flux, StatusOut so);
 
 }  // namespace relx

@@ -1070,21 +1070,6 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(StageArgs a) {
   if (a.f_src) copy_doubles(a.f_dst, a.f_src, a.n_edges, t, stride);
 }
 
-// a set's status from the set-up, its flag and the batch's error flag; and, where hflux is given, the fluxes and
-// statuses out to (pinned or the caller's) buffers
-__global__ void status_kernel(int n_sets, const RelxSetState *__restrict__ st, const int *__restrict__ sflag,
-                              const int *__restrict__ err, int *__restrict__ out, int64_t n_flux,
-                              const double *__restrict__ flux, double *__restrict__ hflux, int *__restrict__ hstatus) {
-  const int64_t t = (int64_t) blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t) gridDim.x * blockDim.x;
-  for (int64_t i = t; i < n_sets; i += stride) {
-    int s = st[i].status;
-    if (s == RELX_OK && sflag[i] != RELX_OK) s = sflag[i];
-    if (s == RELX_OK && *err != RELX_OK) s = *err;
-    out[i] = s;
-    if (hstatus) hstatus[i] = s;
-  }
-  if (hflux) copy_doubles(hflux, flux, n_flux, t, stride);
-}
 // results to the caller's device buffers
 __global__ void __launch_bounds__(kStageThreads) out_kernel(int64_t n_flux, const double *__restrict__ flux, double *__restrict__ dflux,
                                                             int n_sets, const int *__restrict__ status, int *__restrict__ dstatus) {
@@ -1159,7 +1144,7 @@ struct BatchShape {
   bool any_limb = false;  // some set uses a limb-darkening law (relline / relconv limb parameter)
   int64_t n_edges;  // total energy edges
   bool cleared = false;       // stage_kernel has cleared the flags and counters for this launch
-  double *hflux = nullptr;    // pinned memory for the results of a small host batch (status_kernel), or null
+  double *hflux = nullptr;    // pinned memory for the results of a small host batch, or null
   int *hstatus = nullptr;
 };
 
@@ -1228,16 +1213,6 @@ static Context::Side *side_of(Context &C, cudaStream_t s) {
   return &C.sides.back();
 }
 
-// the statuses of the sets [base, base + n), and the results of a whole batch to pinned memory (b.hflux)
-static void launch_status(Workspace &W, const BatchShape &b, cudaStream_t s, int base, int n) {
-  ProfScope ps(PK_STATUS, s);
-  const int64_t nflux = b.n_edges - b.n_sets;
-  double *hf = n == b.n_sets ? b.hflux : nullptr;
-  status_kernel<<<stage_ctas(hf ? std::max<int64_t>(n, nflux) : n), kStageThreads, 0, s>>>(
-      n, W.st.as<RelxSetState>() + base, W.sflag.as<int>() + base, W.err.as<int>(), W.status.as<int>() + base, nflux,
-      W.flux.as<double>(), hf, hf ? b.hstatus : nullptr);
-}
-
 // the kernel sequence for one batch; all pointers are device pointers, asynchronous on `s`
 // The kernel sequence for the sets [base, base + n) of a batch, asynchronous on s.  Per-set
 // arrays are addressed from the range's first set; energy grids and fluxes keep the batch's
@@ -1263,7 +1238,9 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
   float *xill = W.xill.p ? W.xill.as<float>() + (size_t) base * xset : nullptr;
   float *cout = W.cout.p ? W.cout.as<float>() + (size_t) base * nza * RELX_NCONV : nullptr;
   int *sflag = W.sflag.as<int>() + base;
-  double *flux = W.flux.as<double>() - base;  // kernels address set i at e_off(i) - i
+  // kernels address set i at e_off(i) - i; a small host batch's results go to pinned memory (never split into ranges)
+  double *flux = b.hflux ? b.hflux : W.flux.as<double>() - base;
+  const StatusOut so{sflag, W.err.as<int>(), W.status.as<int>() + base, b.hstatus};
   const double *user_e = W.user_e.as<double>();
   if (kind == RELX_XILLVER) {
     if (cp) {
@@ -1273,9 +1250,8 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
     {
       ProfScope ps(PK_XILL, s);
-      RELX_CUDA(launch_xillver_model(s, tab, n, b.n_edges - b.n_sets, sin, user_e, sst, flux, nthq, ntab));
+      RELX_CUDA(launch_xillver_model(s, tab, n, b.n_edges - b.n_sets, sin, user_e, sst, flux, nthq, ntab, so));
     }
-    launch_status(W, b, s, base, n);
     RELX_CUDA(cudaGetLastError());
     return 0;
   }
@@ -1361,18 +1337,15 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
     {
       ProfScope ps(PK_FIN, s);
-      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, sflag, cout, b.nza, user_e, flux, ntab));
+      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, cout, b.nza, user_e, flux, ntab, so));
     }
   } else if (kind == RELX_RELCONV) {
     ProfScope ps(PK_CONV, s, kRelconvKernels);
     RELX_CUDA(launch_relconv(s, tab, n, b.n_edges - b.n_sets, sin, sst, prof, tsum, b.nblk, b.nza, user_e,
-                             W.user_f.as<double>(), xill, cout, sflag, W.err.as<int>(), flux));
+                             W.user_f.as<double>(), xill, cout, sflag, W.err.as<int>(), flux, so));
   } else {
     ProfScope ps(PK_FIN, s);
-    finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, b.nza, flux);
-  }
-  {
-    launch_status(W, b, s, base, n);
+    finalize_relline_kernel<<<n, kFinThreadsH, 0, s>>>(sin, sst, prof, tsum, b.nblk, b.nza, flux, so);
   }
   RELX_CUDA(cudaGetLastError());
   return 0;
@@ -2045,8 +2018,11 @@ int relx_eval_batch_device(int model, int n_sets, const double *d_params, const 
   launch_stage(W, b, env, s, a);
   if ((st = tuned_launch(C, W, b, s, true))) return st;
   const int64_t nflux = b.n_edges - n_sets;
-  out_kernel<<<stage_ctas(nflux), kStageThreads, 0, s>>>(nflux, W.flux.as<double>(), d_flux, n_sets, W.status.as<int>(),
-                                                         d_status);
+  {
+    ProfScope ps(PK_STATUS, s);
+    out_kernel<<<stage_ctas(nflux), kStageThreads, 0, s>>>(nflux, W.flux.as<double>(), d_flux, n_sets, W.status.as<int>(),
+                                                           d_status);
+  }
   RELX_CUDA(cudaGetLastError());
   return 0;
 }

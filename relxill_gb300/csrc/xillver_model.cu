@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(NT) xillver_model_kernel(RelxTables tab, const
                                                                       RelxSetState *__restrict__ sst,
                                                                       double *__restrict__ flux,
                                                                       const double *__restrict__ nthq,
-                                                                      const NthTable *__restrict__ nth) {
+                                                                      const NthTable *__restrict__ nth, StatusOut so) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n0 = tab.x_nener, pad = tab.x_nener_pad;
   float *spec = reinterpret_cast<float *>(smem_raw);                    // [pad]
@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(NT) xillver_model_kernel(RelxTables tab, const
   if (tid == 0 && blockIdx.y == 0) {  // the fields the status pass and the statistics read
     RelxSetState &s = sst[set];
     s.status = ok ? RELX_OK : RELX_ERR_PARAM;
+    put_status(so, set, s.status);
     s.model = RELX_XILLVER;
     s.pmodel = cp ? RELX_XILLVERCP : RELX_XILLVER;
     s.prim = cp ? 1 : 0;
@@ -262,16 +263,16 @@ cudaError_t xillver_model_set_smem(int n_ener, int n_ener_pad) {
 
 cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_sets, int64_t n_bins, const RelxSetIn *sin,
                                  const double *user_e, RelxSetState *sst, double *flux, const double *nthq,
-                                 const NthTable *nth) {
+                                 const NthTable *nth, const StatusOut &so) {
   if (n_sets <= 0) return cudaSuccess;
   const size_t smem = xillver_model_smem_bytes(tab.x_nener, tab.x_nener_pad);
   // a CTA of 1024 threads per SM while that takes one wave (152 sets 29 us, with 256 threads 39 us; 200 sets 43 us
   // and 47 us, 608 sets 89 us and 76 us), their output bins spread over the idle SMs (one set of 3000
   // bins 41 us by one CTA, 17 us by 12: the rebin's FP64 instructions hold an SM's pipe 16 cycles each)
   if (n_sets <= 152)
-    xillver_model_kernel<1024><<<dim3(n_sets, out_parts(n_sets, n_bins, 256, 152)), 1024, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth);
+    xillver_model_kernel<1024><<<dim3(n_sets, out_parts(n_sets, n_bins, 256, 152)), 1024, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth, so);
   else
-    xillver_model_kernel<256><<<n_sets, 256, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth);
+    xillver_model_kernel<256><<<n_sets, 256, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth, so);
   return cudaGetLastError();
 }
 
