@@ -37,8 +37,8 @@ sys.path.insert(0, ROOT)
 METRIC = "relxilllp spectra/s batched vs plain GPU at ≤1e-4 rel err; serve p50/p99 ms"
 N_SETS = 4096
 # DRAM bytes (read + write) of one step's line-profile launches over the 4096-set workload (ncu, one-pass
-# capture): the per-set interpolated table (line_table_kernel) and the line profile (relline_kernel)
-LINE_DRAM_BYTES_4096 = (33.64e6 + 205.33e6) + (391.13e6 + 561.29e6)
+# capture): the per-set interpolated table (line_table_kernel) and the line profile (relline_solo_kernel)
+LINE_DRAM_BYTES_4096 = (330.19e6 + 241.19e6) + (410.45e6 + 31.69e6)
 WORKLOAD = ("relxilllp batched, 4096 sets per GPU, per-set grids 300-5000 log bins 0.3-80 keV, "
             "10 radial zones")
 N_PROF = 9  # kernel kinds of the per-kernel event profiler (relx_profile_name)
@@ -656,7 +656,7 @@ def run_gpu(args):
     fp32 = ctypes.c_double(0.0)
     fp32_gflops = fp32.value if L.relx_fp32_rate(ctypes.byref(fp32)) == 0 else None
     line_ms = per["relline"][0]
-    roof = {"kernel": "relline", "launches": ["line_table_kernel", "relline_kernel"], "bound": "fp32",
+    roof = {"kernel": "relline", "launches": ["line_table_kernel", "relline_solo_kernel"], "bound": "fp32",
             "achieved": None, "peak": None, "unit": "TFLOP/s", "frac": None,
             "traffic": None, "peak_source": "measured FP32 FMA rate (relx_fp32_rate, CUDA events)"}
     if evals_per_set is not None and fp32_gflops:
@@ -669,7 +669,7 @@ def run_gpu(args):
     # the one-pass ncu capture in the profiles folder (dram_traffic_relxilllp_4096sets.md); other batch
     # sizes are scaled by their set count
     roof["traffic"] = LINE_DRAM_BYTES_4096 * S / 4096
-    roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of line_table_kernel and relline_kernel, "
+    roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of line_table_kernel and relline_solo_kernel, "
                               "4096-set launch, scaled by sets")
     ng, nr_tab = 40, 100
     line_bytes = (S * (4 * nr_tab * ng * 16 + nr_tab * ng * 16 + nr_tab * ng * 8 + 1000 * 64) +

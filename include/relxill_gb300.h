@@ -137,7 +137,7 @@ int relx_eval_batch_device(int model, int n_sets, const double *d_params, const 
  * evaluate (memory owned by another framework's caching allocator, a fixed
  * memory budget, or a loop where cudaMalloc/cudaFree would stall other
  * streams).  Intermediate arrays live in one static device array of about
- * 3.8 MB shared by all calls: calls whose device work overlaps race on it, so
+ * 4.0 MB shared by all calls: calls whose device work overlaps race on it, so
  * issue them on one stream or synchronise between them.  The first call on a
  * device looks up that array's address; make it before any stream capture.
  * relx_release (or relx_init with another table path) frees the tables these
@@ -155,7 +155,7 @@ int relx_eval_one_noalloc(int model, const double *d_params, const double *d_ene
 /* Device line-profile cache, the counterpart of the reference's relbase
  * cache (src/Relcache.cpp:311-331, src/Relbase.cpp:461-538): sets whose
  * relativistic parameters match a cached entry reuse its line profile and skip
- * the line-profile kernels.  slots entries of about 260 KB each (rounded up to
+ * the line-profile kernels.  slots entries of about 274 KB each (rounded up to
  * a power of two); 0 turns it off (the default).  Used by every batched,
  * device and serving call; relline (whose profile lives on the caller's grid)
  * and sets with more than 16 zones are not cached. */
@@ -219,8 +219,8 @@ int relx_selftest_wait_timeout(double limit_ms, int *status);
  * batch of 2048 sets or more of a (model, batch-size class, zone count) is run
  * once per candidate (one range, or pipelined chunks of 1024 sets) and the
  * fastest is kept for the class; that batch synchronises its stream (smaller
- * batches have one candidate, recorded without trials; the line-kernel tile is
- * fixed at 512 bins).
+ * batches have one candidate, recorded without trials; the line-kernel tile
+ * in the report is the 128 bins of the kernel for many sets).
  * graphs != 0: a batch shape that recurs on the same workspace is captured
  * into a CUDA graph on its second launch and replayed afterwards.  Both are on
  * by default; every choice gives the same numbers. */

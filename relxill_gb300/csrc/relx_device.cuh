@@ -246,31 +246,6 @@ __device__ __forceinline__ float2 ff_addf(float2 a, float b) {
 }
 __device__ __forceinline__ double ff_to_double(float2 a) { return (double) a.x + (double) a.y; }
 
-// block-wide float-float sum with a fixed reduction tree (deterministic); scratch holds NT/32 + 1
-template <int NT>
-__device__ __forceinline__ float2 block_sum_ff(float2 v, float2 *scratch) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    float2 t;
-    t.x = __shfl_xor_sync(0xffffffffu, v.x, o);
-    t.y = __shfl_xor_sync(0xffffffffu, v.y, o);
-    v = ff_add(v, t);
-  }
-  __syncthreads();
-  if (lane == 0) scratch[w] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float2 r = make_float2(0.0f, 0.0f);
-    for (int i = 0; i < NT / 32; i++) r = ff_add(r, scratch[i]);
-    scratch[NT / 32] = r;
-  }
-  __syncthreads();
-  const float2 r = scratch[NT / 32];
-  __syncthreads();
-  return r;
-}
-
 // block-wide sum in FP64 with a fixed reduction tree (deterministic); in a block of more than NT threads
 // the sum over the first NT
 template <int NT>

@@ -18,7 +18,6 @@ constexpr int kFinThreadsH = 128;
 
 size_t hist_smem_bytes(int nr, int ng);
 size_t conv_smem_bytes();
-size_t fin_smem_bytes();
 
 cudaError_t setup_set_smem();
 cudaError_t launch_setup(cudaStream_t s, int n_sets, const RelxTables &tab, int model, const RelxSetIn *sin,
