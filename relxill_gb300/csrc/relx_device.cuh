@@ -123,10 +123,14 @@ __device__ __forceinline__ double lerp2(double f1, double f2, double r11, double
 }
 
 // ---- Kerr metric (Relphysics.cpp), FP64 -------------------------------------
-__device__ __forceinline__ double kerr_rms(double a) {
-  double sign = (a < 0) ? -1.0 : 1.0;
+// cr: kerr_cbrt(a, 0), (a, 1), (a, 2), three long FP64 chains that three lanes run at once
+__device__ __forceinline__ double kerr_cbrt(double a, int k) {
   // cube roots as cbrt (the reference writes pow(x, 1.0/3.0); the two differ by about an ulp)
-  double z1 = 1.0 + cbrt(1.0 - a * a) * (cbrt(1.0 + a) + cbrt(1.0 - a));
+  return cbrt(k == 0 ? 1.0 - a * a : k == 1 ? 1.0 + a : 1.0 - a);
+}
+__device__ __forceinline__ double kerr_rms(double a, const double *cr) {
+  double sign = (a < 0) ? -1.0 : 1.0;
+  double z1 = 1.0 + cr[0] * (cr[1] + cr[2]);
   double z2 = sqrt((3.0 * a * a) + (z1 * z1));
   return 3.0 + z2 - sign * sqrt((3.0 - z1) * (3.0 + z1 + (2 * z2)));
 }
@@ -138,11 +142,11 @@ __device__ __forceinline__ double calc_g_inf(double h, double a) { return sqrt(1
 __device__ __forceinline__ double doppler_factor(double del, double bet) {
   return sqrt(1.0 - bet * bet) / (1.0 + bet * cos(del));
 }
-// gi_potential_lp, Relphysics.cpp:163-207
-__device__ __forceinline__ double gi_potential_lp(double r, double a, double h, double bet, double del) {
+// gi_potential_lp, Relphysics.cpp:163-207; ut_h: lp_ut_h(h, a), which does not depend on the radius
+__device__ __forceinline__ double lp_ut_h(double h, double a) { return sqrt((h * h + a * a) / (h * h - 2 * h + a * a)); }
+__device__ __forceinline__ double gi_potential_lp(double r, double a, double h, double ut_h, double bet, double del) {
   double sr = sqrt(r);
   double ut_d = ((r * sr + a) / (sr * sqrt(r * r - 3 * r + 2 * a * sr)));
-  double ut_h = sqrt((h * h + a * a) / (h * h - 2 * h + a * a));
   double gi = ut_d / ut_h;
   if (fabs(bet) < 1e-6) return gi;
   double gam = 1.0 / sqrt(1.0 - bet * bet);

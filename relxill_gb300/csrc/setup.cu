@@ -52,6 +52,8 @@ struct SetupSmem {
   };
   double inv_dtab[RELX_MAX_NRTAB];
   double inv_lineE;
+  double kerr_cr[3];  // cube roots of kerr_rms
+  double ut_hd;       // lp_ut_h of the source
   double dgmin_t[RELX_MAX_NRTAB], dgmax_t[RELX_MAX_NRTAB];  // gmin, gmax of table radius i less those of i + 1
   float jet_rad_f[RELX_MAX_NRADLP];
   float lp_dle[RELX_MAX_NRADLP], lp_dlr[RELX_MAX_NRADLP], lp_d[RELX_MAX_NRADLP], lp_di[RELX_MAX_NRADLP];
@@ -103,6 +105,18 @@ static_assert(sizeof(RradSmem) + sizeof(float) * RELX_NFRAD <= sizeof(double) * 
 // ---------------------------------------------------------------------------
 // parameter mapping (lmodel_relxill_public.dat:1-75, ModelDefinition.cpp:153-385)
 // ---------------------------------------------------------------------------
+// position of the spin in a model's parameters (as map_params reads it)
+__device__ __forceinline__ int spin_index(int model) {
+  switch (model) {
+    case RELX_RELLINE: return 4;
+    case RELX_RELCONV:
+    case RELX_RELXILL: return 3;
+    case RELX_RELXILLCP:
+    case RELX_RELXILLLPCP: return 1;
+    default: return 2;  // relxilllp, relline_lp, relconv_lp
+  }
+}
+
 __device__ void map_params(int model, const RelxSetIn &in, SetupSmem &m) {
   RelxSetState &s = m.s;
   const double *v = in.p;
@@ -190,7 +204,7 @@ __device__ void map_params(int model, const RelxSetIn &in, SetupSmem &m) {
   }
   s.gamma = s.gam;
   // check_parameter_bounds, ModelDefinition.cpp:168-273
-  double rms = kerr_rms(s.a);
+  double rms = kerr_rms(s.a, m.kerr_cr);
   m.rms = rms;
   if (s.rin < 0) s.rin = -1.0 * s.rin * rms;
   if (s.rout < 0) s.rout = -1.0 * s.rout * rms;
@@ -285,7 +299,12 @@ __device__ void zone_grid_warp(double rmin, double rmax, int nz, double h, doubl
   int indr = 0;
   if (h > rmin) {
     r_tr = h;
-    for (int ii = lane; ii < nz + 1; ii += 32) rg[ii] = exp(1.0 * ii / nz * (log(rmax) - log(rmin)) + log(rmin));
+    // the two logarithms, and below the two reciprocals, by two lanes at once: each is a long chain, and two lanes
+    // take as long on the FP64 pipe as one
+    double lg = 0.0;
+    if (lane < 2) lg = log(lane ? rmax : rmin);
+    const double lmin = __shfl_sync(0xffffffffu, lg, 0), lmax = __shfl_sync(0xffffffffu, lg, 1);
+    for (int ii = lane; ii < nz + 1; ii += 32) rg[ii] = exp(1.0 * ii / nz * (lmax - lmin) + lmin);
     __syncwarp();
     if (lane == 0) indr = bsearch_asc<double>(rg, nz + 1, r_tr);
     indr = __shfl_sync(0xffffffffu, indr, 0);
@@ -293,9 +312,11 @@ __device__ void zone_grid_warp(double rmin, double rmax, int nz, double h, doubl
     __syncwarp();
   }
   if (indr < nz) {
-    double rlo = r_tr, rhi = rmax;
+    double iv = 0.0;
+    if (lane < 2) iv = 1.0 / (lane ? rmax : r_tr);
+    const double ilo = __shfl_sync(0xffffffffu, iv, 0), ihi = __shfl_sync(0xffffffffu, iv, 1);
     for (int ii = indr + lane; ii < nz + 1; ii += 32) {
-      double v = 1.0 * (ii - indr) / (nz - indr) * (1.0 / rhi - 1.0 / rlo) + 1.0 / rlo;
+      double v = 1.0 * (ii - indr) / (nz - indr) * (ihi - ilo) + ilo;
       rg[ii] = fabs(1.0 / v);
     }
   }
@@ -494,6 +515,10 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
   const int NR = RELX_NFRAD;
   const int kind = relx_kind(model);
 
+  if (tid < 32) {
+    if (tid < 3) m.kerr_cr[tid] = kerr_cbrt(in.p[spin_index(model)], tid);
+    __syncwarp();
+  }
   if (tid == 0) {
     map_params(model, in, m);
     m.status = s.status;
@@ -555,7 +580,8 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
     m.fg_du = (1.0 / sqrt(s.rin) - m.fg_r1) / (NR - 1);
     if (s.emis_type == RELX_EMIS_LP) {
       const double hh = s.height, aa = s.a;
-      m.ut_h = (float) sqrt((hh * hh + aa * aa) / (hh * hh - 2 * hh + aa * aa));
+      m.ut_hd = lp_ut_h(hh, aa);
+      m.ut_h = (float) m.ut_hd;
     } else {
       m.inv_rbr = (float) (1.0 / m.rbr);
     }
@@ -572,7 +598,7 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
       for (int z = tid; z < s.nz; z += 32) {
         m.rmean[z] = 0.5 * (s.rgrid[z] + s.rgrid[z + 1]);
         if (early_shift)  // a source at rest: gi_potential_lp does not read the emission angle
-          m.shift[z] = (s.emis_type == RELX_EMIS_LP) ? gi_potential_lp(m.rmean[z], s.a, s.height, s.beta, 0.0) : 1.0;
+          m.shift[z] = (s.emis_type == RELX_EMIS_LP) ? gi_potential_lp(m.rmean[z], s.a, s.height, m.ut_hd, s.beta, 0.0) : 1.0;
         if (s.ion_grad_type != 2) zone_ionisation(m, s, z);
       }
     }
@@ -840,7 +866,7 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
       const float srf = d2f(sr);
       const float ut_d = fmaf(d2f(r), srf, d2f(aa)) / (srf * sqrtf(d2f(t)));
       float gi = ut_d / ut_h;
-      if (moving) gi = (float) gi_potential_lp(r, aa, hh, s.beta, f2d(del_e));
+      if (moving) gi = (float) gi_potential_lp(r, aa, hh, m.ut_hd, s.beta, f2d(del_e));
       float boost = powf(gi, gam_f);
       if (boosted) {
         const float d = (float) doppler_factor(f2d(del_e), s.beta);
@@ -930,7 +956,7 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
     int z = tid;
     if (!early_shift) {
       m.zdel_emit[z] = rebin_mean_at(m.re, m.pr.del_emit, NR, m.rmean[z]);
-      m.shift[z] = gi_potential_lp(m.rmean[z], s.a, s.height, s.beta, m.zdel_emit[z]);
+      m.shift[z] = gi_potential_lp(m.rmean[z], s.a, s.height, m.ut_hd, s.beta, m.zdel_emit[z]);
     }
     if (s.ion_grad_type == 2) {
       double rin = s.rgrid[0];
