@@ -17,14 +17,14 @@
 // normalisation is linear in the table, sum_j G_j sp_j times the inverse of the
 // table at the 1 keV point.
 //
-// nthcomp_kernel: two lanes per continuum (the source, and each zone whose
+// nthcomp_kernel: four lanes per continuum (the source, and each zone whose
 // energy shift differs from 1).  The tridiagonal coefficients are formed on
 // the fly from the grid and the continuum's tautom and theta, and the system
-// (thermlc, donthcomp.c:194-280) is eliminated from both ends towards the middle in
+// is solved by the Thomas algorithm (thermlc, donthcomp.c:194-280) in
 // float-float arithmetic on the FP32 pipe (about 48 significant bits; the FP64
-// pipe of this part runs at 1/64 of the FP32 rate).  The elimination keeps
-// its two recurrences per point in a scratch laid out [step][continuum][side], so a
-// warp's accesses are contiguous; the sweep outwards recovers the solution, forms
+// pipe of this part runs at 1/64 of the FP32 rate).  The forward sweep keeps
+// its two recurrences per point in a scratch laid out [point][continuum], so a
+// warp's accesses are contiguous; the back sweep recovers the solution, forms
 // E F_E (donthcomp.c:603-610) and accumulates the normalisation.  The source
 // continuum also writes its table for the primary spectrum (c_donthcomp,
 // donthcomp.c:640-793).
@@ -174,23 +174,6 @@ int nth_grid_build(const std::vector<double> &co, double band_lo, double band_hi
 
 __device__ __forceinline__ double nth_lg10(double x) { return 0.43429448190325182765 * log(x); }
 
-// float-float product with both cross terms fused, and the sum that keeps the low parts' rounding: for the
-// cancelling pivots.  With these the system solved from both ends is no further from an 80-bit solution than
-// from one end with ff_mul and ff_add (kTe 20-300 keV, Gamma 1.4-2.8: normalisation 1.34e-12 at
-// most against 1.48e-12, 3.37e-13 against 3.40e-13 rms; table 2.40e-12 of its maximum against 2.56e-12)
-__device__ __forceinline__ float2 nth_mul(float2 a, float2 b) {
-  const float p = __fmul_rn(a.x, b.x);
-  float e = __fmaf_rn(a.x, b.x, -p);
-  e = __fmaf_rn(a.x, b.y, e);
-  e = __fmaf_rn(a.y, b.x, e);
-  return qts(p, e);
-}
-__device__ __forceinline__ float2 nth_add(float2 a, float2 b) {
-  const float2 s = two_sum(a.x, b.x), t = two_sum(a.y, b.y);
-  const float2 v = qts(s.x, __fadd_rn(s.y, t.x));
-  return qts(v.x, __fadd_rn(t.y, v.y));
-}
-
 // reciprocal in float-float: the float reciprocal and one Newton step
 __device__ __forceinline__ float2 ff_rcp(float2 a) {
   const float r = __frcp_rn(a.x);
@@ -205,30 +188,26 @@ __device__ __forceinline__ float2 ff_rcp(float2 a) {
 __device__ __forceinline__ float2 nth_bt(const NthPoint &P, int j, float2 tau, int jnr, int jrel, float2 xnr,
                                          float2 invdx) {
   if (j > jrel) return make_float2(1.0f, 0.0f);
-  float2 y = nth_mul(tau, P.rel3);
-  if (j >= jnr) y = nth_mul(y, ff_addf(ff_neg(nth_mul(ff_add(P.x, ff_neg(xnr)), invdx)), 1.0f));
+  float2 y = ff_mul(tau, P.rel3);
+  if (j >= jnr) y = ff_mul(y, ff_addf(ff_neg(ff_mul(ff_add(P.x, ff_neg(xnr)), invdx)), 1.0f));
   return ff_rcp(ff_addf(y, 1.0f));
 }
 
-// The system is eliminated from both ends at once: rows j = 2 .. M upwards and M + 1 .. jmax - 1 downwards
-// (M = jmax / 2), which halves the serial chain.  With a_j = -A_j, c_j = T_{j-1},
-// b_j = A_{j-1} - T_j + x_j^3 bt_j, A_j = tautom cd_j (theta iw_j + 1/2), T_j = tautom cd_j (1/2 - theta iw_j),
-// row j reads  a_j u(j+1) + b_j u(j) + c_j u(j-1) = d_j,  u(1) = aa u(2), u(jmax) = 0.  The columns are
-// diagonally dominant where T < 0, and each pivot only grows where T > 0, in both directions.
-// One row of either side: the neighbour already eliminated is d - g u with coefficient P, the one still to
-// come has coefficient Q: u = dn - gn u(next).
-__device__ __forceinline__ void nth_row(float2 b, float2 P, float2 Q, float2 xd, float2 &g, float2 &d) {
-  const float2 alp = nth_add(b, ff_neg(nth_mul(P, g)));
-  const float2 num = ff_add(xd, ff_neg(nth_mul(P, d)));
+// The Thomas algorithm on  a_j u(j+1) + b_j u(j) + c_j u(j-1) = d_j,  u(1) = aa u(2), u(jmax) = 0, with
+// a_j = -A_j, c_j = T_{j-1}, b_j = A_{j-1} - T_j + x_j^3 bt_j, A_j = tautom cd_j (theta iw_j + 1/2),
+// T_j = tautom cd_j (1/2 - theta iw_j):  u(j) = d - g u(j+1).  (Eliminating from both ends halves the serial chain
+// and is as accurate, but changes the last bits of the tables, which the FP32 weights made from them turn
+// into 6e-8 of a spectrum.)
+// One row of the forward sweep; c: T_{j-1}, first: j = 2
+__device__ __forceinline__ void nth_row(float2 b, float2 c, float2 A, float2 xd, float2 aa, bool first, float2 &g, float2 &d) {
+  const float2 m = ff_mul(c, first ? aa : g);
+  const float2 alp = ff_add(b, first ? m : ff_neg(m));
+  const float2 num = first ? xd : ff_add(xd, ff_neg(ff_mul(c, d)));
   const float2 ia = ff_rcp(alp);
-  g = nth_mul(Q, ia);
-  d = nth_mul(num, ia);
+  g = ff_mul(ff_neg(A), ia);
+  d = ff_mul(num, ia);
 }
-// u where the sides meet: u = d - g v, v = od - og u
-__device__ __forceinline__ float2 nth_meet(float2 g, float2 d, float2 og, float2 od) {
-  return nth_mul(ff_add(d, ff_neg(nth_mul(g, od))), ff_rcp(ff_addf(ff_neg(nth_mul(g, og)), 1.0f)));
-}
-__device__ __forceinline__ float2 nth_back(float2 g, float2 d, float2 u) { return ff_add(d, ff_neg(nth_mul(g, u))); }
+__device__ __forceinline__ float2 nth_back(float2 g, float2 d, float2 u) { return ff_add(d, ff_neg(ff_mul(g, u))); }
 
 // Scalars of a continuum.  Returns false for a kTe that leaves fewer than 4 points (kTe <= 0 or far below
 // the seed temperature, donthcomp.c:320-375), which has no spectrum
@@ -250,15 +229,15 @@ __device__ __forceinline__ bool nth_cont(const NthGrid *__restrict__ G, double g
   c.th = ff_from_double(theta);
   c.xnr = G->p[c.jnr].x;
   c.invdx = ff_from_double(1.0 / (G->x[c.jrel] - G->x[c.jnr]));
-  const float2 u1 = nth_mul(c.th, G->p[1].iw);
-  c.aa = nth_mul(ff_addf(u1, .5f), ff_rcp(ff_addf(u1, -.5f)));
+  const float2 u1 = ff_mul(c.th, G->p[1].iw);
+  c.aa = ff_mul(ff_addf(u1, .5f), ff_rcp(ff_addf(u1, -.5f)));
   return true;
 }
 // A and T of a point
 __device__ __forceinline__ void nth_at(const NthPoint &P, const NthCont &c, float2 &A, float2 &T) {
-  const float2 u = nth_mul(c.th, P.iw), Pj = nth_mul(c.tau, P.cd);
-  A = nth_mul(Pj, ff_addf(u, .5f));
-  T = nth_mul(Pj, ff_addf(ff_neg(u), .5f));
+  const float2 u = ff_mul(c.th, P.iw), Pj = ff_mul(c.tau, P.cd);
+  A = ff_mul(Pj, ff_addf(u, .5f));
+  T = ff_mul(Pj, ff_addf(ff_neg(u), .5f));
 }
 // normalisation on the coarse grid from the sum over the table and E F_E at the points around 1 keV
 // (donthcomp.c:617-638, 754-758)
@@ -288,9 +267,15 @@ __device__ __forceinline__ bool nth_which(const RelxSetIn *__restrict__ sin, con
   return true;
 }
 
-// Two neighbouring lanes per continuum, one for each side.  Bound by the latency of the chain: 1000 sets of 11
-// continua are 2 to 5 warps per SM; one thread per continuum from one end 382 us, so 248 us.
-// scr: the sides' recurrences, [step][continuum][side] with this launch's continua from c_off of ncont_all.
+// Four neighbouring lanes per continuum: the lanes form the coefficients of four points at once, then all four run
+// the recurrence over these points (the coefficients by shuffles), and on the way back each forms its own
+// point of the table.  Bound by the latency of the chain: 1000 sets of 11 continua are 9 warps per SM; one lane
+// per continuum 382 us, so 276 us.
+// scr: the recurrences, [point][continuum] with this launch's continua from c_off of ncont_all.
+constexpr int kNthLanes = 4;
+__device__ __forceinline__ float2 nth_shfl(float2 v, int src) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src, kNthLanes), __shfl_sync(0xffffffffu, v.y, src, kNthLanes));
+}
 __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__restrict__ G,
                                                               const RelxSetIn *__restrict__ sin,
                                                               const RelxSetState *__restrict__ sst, bool params,
@@ -306,8 +291,8 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
     for (int i = threadIdx.x; i < (RELX_NTH_N + 1) * 4; i += kNthThreads) dst[i] = src[i];
   }
   __syncthreads();
-  const int64_t gid = (int64_t) blockIdx.x * kNthThreads + threadIdx.x, c = gid >> 1;
-  const bool down = (gid & 1) != 0;
+  const int64_t gid = (int64_t) blockIdx.x * kNthThreads + threadIdx.x, c = gid / kNthLanes;
+  const int r = (int) (gid & (kNthLanes - 1));
   double gam, kte;
   const int set = (int) (c / per), k = (int) (c - (int64_t) set * per);
   bool act = c < (int64_t) n_sets * per && nth_which(sin, sst, params, set, k, gam, kte);
@@ -315,122 +300,116 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
   NthTable *T = (act && k == 0) ? &tabs[set] : nullptr;
   NthCont C;
   if (act && !nth_cont(G, gam, kte, C)) {  // a non-finite normalisation marks the set
-    if (!down) {
+    if (r == 0) {
       *q = __longlong_as_double(0x7ff8000000000000ll);
       if (T) T->n = 0;
     }
     act = false;
   }
-  if (!act) C.jmax = 0;  // no rows; the lanes take part in the exchanges
-  const int jmax = C.jmax, M = jmax >> 1;
-  const int n = act ? (down ? jmax - 1 - M : M - 1) : 0;  // rows of the side
-  float4 *sc = scr + (c_off + c) * 2 + (gid & 1);
-  const size_t pitch = (size_t) ncont_all * 2;
-  float2 g = make_float2(0.f, 0.f), d = g;
-  if (act) {
-    // a point ahead of the rows: 1 upwards, jmax - 1 downwards
-    NthPoint P = Pg[down ? jmax - 1 : 1];
-    float2 A0, T0, y0 = g, xd0 = P.xd;
-    nth_at(P, C, A0, T0);
-    if (down) y0 = nth_mul(P.x3, nth_bt(P, jmax - 1, C.tau, C.jnr, C.jrel, C.xnr, C.invdx));
-    else g = ff_neg(C.aa);
-    for (int i = 0; i < n; i++) {
-      const int jn = down ? jmax - 2 - i : 2 + i;  // the new point: the row's upwards, the one below it downwards
-      P = Pg[jn];
-      float2 A1, T1;
-      nth_at(P, C, A1, T1);
-      const float2 y1 = nth_mul(P.x3, nth_bt(P, jn, C.tau, C.jnr, C.jrel, C.xnr, C.invdx));
-      const float2 Al = down ? A1 : A0, Tl = down ? T1 : T0;  // of the row's lower point
-      const float2 Ah = down ? A0 : A1, Th = down ? T0 : T1;  // of its own
-      const float2 b = nth_add(nth_add(Al, ff_neg(Th)), down ? y0 : y1);
-      const float2 nA = ff_neg(Ah);
-      nth_row(b, down ? nA : Tl, down ? Tl : nA, down ? xd0 : P.xd, g, d);
-      sc[(size_t) i * pitch] = make_float4(g.x, g.y, d.x, d.y);
-      A0 = A1;
-      T0 = T1;
-      y0 = y1;
-      xd0 = P.xd;
-    }
+  const float2 zero = make_float2(0.f, 0.f);
+  if (!act) {  // no points; the lanes take part in the exchanges
+    C.jmax = 0;
+    C.jnr = C.jrel = 0;
+    C.tau = C.th = C.xnr = C.invdx = C.aa = zero;
   }
-  float2 og, od;
-  og.x = __shfl_xor_sync(0xffffffffu, g.x, 1);
-  og.y = __shfl_xor_sync(0xffffffffu, g.y, 1);
-  od.x = __shfl_xor_sync(0xffffffffu, d.x, 1);
-  od.y = __shfl_xor_sync(0xffffffffu, d.y, 1);
-  // outwards: u, E F_E = x^4 u bt (donthcomp.c:603-610), the normalisation sum (step i in partial sum i mod 8)
-  // and the table
+  const int jmax = C.jmax, jtop = __reduce_max_sync(0xffffffffu, jmax);  // of the warp's continua
+  float4 *sc = scr + c_off + c;
+  // forward sweep, four points at a time
+  float2 A3, T3;  // of the point before the four
+  nth_at(Pg[1], C, A3, T3);
+  float2 g = zero, d = zero;
+  for (int j0 = 2; j0 <= jtop - 1; j0 += kNthLanes) {
+    const int jr = min(j0 + r, RELX_NTH_N);
+    const NthPoint P = Pg[jr];
+    float2 A, Tj;
+    nth_at(P, C, A, Tj);
+    const float2 y = ff_mul(P.x3, nth_bt(P, jr, C.tau, C.jnr, C.jrel, C.xnr, C.invdx));
+    const float2 Au = nth_shfl(A, max(r - 1, 0)), Tu = nth_shfl(Tj, max(r - 1, 0));
+    const float2 Al = r == 0 ? A3 : Au, Tl = r == 0 ? T3 : Tu;  // of the point below
+    const float2 b = ff_add(ff_add(Al, ff_neg(Tj)), y);
+    float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kNthLanes; i++) {
+      const float2 bi = nth_shfl(b, i), ci = nth_shfl(Tl, i), Ai = nth_shfl(A, i), xi = nth_shfl(P.xd, i);
+      if (j0 + i <= jmax - 1) nth_row(bi, ci, Ai, xi, C.aa, i == 0 && j0 == 2, g, d);
+      if (r == i) mine = make_float4(g.x, g.y, d.x, d.y);
+    }
+    if (j0 + r <= jmax - 1) sc[(size_t) (j0 + r) * ncont_all] = mine;
+    A3 = nth_shfl(A, kNthLanes - 1);
+    T3 = nth_shfl(Tj, kNthLanes - 1);
+  }
+  // back sweep from j = jmax - 1 to 1: u, E F_E = x^4 u bt (donthcomp.c:603-610), the normalisation sum and the table;
+  // the lane's next point of the scratch is fetched ahead
   const int ih = min(G->ih0, jmax), il = ih - 1;
-  float2 u = make_float2(0.f, 0.f), s_il = u, s_ih = u;
-  float2 qs[8];
+  float2 u = zero, qs = zero, s_il = zero, s_ih = zero;
+  float4 nx = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (jmax - 1 - r >= 2) nx = sc[(size_t) (jmax - 1 - r) * ncont_all];
+  for (int o = 0; o < jtop - 1; o += kNthLanes) {
+    const int jr = jmax - 1 - o - r;
+    const float4 v = nx;
+    if (jr - kNthLanes >= 2) nx = sc[(size_t) (jr - kNthLanes) * ncont_all];
+    float2 uo = zero;
 #pragma unroll
-  for (int e = 0; e < 8; e++) qs[e] = u;
-  if (act) {
-    const int cnt = down ? n : n + 1;  // the lower side ends with u(1) = aa u(2)
-    // the scratch is read 8 points at a time (independent loads in flight together)
-    for (int i0 = 0; i0 < cnt; i0 += 8) {
-      float4 vb[8];
+    for (int i = 0; i < kNthLanes; i++) {
+      const int j = jmax - 1 - o - i;
+      const float2 gi = nth_shfl(make_float2(v.x, v.y), i), di = nth_shfl(make_float2(v.z, v.w), i);
+      if (j >= 2) u = nth_back(gi, di, u);
+      else if (j == 1) u = ff_mul(C.aa, u);
+      if (r == i) uo = u;
+    }
+    const NthPoint P = Pg[max(jr, 0)];
+    const float2 sp = ff_mul(ff_mul(P.x4, uo), nth_bt(P, jr, C.tau, C.jnr, C.jrel, C.xnr, C.invdx));
+    const float2 t = ff_mul(P.g, sp);
 #pragma unroll
-      for (int e = 0; e < 8; e++)
-        if (i0 + e > 0 && i0 + e < n) vb[e] = sc[(size_t) (n - 1 - i0 - e) * pitch];
-#pragma unroll
-      for (int e = 0; e < 8; e++) {
-        const int i = i0 + e;
-        if (i >= cnt) break;
-        const int j = down ? M + 1 + i : M - i;
-        if (i == 0) u = nth_meet(g, d, og, od);
-        else if (i < n) u = nth_back(make_float2(vb[e].x, vb[e].y), make_float2(vb[e].z, vb[e].w), u);
-        else u = nth_mul(C.aa, u);
-        const NthPoint P = Pg[j];
-        const float2 sp = nth_mul(nth_mul(P.x4, u), nth_bt(P, j, C.tau, C.jnr, C.jrel, C.xnr, C.invdx));
-        qs[e] = ff_add(qs[e], nth_mul(P.g, sp));
-        if (j == il) s_il = sp;
-        if (j == ih) s_ih = sp;
-        if (T) {
-          T->sp[j] = ff_to_double(sp);
-          T->spf[j] = __fadd_rn(sp.x, sp.y);
-        }
+    for (int i = 0; i < kNthLanes; i++) {
+      const float2 ti = nth_shfl(t, i);
+      if (jmax - 1 - o - i >= 1) qs = ff_add(qs, ti);
+    }
+    if (jr >= 1) {
+      if (jr == il) s_il = sp;
+      if (jr == ih) s_ih = sp;
+      if (T) {
+        T->sp[jr] = ff_to_double(sp);
+        T->spf[jr] = __fadd_rn(sp.x, sp.y);
       }
     }
   }
-  float2 q1 = ff_add(ff_add(ff_add(qs[0], qs[1]), ff_add(qs[2], qs[3])), ff_add(ff_add(qs[4], qs[5]), ff_add(qs[6], qs[7])));
-  const auto other = [](float2 v) {
-    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, 1), __shfl_xor_sync(0xffffffffu, v.y, 1));
-  };
-  q1 = ff_add(q1, other(q1));
-  const float2 oil = other(s_il), oih = other(s_ih);
-  if (act && !down) {
+  s_il = nth_shfl(s_il, (jmax - 1 - il) & (kNthLanes - 1));  // zero where the point is jmax
+  s_ih = nth_shfl(s_ih, (jmax - 1 - ih) & (kNthLanes - 1));
+  if (act && r == 0) {
     if (T) {
       T->sp[jmax] = 0.0;
       T->spf[jmax] = 0.0f;
       T->n = jmax;
     }
-    *q = nth_norm(G, q1, il > M ? oil : s_il, ih > M ? oih : s_ih, il, ih);
+    *q = nth_norm(G, qs, s_il, s_ih, il, ih);
   }
 }
 
-// The same continua for few sets, one CTA per continuum: the per-point and per-row quantities and the table
-// are formed by all threads at once in shared memory, and one warp runs only the recurrences, a lane for
-// each side, with the operations and the order of nthcomp_kernel: the same numbers, with a serial
-// chain a few times shorter (one set: from one end 128 us, so 52 us).
+// The same continua for few sets, one CTA per continuum: the per-point quantities are formed by all threads at once
+// in shared memory, and one warp runs only the recurrences, with the operations and the order of
+// nthcomp_kernel: the same numbers.  On the way back the table's points and the normalisation sum follow the
+// recurrence in other warps, kNthChunk points behind each other (one set: 128 us with sums and table on the recurrence's
+// thread, 84 us so).
 struct NthCoopSmem {
   union {
     struct { float2 A[RELX_NTH_N + 1], T[RELX_NTH_N + 1]; };  // until the rows are formed
-    float4 gd[RELX_NTH_N + 1];                                // the sides' recurrences
+    float4 gd[RELX_NTH_N + 1];                                // the recurrences
   };
   union {
     float4 bd[RELX_NTH_N + 1];                                  // rows' b and right-hand side, then
     struct { float2 sp[RELX_NTH_N + 1], t[RELX_NTH_N + 1]; };  // the table and the sum's terms
   };
-  float4 pq[RELX_NTH_N + 1];                               // rows' P and Q
+  float4 ca[RELX_NTH_N + 1];                               // rows' T_{j-1} and A_j
   union { float2 y[RELX_NTH_N + 1], u[RELX_NTH_N + 1]; };  // x^3 bt until the rows are formed, then u
   float2 bt[RELX_NTH_N + 1];
 };
 static_assert(3 * (sizeof(NthCoopSmem) + 1024) <= 228 * 1024, "three CTAs per SM");
 
 constexpr int kNthCoopThreads = 128;
-// up to three waves of three CTAs per SM (912 continua 103 us, 1368 150 us, 2000 234 us; by two lanes each 203 us at
-// any of these)
-constexpr int kNthCoop = 3 * 3 * 152;
+constexpr int kNthChunk = 64;
+// one wave of three CTAs per SM (456 continua 108 us, by four lanes each 197 us; 912 209 us and 199 us)
+constexpr int kNthCoop = 3 * 152;
 
 __global__ void __launch_bounds__(kNthCoopThreads) nthcomp_coop_kernel(const NthGrid *__restrict__ G,
                                                                        const RelxSetIn *__restrict__ sin,
@@ -440,7 +419,7 @@ __global__ void __launch_bounds__(kNthCoopThreads) nthcomp_coop_kernel(const Nth
                                                                        NthTable *__restrict__ tabs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NthCoopSmem &m = *reinterpret_cast<NthCoopSmem *>(smem_raw);
-  const int set = blockIdx.x / per, k = blockIdx.x - set * per, tid = threadIdx.x, lane = tid & 31;
+  const int set = blockIdx.x / per, k = blockIdx.x - set * per, tid = threadIdx.x, warp = tid >> 5;
   double gam, kte;
   if (!nth_which(sin, sst, params, set, k, gam, kte)) return;  // block-uniform
   double *q = qout + (size_t) set * nq + k;
@@ -453,91 +432,81 @@ __global__ void __launch_bounds__(kNthCoopThreads) nthcomp_coop_kernel(const Nth
     }
     return;
   }
-  const int jmax = C.jmax, M = jmax >> 1;
+  const int jmax = C.jmax;
   // per point, in parallel
   for (int j = 1 + tid; j <= jmax - 1; j += kNthCoopThreads) {
     const NthPoint P = G->p[j];
     nth_at(P, C, m.A[j], m.T[j]);
     const float2 bt = nth_bt(P, j, C.tau, C.jnr, C.jrel, C.xnr, C.invdx);
     m.bt[j] = bt;
-    m.y[j] = nth_mul(P.x3, bt);
+    m.y[j] = ff_mul(P.x3, bt);
   }
   __syncthreads();
   for (int j = 2 + tid; j <= jmax - 1; j += kNthCoopThreads) {
-    const float2 b = nth_add(nth_add(m.A[j - 1], ff_neg(m.T[j])), m.y[j]), xd = G->p[j].xd;
-    const float2 Tl = m.T[j - 1], nA = ff_neg(m.A[j]);
-    const float2 P = j > M ? nA : Tl, Q = j > M ? Tl : nA;
+    const float2 b = ff_add(ff_add(m.A[j - 1], ff_neg(m.T[j])), m.y[j]), xd = G->p[j].xd;
     m.bd[j] = make_float4(b.x, b.y, xd.x, xd.y);
-    m.pq[j] = make_float4(P.x, P.y, Q.x, Q.y);
+    m.ca[j] = make_float4(m.T[j - 1].x, m.T[j - 1].y, m.A[j].x, m.A[j].y);
   }
   __syncthreads();
-  const int ih = min(G->ih0, jmax), il = ih - 1;
-  if (tid < 32) {
-    const bool down = (lane & 1) != 0;  // the lanes of a side do the same
-    const int n = down ? jmax - 1 - M : M - 1, step = down ? -1 : 1;
+  if (warp == 0) {  // every lane the same
     float2 g = make_float2(0.f, 0.f), d = g;
-    if (!down) g = ff_neg(C.aa);
-    int j = down ? jmax - 1 : 2;
-    float4 bd = m.bd[j], pq = m.pq[j];
-    for (int i = 0; i < n; i++, j += step) {
-      const int jn = i + 1 < n ? j + step : j;  // the next row's loads do not wait for the chain
-      const float4 bdn = m.bd[jn], pqn = m.pq[jn];
-      nth_row(make_float2(bd.x, bd.y), make_float2(pq.x, pq.y), make_float2(pq.z, pq.w), make_float2(bd.z, bd.w), g, d);
+    float4 bd = m.bd[2], ca = m.ca[2];
+    nth_row(make_float2(bd.x, bd.y), make_float2(ca.x, ca.y), make_float2(ca.z, ca.w), make_float2(bd.z, bd.w), C.aa, true,
+            g, d);
+    m.gd[2] = make_float4(g.x, g.y, d.x, d.y);
+    bd = m.bd[3];  // jmax is at least 4
+    ca = m.ca[3];
+#pragma unroll 2
+    for (int j = 3; j <= jmax - 1; j++) {
+      const float4 bdn = m.bd[j + 1], can = m.ca[j + 1];  // the next row's loads do not wait for the chain
+      nth_row(make_float2(bd.x, bd.y), make_float2(ca.x, ca.y), make_float2(ca.z, ca.w), make_float2(bd.z, bd.w), C.aa,
+              false, g, d);
       m.gd[j] = make_float4(g.x, g.y, d.x, d.y);
       bd = bdn;
-      pq = pqn;
-    }
-    float2 og, od;
-    og.x = __shfl_xor_sync(0xffffffffu, g.x, 1);
-    og.y = __shfl_xor_sync(0xffffffffu, g.y, 1);
-    od.x = __shfl_xor_sync(0xffffffffu, d.x, 1);
-    od.y = __shfl_xor_sync(0xffffffffu, d.y, 1);
-    float2 u = nth_meet(g, d, og, od);
-    j = down ? M + 1 : M;
-    m.u[j] = u;
-    float4 gd = m.gd[n > 1 ? j - step : j];
-    for (int i = 1; i < n; i++) {
-      j -= step;
-      const float4 gdn = m.gd[i + 1 < n ? j - step : j];
-      u = nth_back(make_float2(gd.x, gd.y), make_float2(gd.z, gd.w), u);
-      m.u[j] = u;
-      gd = gdn;
-    }
-    if (!down) m.u[1] = nth_mul(C.aa, u);
-  }
-  __syncthreads();
-  for (int j = 1 + tid; j <= jmax - 1; j += kNthCoopThreads) {
-    const NthPoint &P = G->p[j];
-    const float2 sp = nth_mul(nth_mul(P.x4, m.u[j]), m.bt[j]);
-    m.sp[j] = sp;
-    m.t[j] = nth_mul(P.g, sp);
-    if (Tt) {
-      Tt->sp[j] = ff_to_double(sp);
-      Tt->spf[j] = __fadd_rn(sp.x, sp.y);
+      ca = can;
     }
   }
   __syncthreads();
-  if (tid < 32) {  // lanes 0-7 the lower side's partial sums, 8-15 the upper side's
-    const bool down = (lane & 8) != 0;
-    const int cnt = down ? jmax - 1 - M : M;
-    float2 qs = make_float2(0.f, 0.f);
-    if (lane < 16)
-      for (int i = lane & 7; i < cnt; i += 8) qs = ff_add(qs, m.t[down ? M + 1 + i : M - i]);
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      float2 v;
-      v.x = __shfl_xor_sync(0xffffffffu, qs.x, o);
-      v.y = __shfl_xor_sync(0xffffffffu, qs.y, o);
-      qs = ff_add(qs, v);
-    }
-    if (lane == 0) {
-      *q = nth_norm(G, qs, il >= 1 && il <= jmax - 1 ? m.sp[il] : make_float2(0.f, 0.f),
-                    ih >= 1 && ih <= jmax - 1 ? m.sp[ih] : make_float2(0.f, 0.f), il, ih);
-      if (Tt) {
-        Tt->sp[jmax] = 0.0;
-        Tt->spf[jmax] = 0.0f;
-        Tt->n = jmax;
+  // step s: warp 0 the recurrence of chunk s (downwards from jmax - 1), warps 2 and 3 the table of chunk s - 1, warp 1
+  // the sum over chunk s - 2
+  const int ih = min(G->ih0, jmax), il = ih - 1;
+  const int nch = (jmax - 1 + kNthChunk - 1) / kNthChunk;
+  float2 u = make_float2(0.f, 0.f), qs = u;
+  for (int st = 0; st < nch + 2; st++) {
+    const int ch = st - (warp == 0 ? 0 : warp == 1 ? 2 : 1);
+    const int hi = jmax - 1 - ch * kNthChunk, lo = max(hi - kNthChunk + 1, 1);
+    if (ch >= 0 && ch < nch) {
+      if (warp == 0) {
+        float4 gd = m.gd[max(hi, 2)];
+        for (int j = hi; j >= lo; j--) {
+          const float4 gdn = m.gd[max(j - 1, 2)];
+          u = j >= 2 ? nth_back(make_float2(gd.x, gd.y), make_float2(gd.z, gd.w), u) : ff_mul(C.aa, u);
+          m.u[j] = u;
+          gd = gdn;
+        }
+      } else if (warp == 1) {
+        for (int j = hi; j >= lo; j--) qs = ff_add(qs, m.t[j]);
+      } else {
+        for (int j = hi - (tid - 64); j >= lo; j -= kNthCoopThreads - 64) {
+          const float2 sp = ff_mul(ff_mul(G->p[j].x4, m.u[j]), m.bt[j]);
+          m.sp[j] = sp;
+          m.t[j] = ff_mul(G->p[j].g, sp);
+          if (Tt) {
+            Tt->sp[j] = ff_to_double(sp);
+            Tt->spf[j] = __fadd_rn(sp.x, sp.y);
+          }
+        }
       }
+    }
+    __syncthreads();
+  }
+  if (tid == 32) {
+    const float2 zero = make_float2(0.f, 0.f);
+    *q = nth_norm(G, qs, m.sp[il], ih <= jmax - 1 ? m.sp[ih] : zero, il, ih);
+    if (Tt) {
+      Tt->sp[jmax] = 0.0;
+      Tt->spf[jmax] = 0.0f;
+      Tt->n = jmax;
     }
   }
 }
@@ -601,7 +570,7 @@ cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetI
     nthcomp_coop_kernel<<<(unsigned) ncont, kNthCoopThreads, sizeof(NthCoopSmem), s>>>(tab.nth_grid, sin, sst, params,
                                                                                      per, nq, q, tabs);
   } else {
-    nthcomp_kernel<<<(unsigned) ((2 * ncont + kNthThreads - 1) / kNthThreads), kNthThreads,
+    nthcomp_kernel<<<(unsigned) ((kNthLanes * ncont + kNthThreads - 1) / kNthThreads), kNthThreads,
                      sizeof(NthPoint) * (RELX_NTH_N + 1), s>>>(tab.nth_grid, sin, sst, params, per, n_sets, nq, q,
                                                               tabs, scr, ncont_all, c_off);
   }

@@ -1,5 +1,5 @@
-"""nthcomp solved from both ends: the shortest systems (kTe near the seed temperature), the longest, odd and even
-lengths, and the same numbers by one CTA per continuum and by two lanes per continuum."""
+"""nthcomp: the shortest systems (kTe near the seed temperature), the longest, lengths that leave lanes of the last
+four points or chunks empty, and the same numbers by one CTA per continuum and by four lanes per continuum."""
 import numpy as np
 import pytest
 
