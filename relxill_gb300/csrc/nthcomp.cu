@@ -17,7 +17,7 @@
 // normalisation is linear in the table, sum_j G_j sp_j times the inverse of the
 // table at the 1 keV point.
 //
-// nthcomp_kernel: four lanes per continuum (the source, and each zone whose
+// nthcomp_kernel: one to four lanes per continuum (the source, and each zone whose
 // energy shift differs from 1).  The tridiagonal coefficients are formed on
 // the fly from the grid and the continuum's tautom and theta, and the system
 // is solved by the Thomas algorithm (thermlc, donthcomp.c:194-280) in
@@ -267,15 +267,17 @@ __device__ __forceinline__ bool nth_which(const RelxSetIn *__restrict__ sin, con
   return true;
 }
 
-// Four neighbouring lanes per continuum: the lanes form the coefficients of four points at once, then all four run
-// the recurrence over these points (the coefficients by shuffles), and on the way back each forms its own
-// point of the table.  Bound by the latency of the chain: 1000 sets of 11 continua are 9 warps per SM; one lane
+// Four, two or one neighbouring lanes per continuum: the lanes form the coefficients of as many points at once, then
+// all of them run the recurrence over these points (the coefficients by shuffles), and on the way back each forms
+// its own point of the table.  Bound by the latency of the chain: 1000 sets of 11 continua are 9 warps per SM; one lane
 // per continuum 382 us, so 276 us.
 // scr: the recurrences, [point][continuum] with this launch's continua from c_off of ncont_all.
-constexpr int kNthLanes = 4;
+template <int kNthLanes>
 __device__ __forceinline__ float2 nth_shfl(float2 v, int src) {
-  return make_float2(__shfl_sync(0xffffffffu, v.x, src, kNthLanes), __shfl_sync(0xffffffffu, v.y, src, kNthLanes));
+  if constexpr (kNthLanes == 1) return v;
+  else return make_float2(__shfl_sync(0xffffffffu, v.x, src, kNthLanes), __shfl_sync(0xffffffffu, v.y, src, kNthLanes));
 }
+template <int kNthLanes>
 __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__restrict__ G,
                                                               const RelxSetIn *__restrict__ sin,
                                                               const RelxSetState *__restrict__ sst, bool params,
@@ -314,8 +316,8 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
   }
   const int jmax = C.jmax, jtop = __reduce_max_sync(0xffffffffu, jmax);  // of the warp's continua
   float4 *sc = scr + c_off + c;
-  // forward sweep, four points at a time
-  float2 A3, T3;  // of the point before the four
+  // forward sweep, kNthLanes points at a time
+  float2 A3, T3;  // of the point before them
   nth_at(Pg[1], C, A3, T3);
   float2 g = zero, d = zero;
   for (int j0 = 2; j0 <= jtop - 1; j0 += kNthLanes) {
@@ -324,35 +326,43 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
     float2 A, Tj;
     nth_at(P, C, A, Tj);
     const float2 y = ff_mul(P.x3, nth_bt(P, jr, C.tau, C.jnr, C.jrel, C.xnr, C.invdx));
-    const float2 Au = nth_shfl(A, max(r - 1, 0)), Tu = nth_shfl(Tj, max(r - 1, 0));
+    const float2 Au = nth_shfl<kNthLanes>(A, max(r - 1, 0)), Tu = nth_shfl<kNthLanes>(Tj, max(r - 1, 0));
     const float2 Al = r == 0 ? A3 : Au, Tl = r == 0 ? T3 : Tu;  // of the point below
     const float2 b = ff_add(ff_add(Al, ff_neg(Tj)), y);
     float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < kNthLanes; i++) {
-      const float2 bi = nth_shfl(b, i), ci = nth_shfl(Tl, i), Ai = nth_shfl(A, i), xi = nth_shfl(P.xd, i);
+      const float2 bi = nth_shfl<kNthLanes>(b, i), ci = nth_shfl<kNthLanes>(Tl, i), Ai = nth_shfl<kNthLanes>(A, i), xi = nth_shfl<kNthLanes>(P.xd, i);
       if (j0 + i <= jmax - 1) nth_row(bi, ci, Ai, xi, C.aa, i == 0 && j0 == 2, g, d);
       if (r == i) mine = make_float4(g.x, g.y, d.x, d.y);
     }
     if (j0 + r <= jmax - 1) sc[(size_t) (j0 + r) * ncont_all] = mine;
-    A3 = nth_shfl(A, kNthLanes - 1);
-    T3 = nth_shfl(Tj, kNthLanes - 1);
+    A3 = nth_shfl<kNthLanes>(A, kNthLanes - 1);
+    T3 = nth_shfl<kNthLanes>(Tj, kNthLanes - 1);
   }
   // back sweep from j = jmax - 1 to 1: u, E F_E = x^4 u bt (donthcomp.c:603-610), the normalisation sum and the table;
-  // the lane's next point of the scratch is fetched ahead
+  // the lane's next points of the scratch are fetched ahead
   const int ih = min(G->ih0, jmax), il = ih - 1;
   float2 u = zero, qs = zero, s_il = zero, s_ih = zero;
-  float4 nx = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (jmax - 1 - r >= 2) nx = sc[(size_t) (jmax - 1 - r) * ncont_all];
-  for (int o = 0; o < jtop - 1; o += kNthLanes) {
+  constexpr int kAhead = 8 / kNthLanes;  // points of a lane in flight
+  float4 nx[kAhead];
+#pragma unroll
+  for (int e = 0; e < kAhead; e++) {
+    const int j = jmax - 1 - r - e * kNthLanes;
+    nx[e] = j >= 2 ? sc[(size_t) j * ncont_all] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int ox = 0; ox < jtop - 1; ox += kNthLanes * kAhead)
+#pragma unroll
+  for (int e = 0; e < kAhead; e++) {  // beyond the last point nothing is added or written
+    const int o = ox + e * kNthLanes;
     const int jr = jmax - 1 - o - r;
-    const float4 v = nx;
-    if (jr - kNthLanes >= 2) nx = sc[(size_t) (jr - kNthLanes) * ncont_all];
+    const float4 v = nx[e];
+    if (jr - kNthLanes * kAhead >= 2) nx[e] = sc[(size_t) (jr - kNthLanes * kAhead) * ncont_all];
     float2 uo = zero;
 #pragma unroll
     for (int i = 0; i < kNthLanes; i++) {
       const int j = jmax - 1 - o - i;
-      const float2 gi = nth_shfl(make_float2(v.x, v.y), i), di = nth_shfl(make_float2(v.z, v.w), i);
+      const float2 gi = nth_shfl<kNthLanes>(make_float2(v.x, v.y), i), di = nth_shfl<kNthLanes>(make_float2(v.z, v.w), i);
       if (j >= 2) u = nth_back(gi, di, u);
       else if (j == 1) u = ff_mul(C.aa, u);
       if (r == i) uo = u;
@@ -362,7 +372,7 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
     const float2 t = ff_mul(P.g, sp);
 #pragma unroll
     for (int i = 0; i < kNthLanes; i++) {
-      const float2 ti = nth_shfl(t, i);
+      const float2 ti = nth_shfl<kNthLanes>(t, i);
       if (jmax - 1 - o - i >= 1) qs = ff_add(qs, ti);
     }
     if (jr >= 1) {
@@ -374,8 +384,8 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
       }
     }
   }
-  s_il = nth_shfl(s_il, (jmax - 1 - il) & (kNthLanes - 1));  // zero where the point is jmax
-  s_ih = nth_shfl(s_ih, (jmax - 1 - ih) & (kNthLanes - 1));
+  s_il = nth_shfl<kNthLanes>(s_il, (jmax - 1 - il) & (kNthLanes - 1));  // zero where the point is jmax
+  s_ih = nth_shfl<kNthLanes>(s_ih, (jmax - 1 - ih) & (kNthLanes - 1));
   if (act && r == 0) {
     if (T) {
       T->sp[jmax] = 0.0;
@@ -548,15 +558,24 @@ __global__ void nthcomp_apply_kernel(RelxSetState *__restrict__ sst, int *__rest
 }
 
 cudaError_t nthcomp_set_smem() {
-  cudaError_t e = cudaFuncSetAttribute(nthcomp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int) (sizeof(NthPoint) * (RELX_NTH_N + 1)));
-  if (e != cudaSuccess) return e;
+  const int grid = (int) (sizeof(NthPoint) * (RELX_NTH_N + 1));
+  for (auto k : {nthcomp_kernel<1>, nthcomp_kernel<2>, nthcomp_kernel<4>}) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, grid);
+    if (e != cudaSuccess) return e;
+  }
   return cudaFuncSetAttribute(nthcomp_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int) sizeof(NthCoopSmem));
 }
 
 size_t nthcomp_scratch_bytes(int n_sets, int nza, bool params) {
   return (size_t) n_sets * (params ? 1 : nza + 1) * (kNthMaxJ + 1) * sizeof(float4);
+}
+
+// lanes per continuum: as many as still run in one wave of three CTAs per SM (us with 1 / 2 / 4 lanes: 3.3k continua
+// 407 / 289 / 215, 11k 409 / 320 / 277, 15k 413 / 328 / 446, 26k 464 / 381 / 525, 33k 473 / 653 / 712)
+static int nth_lanes(int64_t ncont) {
+  constexpr int64_t wave = 3 * 152 * (int64_t) kNthThreads;
+  return 4 * ncont <= wave ? 4 : 2 * ncont <= wave ? 2 : 1;
 }
 
 cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetIn *sin, RelxSetState *sst, int n_sets,
@@ -570,9 +589,10 @@ cudaError_t launch_nthcomp(cudaStream_t s, const RelxTables &tab, const RelxSetI
     nthcomp_coop_kernel<<<(unsigned) ncont, kNthCoopThreads, sizeof(NthCoopSmem), s>>>(tab.nth_grid, sin, sst, params,
                                                                                      per, nq, q, tabs);
   } else {
-    nthcomp_kernel<<<(unsigned) ((kNthLanes * ncont + kNthThreads - 1) / kNthThreads), kNthThreads,
-                     sizeof(NthPoint) * (RELX_NTH_N + 1), s>>>(tab.nth_grid, sin, sst, params, per, n_sets, nq, q,
-                                                              tabs, scr, ncont_all, c_off);
+    const int lanes = nth_lanes(ncont);
+    const auto kernel = lanes == 4 ? nthcomp_kernel<4> : lanes == 2 ? nthcomp_kernel<2> : nthcomp_kernel<1>;
+    kernel<<<(unsigned) ((lanes * ncont + kNthThreads - 1) / kNthThreads), kNthThreads, sizeof(NthPoint) * (RELX_NTH_N + 1), s>>>(
+        tab.nth_grid, sin, sst, params, per, n_sets, nq, q, tabs, scr, ncont_all, c_off);
   }
   if (!params) nthcomp_apply_kernel<<<n_sets, 128, 0, s>>>(sst, sflag, q, nq, cor, zcor);
   return cudaGetLastError();

@@ -22,14 +22,14 @@ def test_against_oracle(gpu, oracle, kte, gamma):
     assert_close(out[0], ref, f"kTe {kte} Gamma {gamma}")
 
 
-def test_few_and_many(gpu):
-    n = 1400  # beyond the continua that get a CTA each
+@pytest.mark.parametrize("n", [1400, 15000, 30000])  # four, two and one lanes per continuum
+def test_few_and_many(gpu, n):
     p = np.tile(gpu.default_params("xillverCp"), (n, 1))
     p[:, 2] = np.linspace(5.0, 400.0, n)
     p[:, 7] = 1.0
-    grid = GRID[::30]
+    grid = GRID[::60]
     many, st = gpu.eval_batch("xillverCp", p, [grid] * n)
     assert not st.any()
-    for i in (0, 1, 700, n - 1):
+    for i in (0, 1, 700, n // 2, n - 1):
         few, _ = gpu.eval_batch("xillverCp", p[i:i + 1], [grid])
         assert np.array_equal(few[0], many[i])
