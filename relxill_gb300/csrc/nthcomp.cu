@@ -340,6 +340,7 @@ __global__ void __launch_bounds__(kNthThreads) nthcomp_kernel(const NthGrid *__r
     A3 = nth_shfl<kNthLanes>(A, kNthLanes - 1);
     T3 = nth_shfl<kNthLanes>(Tj, kNthLanes - 1);
   }
+  __syncwarp();  // the back sweep's lanes load points that other lanes of the warp have stored (shuffles order no memory)
   // back sweep from j = jmax - 1 to 1: u, E F_E = x^4 u bt (donthcomp.c:603-610), the normalisation sum and the table;
   // the lane's next points of the scratch are fetched ahead
   const int ih = min(G->ih0, jmax), il = ih - 1;
