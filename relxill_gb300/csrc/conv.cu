@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(kConvThreads) relconv_rebin_kernel(RelxTables 
   __syncthreads();
   float v = 0.0f;
   if (dge(ehi0, ue[0]) && dge(ue[nu], elo0)) {
-    const int imin = at[tid], imax = min(at[tid + 1], nu - 1);
+    // a conv bin that starts at the caller's last edge lies beyond the caller's bins: no width, nothing of them
+    const int imin = min(at[tid], nu - 1), imax = min(at[tid + 1], nu - 1);
     const double elo = dgt(ue[imin], elo0) ? ue[imin] : elo0;
     const double ehi = dgt(ehi0, ue[imax + 1]) ? ue[imax + 1] : ehi0;
     if (imax == imin) {
