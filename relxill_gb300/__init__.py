@@ -219,6 +219,8 @@ def eval_batch(model: str, params, energies: Sequence[np.ndarray], flux_in: Opti
             raise ValueError(f"{model} needs the input spectra")
         if plain is None:
             fin = np.concatenate([np.asarray(f, dtype=np.float64) for f in flux_in])
+            if fin.size < nflux:
+                raise ValueError(f"the input spectra hold {fin.size} values, the grids {nflux} bins")
     igt = None if ion_grad_type is None else np.ascontiguousarray(ion_grad_type, dtype=np.int32)
     igi = None if iongrad_index is None else np.ascontiguousarray(iongrad_index, dtype=np.float64)
     tail = (_ptr(flux), _ptr(status, _ip), _ptr(igt, _ip) if igt is not None else None,
@@ -375,21 +377,31 @@ class Server:
         rid = self._submit(self._submit_fn, self._h, MODELS[model], len(PARAMS[model]), params, energy, out, flux_in,
                            ion_grad_type, iongrad_index)
         if rid is None:  # arrays that need a conversion, or a refusal
-            rid = self._submit_any(model, params, energy, out, flux_in, ion_grad_type, iongrad_index)
+            rid, flux_in = self._submit_any(model, params, energy, out, flux_in, ion_grad_type, iongrad_index)
         if rid < 0:
             raise RelxillError(int(-rid), last_error())
         self._keep[rid] = (energy, out, flux_in)
         return rid
 
-    def _submit_any(self, model, params, energy, out, flux_in, ion_grad_type, iongrad_index) -> int:
+    def _submit_any(self, model, params, energy, out, flux_in, ion_grad_type, iongrad_index):
+        """Returns the request's id (or a negative status) and the input spectrum as the library reads it."""
         p = np.ascontiguousarray(params, dtype=np.float64)
+        if p.size < len(PARAMS[model]):
+            raise ValueError(f"{model} takes {len(PARAMS[model])} parameters, got {p.size}")
         if energy.dtype != np.float64 or not energy.flags.c_contiguous:
             raise ValueError("energy must be a contiguous float64 array")
         if out.dtype != np.float64 or not out.flags.c_contiguous or len(out) != len(energy) - 1:
             raise ValueError("out must be a contiguous float64 array of len(energy) - 1")
-        return int(lib().relx_serve_submit(self._h, MODELS[model], _ptr(p), _ptr(energy), len(energy) - 1,
-                                           _ptr(flux_in) if flux_in is not None else None, _ptr(out),
-                                           int(ion_grad_type), float(iongrad_index)))
+        if model in CONV_MODELS and flux_in is not None:
+            if not isinstance(flux_in, np.ndarray):
+                raise ValueError("flux_in must be an array")
+            flux_in = np.ascontiguousarray(flux_in, dtype=np.float64)
+            if flux_in.size < len(out):
+                raise ValueError(f"flux_in holds {flux_in.size} values, the grid {len(out)} bins")
+        rid = lib().relx_serve_submit(self._h, MODELS[model], _ptr(p), _ptr(energy), len(energy) - 1,
+                                      _ptr(flux_in) if flux_in is not None else None, _ptr(out),
+                                      int(ion_grad_type), float(iongrad_index))
+        return int(rid), flux_in
 
     def poll(self, max_n: int = 4096) -> List[Tuple[int, int, float]]:
         ids = np.zeros(max_n, dtype=np.int64)
