@@ -243,6 +243,8 @@ def _lmod(model: str, energy, params, flux_in=None) -> np.ndarray:
     p = _as_params(model, params)[0].copy()
     nflux = len(e) - 1
     flux = np.zeros(nflux) if flux_in is None else np.array(flux_in, dtype=np.float64)
+    if flux.size < nflux:  # the library reads and writes one value per bin
+        raise ValueError(f"flux holds {flux.size} values, the grid {nflux} bins")
     getattr(L, LMOD_SYMBOL[model])(_ptr(e), nflux, _ptr(p), 0, _ptr(flux), None, None)
     st = L.relx_last_status()
     if st:

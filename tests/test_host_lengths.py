@@ -76,6 +76,14 @@ def test_eval_batch_refuses(rec):
     assert len(rec.spectra) == 1
 
 
+def test_local_model_refuses(rec):
+    for short in (np.ones(N - 1), np.ones(0)):
+        with pytest.raises(ValueError):
+            R.relconv(E, P, short)
+    assert not rec.spectra
+    assert R.relconv(E, P, np.ones(N + 2)).shape == (N + 2,)  # values beyond the bins are left alone
+
+
 @pytest.mark.gpu
 def test_served_spectra(gpu):
     f = np.arange(1.0, N + 1)
