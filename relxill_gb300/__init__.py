@@ -223,6 +223,9 @@ def eval_batch(model: str, params, energies: Sequence[np.ndarray], flux_in: Opti
                 raise ValueError(f"the input spectra hold {fin.size} values, the grids {nflux} bins")
     igt = None if ion_grad_type is None else np.ascontiguousarray(ion_grad_type, dtype=np.int32)
     igi = None if iongrad_index is None else np.ascontiguousarray(iongrad_index, dtype=np.float64)
+    for name, a in (("ion_grad_type", igt), ("iongrad_index", igi)):
+        if a is not None and a.size < n:
+            raise ValueError(f"{name} holds {a.size} values for {n} parameter sets")
     tail = (_ptr(flux), _ptr(status, _ip), _ptr(igt, _ip) if igt is not None else None,
             _ptr(igi) if igi is not None else None)
     if plain is not None:

@@ -84,6 +84,13 @@ def test_local_model_refuses(rec):
     assert R.relconv(E, P, np.ones(N + 2)).shape == (N + 2,)  # values beyond the bins are left alone
 
 
+@pytest.mark.parametrize("short", [dict(ion_grad_type=[1]), dict(ion_grad_type=[1, 1], iongrad_index=[0.5])])
+def test_gradients_refused(rec, short):
+    with pytest.raises(ValueError):
+        R.eval_batch("relxilllp", np.tile(R.default_params("relxilllp"), (2, 1)), [E, E], **short)
+    assert not rec.spectra
+
+
 @pytest.mark.gpu
 def test_served_spectra(gpu):
     f = np.arange(1.0, N + 1)
