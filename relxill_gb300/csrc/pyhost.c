@@ -15,7 +15,8 @@ static int plain(PyObject *o, void **p, Py_ssize_t *n) {
     PyErr_Clear();
     return 0;
   }
-  const int ok = v.ndim == 1 && v.itemsize == 8 && v.format && strcmp(v.format, "d") == 0;
+  /* v.obj: a buffer that another object provides (a class's __buffer__) may go with the release below */
+  const int ok = v.obj == o && v.ndim == 1 && v.itemsize == 8 && v.format && strcmp(v.format, "d") == 0;
   *p = v.buf;
   *n = v.len / 8;
   PyBuffer_Release(&v);
