@@ -139,16 +139,25 @@ def lib() -> ctypes.CDLL:
 
 
 def _host():
-    """The extension that reads arrays' addresses (csrc/pyhost.c)."""
+    """The extension that reads arrays' addresses (csrc/pyhost.c), or None where it has not been built for
+    this interpreter: the calls then join arrays with numpy, which takes longer and gives the same numbers."""
     global _host_ext
     if _host_ext is None:
-        if not os.path.exists(HOST_EXT_PATH):
-            raise RuntimeError(f"{HOST_EXT_PATH} is missing: build it with `python -m relxill_gb300.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_relx_host", HOST_EXT_PATH)
-        ext = importlib.util.module_from_spec(importlib.util.spec_from_loader("_relx_host", loader))
-        loader.exec_module(ext)
-        _host_ext = ext
-    return _host_ext
+        _host_ext = False
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("_relx_host", HOST_EXT_PATH)
+            ext = importlib.util.module_from_spec(importlib.util.spec_from_loader("_relx_host", loader))
+            loader.exec_module(ext)
+            _host_ext = ext
+        except ImportError:
+            pass
+    return _host_ext or None
+
+
+def _addresses(arrays: list):
+    """Addresses and lengths of plain arrays, or None (some need a conversion, or there is no extension)."""
+    host = _host()
+    return None if host is None else host.arrays(arrays)
 
 
 def _ptr(a: np.ndarray, t=_dp):
@@ -197,10 +206,10 @@ def eval_batch(model: str, params, energies: Sequence[np.ndarray], flux_in: Opti
     if len(energies) != n:
         raise ValueError("one energy grid per parameter set")
     energies = list(energies)  # the arrays stay alive and in place while their addresses are in use
-    plain = _host().arrays(energies)
+    plain = _addresses(energies)
     if plain is not None and model in CONV_MODELS and flux_in is not None:
         flux_in = list(flux_in)
-        spectra = _host().arrays(flux_in)
+        spectra = _addresses(flux_in)
         # as many values as bins in each, or they are joined as they come
         if spectra is None or not np.array_equal(np.frombuffer(spectra[1], np.int64) + 1,
                                                  np.frombuffer(plain[1], np.int64)):
@@ -374,13 +383,15 @@ class Server:
         if not self._h:
             raise RelxillError(last_status_or(6), last_error())
         self._keep: Dict[int, tuple] = {}
-        self._submit = _host().submit
-        self._submit_fn = ctypes.cast(L.relx_serve_submit, ctypes.c_void_p).value
+        host = _host()
+        self._submit = None if host is None else host.submit
+        self._submit_fn = None if host is None else ctypes.cast(L.relx_serve_submit, ctypes.c_void_p).value
 
     def submit(self, model: str, params, energy: np.ndarray, out: np.ndarray, flux_in: Optional[np.ndarray] = None,
                ion_grad_type: int = 0, iongrad_index: float = 0.0) -> int:
-        rid = self._submit(self._submit_fn, self._h, MODELS[model], len(PARAMS[model]), params, energy, out, flux_in,
-                           ion_grad_type, iongrad_index)
+        rid = None if self._submit is None else self._submit(
+            self._submit_fn, self._h, MODELS[model], len(PARAMS[model]), params, energy, out, flux_in, ion_grad_type,
+            iongrad_index)
         if rid is None:  # arrays that need a conversion, or a refusal
             rid, flux_in = self._submit_any(model, params, energy, out, flux_in, ion_grad_type, iongrad_index)
         if rid < 0:

@@ -40,9 +40,12 @@ def _compile(src: str, obj: str, verbose: bool) -> str:
 
 
 def _compile_host_ext() -> str:
-    cc = shutil.which("gcc") or shutil.which("cc") or "gcc"
-    cmd = [cc, "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], os.path.join(SRC, "pyhost.c"),
-           "-o", HOST_EXT]
+    """Compiles the Python layer's extension; without a C compiler or Python's headers the package does without it."""
+    cc = shutil.which("gcc") or shutil.which("cc")
+    include = sysconfig.get_paths()["include"]
+    if cc is None or not os.path.exists(os.path.join(include, "Python.h")):
+        return f"pyhost.c not compiled: no {'C compiler' if cc is None else 'Python.h in ' + include}\n"
+    cmd = [cc, "-O2", "-Wall", "-shared", "-fPIC", "-I", include, os.path.join(SRC, "pyhost.c"), "-o", HOST_EXT]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"gcc failed for pyhost.c:\n{r.stdout}\n{r.stderr}")
