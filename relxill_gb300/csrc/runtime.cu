@@ -1078,6 +1078,17 @@ __global__ void __launch_bounds__(kStageThreads) out_kernel(int64_t n_flux, cons
   if (dstatus)
     for (int64_t i = t; i < n_sets; i += stride) dstatus[i] = status[i];
 }
+// Whether a kernel on the current device can use a caller's array of elements of this size.  The copy engines also
+// reach arrays that are not aligned to their elements, and memory of other devices that this one does not map.
+static bool kernel_reaches(const void *p, size_t size) {
+  cudaPointerAttributes at;
+  if ((uintptr_t) p % size) return false;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.devicePointer != nullptr;
+}
 // CTAs for n grid-stride items
 static int stage_ctas(int64_t n) { return (int) std::max<int64_t>(1, std::min<int64_t>((n + kStageThreads - 1) / kStageThreads, 8 * 152)); }
 
@@ -2013,15 +2024,22 @@ int relx_eval_batch_device(int model, int n_sets, const double *d_params, const 
   a.eoff = d_energy_offsets;
   a.igt = d_ion_grad_type;
   a.igi = d_iongrad_index;
-  a.e_src = d_energy;
-  a.f_src = conv ? d_flux_in : nullptr;
+  a.e_src = kernel_reaches(d_energy, sizeof(double)) ? d_energy : nullptr;
+  a.f_src = conv && kernel_reaches(d_flux_in, sizeof(double)) ? d_flux_in : nullptr;
+  const size_t ebytes = sizeof(double) * b.n_edges;
+  if (!a.e_src) RELX_CUDA(cudaMemcpyAsync(W.user_e.p, d_energy, ebytes, cudaMemcpyDeviceToDevice, s));
+  if (conv && !a.f_src) RELX_CUDA(cudaMemcpyAsync(W.user_f.p, d_flux_in, ebytes, cudaMemcpyDeviceToDevice, s));
   launch_stage(W, b, env, s, a);
   if ((st = tuned_launch(C, W, b, s, true))) return st;
   const int64_t nflux = b.n_edges - n_sets;
-  {
+  const bool fk = kernel_reaches(d_flux, sizeof(double)), sk = d_status && kernel_reaches(d_status, sizeof(int));
+  if (!fk) RELX_CUDA(cudaMemcpyAsync(d_flux, W.flux.p, sizeof(double) * nflux, cudaMemcpyDeviceToDevice, s));
+  if (d_status && !sk)
+    RELX_CUDA(cudaMemcpyAsync(d_status, W.status.p, sizeof(int) * n_sets, cudaMemcpyDeviceToDevice, s));
+  if (fk || sk) {
     ProfScope ps(PK_STATUS, s);
-    out_kernel<<<stage_ctas(nflux), kStageThreads, 0, s>>>(nflux, W.flux.as<double>(), d_flux, n_sets, W.status.as<int>(),
-                                                           d_status);
+    out_kernel<<<stage_ctas(fk ? nflux : n_sets), kStageThreads, 0, s>>>(fk ? nflux : 0, W.flux.as<double>(), d_flux, n_sets,
+                                                                         W.status.as<int>(), sk ? d_status : nullptr);
   }
   RELX_CUDA(cudaGetLastError());
   return 0;
