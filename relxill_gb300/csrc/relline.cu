@@ -1297,6 +1297,7 @@ __device__ __noinline__ int cosne_bin_fp64(const RelxTables &tab, const RelxSetS
 // shared memory with two barriers per 128 radii; with the points unrolled, a radius's loads in flight together, the
 // next radius's record fetched ahead and flushes without branches 681 us, 177 us and 35 us.
 constexpr int kHistFull = 5;  // the 40 points of the relline tables, 5 for each of 8 lanes
+constexpr int kHistFew = 3;   // tables of up to 24 points
 
 template <int GP>
 struct HistLane {
@@ -1304,8 +1305,8 @@ struct HistLane {
   float gsf[GP], gfac[GP];
 };
 
-// class w of zone [i0, i1]; the lane's sums end in lh
-template <int GP>
+// class w of zone [i0, i1]; the lane's sums end in lh; FULL: every lane has GP points
+template <int GP, bool FULL>
 __device__ __forceinline__ void hist_class(const RelxTables &tab, const RelxSetState &s, const RelxRadial &R,
                                            const float2 *__restrict__ T, const HistLane<GP> &L, int i0, int i1, int w,
                                            float *lh) {
@@ -1354,7 +1355,7 @@ __device__ __forceinline__ void hist_class(const RelxTables &tab, const RelxSetS
       for (int k = 0; k < 2; k++) {
         const float x = __fmaf_rn(wh_, k ? wh[e].y : wh[e].x, __fmaf_rn(wl_, k ? wl[e].y : wl[e].x, fn - 0.5f));
         const float q = __fadd_rn(x, kMagic);
-        edge = fmaxf(edge, fabsf(__fadd_rn(x, -__fadd_rn(q, -kMagic))));
+        if (FULL || e < L.np) edge = fmaxf(edge, fabsf(__fadd_rn(x, -__fadd_rn(q, -kMagic))));
         b[e][k] = max(kMagicBits, min(__float_as_int(q), kMagicBits + n_incl - 1));
       }
     }
@@ -1407,7 +1408,7 @@ __device__ __forceinline__ void hist_class(const RelxTables &tab, const RelxSetS
         const bool in = on && e < L.np;
         const bool f0 = in && b[e][0] != cur[0], f1 = in && b[e][1] != cur[1];
         flush(f0, f1);
-        if (GP != kHistFull && !in) continue;
+        if (!FULL && !in) continue;
         run[0] = __fmaf_rn(cg, t0, f0 ? 0.0f : run[0]);
         run[1] = __fadd_rn(f1 ? 0.0f : run[1], __fmul_rn(cg, t1));
       }
@@ -1435,8 +1436,8 @@ __device__ __forceinline__ float hist_lanes(float (*lh)[32], int n_incl) {
   return h;
 }
 
-template <int GP>
-__global__ void __launch_bounds__(kHistWarps * 32, GP == kHistFull ? 3 : 1)
+template <int GP, bool FULL>
+__global__ void __launch_bounds__(kHistWarps * 32, GP <= kHistFew ? 4 : GP <= kHistFull ? 3 : 2)
     hist_kernel(RelxTables tab, const RelxSetState *__restrict__ sst, const RelxRadial *__restrict__ srad, int nza,
                 const float4 *__restrict__ htab, float *__restrict__ dist) {
   __shared__ float lhs[kHistWarps][RELX_MAX_INCL + 1][32];  // per-lane histograms, lane fastest (no bank conflicts), and a row for nothing
@@ -1446,9 +1447,9 @@ __global__ void __launch_bounds__(kHistWarps * 32, GP == kHistFull ? 3 : 1)
   if (s.status != RELX_OK || s.model < RELX_RELXILL || s.cached || z >= s.nz) return;
   const int ng = tab.rel_ng, n_incl = tab.x_nincl;
   HistLane<GP> L;
-  const int gper = GP == kHistFull ? kHistFull : (ng + 7) >> 3;
+  const int gper = FULL ? GP : (ng + 7) >> 3;
   L.g0 = (lane & 7) * gper;
-  L.np = GP == kHistFull ? kHistFull : max(0, min(gper, ng - L.g0));
+  L.np = FULL ? GP : max(0, min(gper, ng - L.g0));
 #pragma unroll
   for (int e = 0; e < GP; e++) {
     const float2 g = __ldg(&tab.rel_gs[min(L.g0 + e, ng - 1)]);
@@ -1459,7 +1460,7 @@ __global__ void __launch_bounds__(kHistWarps * 32, GP == kHistFull ? 3 : 1)
   const float2 *__restrict__ T = reinterpret_cast<const float2 *>(htab + (size_t) set * tab.rel_nr * ng) + min(L.g0, ng - 1);
   float(*lh)[32] = lhs[warp];
   for (int j = 0; j <= RELX_MAX_INCL; j++) lh[j][lane] = 0.0f;
-  hist_class<GP>(tab, s, srad[set], T, L, s.zi0[z], s.zi1[z], warp, &lh[0][lane]);
+  hist_class<GP, FULL>(tab, s, srad[set], T, L, s.zi0[z], s.zi1[z], warp, &lh[0][lane]);
   const float h = hist_lanes(lh, n_incl);
   if (lane < n_incl) hw[warp][lane] = h;
   __syncthreads();
@@ -1557,13 +1558,21 @@ cudaError_t launch_relline(int n_sets, int nblk, cudaStream_t s, const RelxTable
   return cudaGetLastError();
 }
 
+// The instance by the points of a lane: with fewer unrolled points than eight more CTAs fit an SM.  4096 relxilllp sets,
+// histograms, us: tables of 20 points 2280 by the instance of eight points whose missing points all counted as near an
+// edge, so 479 (a loop over the points before that 587); 33 points 2618, so 755 (774); 64 points 2339 at one CTA per SM,
+// so 1500 at two (1467).
 cudaError_t launch_hist(int n_sets, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
                         const RelxRadial *srad, int nza, float *dist, const float4 *htab) {
   const dim3 grid(nza, n_sets);
   if (tab.rel_ng == 8 * kHistFull)
-    hist_kernel<kHistFull><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
+    hist_kernel<kHistFull, true><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
+  else if (tab.rel_ng <= 8 * kHistFew)
+    hist_kernel<kHistFew, false><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
+  else if (tab.rel_ng < 8 * kHistFull)
+    hist_kernel<kHistFull, false><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
   else
-    hist_kernel<RELX_MAX_NG / 8><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
+    hist_kernel<RELX_MAX_NG / 8, false><<<grid, kHistWarps * 32, 0, s>>>(tab, sst, srad, nza, htab, dist);
   return cudaGetLastError();
 }
 
