@@ -1505,15 +1505,19 @@ cudaError_t relline_set_smem(int nr, int ng) {
 // the GPU several times; up to there the team kernel, which spends about half as much again per bin on
 // narrower tiles and its ordered sums, is ahead.  Measured (line profile, us, solo / team): 10 zones
 // 128 sets 290 / 190, 256 360 / 370, 512 440 / 620; 25 zones 32 sets 145 / 145, 128 200 / 250; one
-// zone 1024 sets 1280 / 1040, 2048 1690 / 2000.
-static bool line_solo(int n_sets, int nza) { return (int64_t) n_sets * nza >= (nza > 1 ? 2560 : 1536); }
+// zone 1024 sets 1280 / 1040, 2048 1690 / 2000.  Between few table points the interpolant jumps so far that most bins
+// need more than two Romberg levels, which a warp does one after the other: one zone, 20 points, 1600 sets
+// 2670 / 1540, 4096 5020 / 3420 (12 points, 8192 sets 6890 / 6730); from 24 points on as above (4096 sets 2860 / 2950).
+static bool line_solo(int n_sets, int nza, int ng) {
+  return nza > 1 ? (int64_t) n_sets * nza >= 2560 : n_sets >= 1536 && ng >= 24;
+}
 
 // list: line_list_entries() entries for the solo kernel's tasks, cnt: its two counters (zero); both may be
 // null (then the team kernel runs whatever the number of sets)
 cudaError_t launch_line_table(int n_sets, int nza, cudaStream_t s, const RelxTables &tab, const RelxSetState *sst,
                               float4 *htab, RelxRadial *srad, uint2 *list, int *cnt) {
   const int nq = tab.rel_nr * tab.rel_ng;
-  const bool solo = list && line_solo(n_sets, nza);
+  const bool solo = list && line_solo(n_sets, nza, tab.rel_ng);
   line_table_kernel<<<dim3((nq + kLineThreads - 1) / kLineThreads, n_sets), kLineThreads, 0, s>>>(
       tab, sst, htab, srad, solo ? list : nullptr, cnt, kSoloTile);
   return cudaGetLastError();
@@ -1546,7 +1550,7 @@ static void launch_team(int n_sets, int nblk, cudaStream_t s, const RelxTables &
 cudaError_t launch_relline(int n_sets, int nblk, cudaStream_t s, const RelxTables &tab, const RelxSetIn *sin,
                            const RelxSetState *sst, const RelxRadial *srad, const double *line_e, int nza, float *prof,
                            double *tsum, bool any_limb, const float4 *htab, const uint2 *list, int *cnt) {
-  if (list && line_solo(n_sets, nza)) {
+  if (list && line_solo(n_sets, nza, tab.rel_ng)) {
     const int64_t most = (int64_t) line_list_entries(n_sets, nza, nblk);
     const int grid = (int) std::min<int64_t>(152 * kSoloCtas, (most + kSoloWarps - 1) / kSoloWarps);
     relline_solo_kernel<kSoloTile><<<grid, kSoloWarps * 32, line_solo_smem(tab.rel_ng), s>>>(
