@@ -732,13 +732,25 @@ __device__ __forceinline__ bool line_group(const RelxTables &tab, const RelxSetS
       }
     } else {
       const float2 *__restrict__ C = T + tab.rel_nr * ng;
+      // The points [pa, pb) that the tile's bins reach: an abscissa between its ends reads the point below it, one
+      // further down where it lies on a point, and the next; one point more either side than that.  Points 1 and
+      // ng - 2 of line_edges are among them where a bin has an edge term.  (All points of four functions cost a tile of 32
+      // bins more than its bins: 4096 relline sets, 64 points 6.08 ms so, 5.57 ms with these.)
+      int pa = 0, pb = ng;
+      {
+        RadL q;
+        line_rad(q, rr);
+        const float xa = edge_gc(eff[0], q).x, xb = edge_gc(eff[thi - tlo], q).x;
+        if (xa > kH) pa = max(0, (int) ((xa - kH) * lc.inv_dgs) - 2) & ~1;
+        if (xb < 1.0f - kH) pb = min(ng, (int) ((fmaxf(xb, kH) - kH) * lc.inv_dgs) + 4);
+      }
       if ((ng & 1) == 0) {
         const float4 *thi4 = reinterpret_cast<const float4 *>(T + it * ng);
         const float4 *tlo4 = reinterpret_cast<const float4 *>(T + (it + 1) * ng);
         const float4 *chi4 = reinterpret_cast<const float4 *>(C + it * ng);
         const float4 *clo4 = reinterpret_cast<const float4 *>(C + (it + 1) * ng);
 #pragma unroll 2
-        for (int g = sub; g < ng >> 1; g += kRadLanes) {
+        for (int g = (pa >> 1) + sub; 2 * g < pb; g += kRadLanes) {
           const float4 lo = __ldg(tlo4 + g), hi = __ldg(thi4 + g), cl = __ldg(clo4 + g), ch = __ldg(chi4 + g);
           tw[2 * g].t = make_float4(sum2(fr1, lo.x, fr, hi.x), sum2(fr1, lo.y, fr, hi.y), sum2(fr1, cl.x, fr, ch.x),
                                     sum2(fr1, cl.y, fr, ch.y));
@@ -746,7 +758,7 @@ __device__ __forceinline__ bool line_group(const RelxTables &tab, const RelxSetS
                                         sum2(fr1, cl.z, fr, ch.z), sum2(fr1, cl.w, fr, ch.w));
         }
       } else {
-        for (int g = sub; g < ng; g += kRadLanes) {
+        for (int g = pa + sub; g < pb; g += kRadLanes) {
           const float2 lo = __ldg(&T[(it + 1) * ng + g]), hi = __ldg(&T[it * ng + g]);
           const float2 cl = __ldg(&C[(it + 1) * ng + g]), ch = __ldg(&C[it * ng + g]);
           tw[g].t = make_float4(sum2(fr1, lo.x, fr, hi.x), sum2(fr1, lo.y, fr, hi.y), sum2(fr1, cl.x, fr, ch.x),
