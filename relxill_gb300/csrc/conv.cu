@@ -487,7 +487,6 @@ __device__ __forceinline__ double rebin_bin(const RelxTables &tab, double elo0, 
 
 struct FinSmem {
   float spec[kN];
-  double red[kFinThreads / 32 + 1];
   float nrm;
   double nth_norm;  // nthcomp: 1 / (E F_E at the shifted 1 keV point)
 };

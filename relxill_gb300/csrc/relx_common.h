@@ -116,7 +116,6 @@ struct RelxTables {
   // conv grid and precomputed maps
   const double *conv_e;      // [RELX_NCONV+1]
   const float2 *conv_eff;    // float-float edges
-  const float *conv_inv_emid;  // 1/(0.5(e_j+e_j+1))
   const float *conv_cf;      // 0.5(e_j+e_j+1)/(e_j+1-e_j)  (Relbase.cpp:93-103)
   const float2 *conv_cw;     // (float) 0.5(e_j+e_j+1), (float) (e_j+1-e_j)
   int conv_pos1;             // binary_search(conv_e, 1.0)  (Relbase.cpp:133-137)

@@ -71,40 +71,6 @@ __device__ __forceinline__ int conv_index(const RelxTables &tab, double e) {
   return k;
 }
 
-// Searches over FP64 arrays guided by float copies.  Rounding to float is monotone, so a strict
-// float comparison decides the FP64 one; only float ties are compared in FP64 (FP64 compares
-// share the narrow FP64 pipe).
-// number of entries of the descending array a that are > v
-__device__ __forceinline__ int count_gt_desc(const double *a, const float *af, int n, double v, float vf) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int k = (lo + hi) >> 1;
-    if (af[k] > vf) lo = k + 1; else hi = k;
-  }
-  while (lo < n && af[lo] == vf && a[lo] > v) lo++;
-  return lo;
-}
-// bsearch_asc (largest k in [0, n-2] with a[k] <= v, 0 below the range) of an ascending array
-__device__ __forceinline__ int bsearch_asc_exact(const double *a, const float *af, int n, double v, float vf) {
-  int lo = 0, hi = n;  // count of entries < v in float
-  while (lo < hi) {
-    const int k = (lo + hi) >> 1;
-    if (af[k] < vf) lo = k + 1; else hi = k;
-  }
-  while (lo < n && af[lo] == vf && a[lo] <= v) lo++;  // lo = count of entries <= v
-  return max(0, min(lo - 1, n - 2));
-}
-// bsearch_desc of a strictly descending array (the largest k in [0, n-2] with a[k] >= v, 0 when
-// there is none), guided by the float copy af
-__device__ __forceinline__ int bsearch_desc_exact(const double *a, const float *af, int n, double v, float vf) {
-  int lo = 0, hi = n;  // count of entries > v in float
-  while (lo < hi) {
-    const int k = (lo + hi) >> 1;
-    if (af[k] > vf) lo = k + 1; else hi = k;
-  }
-  while (lo < n && af[lo] == vf && a[lo] >= v) lo++;  // lo = count of entries >= v
-  return max(0, min(lo - 1, n - 2));
-}
 // descending arr (inv_binary_search, relutility.c:195-211)
 __device__ __forceinline__ int bsearch_desc(const double *arr, int n, double val) {
   int klo = 0, khi = n - 1;
@@ -192,17 +158,6 @@ __device__ __forceinline__ float2 ff_split(double d) {
 // ulp there; elsewhere both roundings are an ulp of the result
 __device__ __forceinline__ float ff_diff(float2 a, float2 b) {
   return __fadd_rn(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
-}
-// a > b and a >= b for doubles with their float roundings af, bf: rounding to float is monotone,
-// so float copies that differ decide, and only tied copies are compared in FP64
-__device__ __forceinline__ bool gt_f(double a, float af, double b, float bf) { return af != bf ? af > bf : a > b; }
-__device__ __forceinline__ bool ge_f(double a, float af, double b, float bf) { return af != bf ? af > bf : a >= b; }
-// (a.hi + a.lo) - (b.hi + b.lo) rounded to float, error ~1 ulp of the result
-__device__ __forceinline__ float ff_sub_to_float(float2 a, float2 b) {
-  float s = __fsub_rn(a.x, b.x);
-  float bb = __fsub_rn(s, a.x);
-  float err = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, bb)), __fsub_rn(-b.x, bb));  // two-sum error
-  return __fadd_rn(s, __fadd_rn(err, __fsub_rn(a.y, b.y)));
 }
 
 // ---- float-float arithmetic on the FP32 pipe (FP64 runs at 1/64 of the FP32 rate on this part)

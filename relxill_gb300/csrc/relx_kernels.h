@@ -10,13 +10,11 @@
 
 namespace relx {
 
-constexpr int kLineThreadsH = 256;
 constexpr int kSumBinsH = 32;    // bins per profile-sum block (tsum)
 constexpr int kLineTileH = 128;   // bins per task of the line profile of many sets
 constexpr int kConvThreadsH = 256;
 constexpr int kFinThreadsH = 128;
 
-size_t hist_smem_bytes(int nr, int ng);
 size_t conv_smem_bytes();
 
 cudaError_t setup_set_smem();

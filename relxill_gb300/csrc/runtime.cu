@@ -233,12 +233,12 @@ struct Tables {
   RelxTables dcp{};     // d with the xillver fields of the nthcomp table (valid if has_cp)
   bool has_cp = false;
   DevBuf rr_spin, rr_rlo, rr_rhi, rr_tfr, rr_g;
-  DevBuf conv_e, conv_eff, conv_inv_emid, conv_cf, conv_cw, coarse_e, coarse_t, nth_grid;
+  DevBuf conv_e, conv_eff, conv_cf, conv_cw, coarse_e, coarse_t, nth_grid;
   size_t bytes_total = 0;
   bool loaded = false;
   void release() {
     for (DevBuf *b : {&rel_a, &rel_mu0, &rel_r, &rel_gmin, &rel_gmax, &rel_tc, &rel_gs, &lp_a, &lp_h, &lp_rad, &lp_intens,
-                      &lp_del, &lp_delinc, &rr_spin, &rr_rlo, &rr_rhi, &rr_tfr, &rr_g, &conv_e, &conv_eff, &conv_inv_emid, &conv_cf,
+                      &lp_del, &lp_delinc, &rr_spin, &rr_rlo, &rr_rhi, &rr_tfr, &rr_g, &conv_e, &conv_eff, &conv_cf,
                       &conv_cw, &coarse_e, &coarse_t, &nth_grid})
       b->release();
     x.release();
@@ -674,7 +674,7 @@ static int load_tables(const std::string &dir, Tables &T) {
   std::vector<double> ce;
   log_grid(ce, RELX_NCONV + 1, RELX_EMIN_CONV, RELX_EMAX_CONV);
   std::vector<float2> ceff(ce.size());
-  std::vector<float> inv_emid(RELX_NCONV), cf(RELX_NCONV);
+  std::vector<float> cf(RELX_NCONV);
   std::vector<float2> cw(RELX_NCONV);
   for (size_t i = 0; i < ce.size(); i++) {
     float hi = (float) ce[i];
@@ -682,7 +682,6 @@ static int load_tables(const std::string &dir, Tables &T) {
   }
   int band_lo = RELX_NCONV, band_hi = -1;
   for (int j = 0; j < RELX_NCONV; j++) {
-    inv_emid[j] = (float) (1.0 / (0.5 * (ce[j] + ce[j + 1])));
     cf[j] = (float) (0.5 * (ce[j] + ce[j + 1]) / (ce[j + 1] - ce[j]));  // Relbase.cpp:93-103
     cw[j] = make_float2((float) (0.5 * (ce[j] + ce[j + 1])), (float) (ce[j + 1] - ce[j]));
     if (ce[j] >= RELX_EMIN_XILL && ce[j + 1] < RELX_EMAX_XILL) {   // Relbase.cpp:205
@@ -748,13 +747,12 @@ static int load_tables(const std::string &dir, Tables &T) {
     return 0;
   };
   if ((st = rebin_tables(xe, T.x, T.d)) || (has_cp && (st = rebin_tables(xe_cp, T.xcp, T.dcp)))) return st;
-  if ((st = upload(T.conv_e, ce)) || (st = upload(T.conv_eff, ceff)) || (st = upload(T.conv_inv_emid, inv_emid)) ||
+  if ((st = upload(T.conv_e, ce)) || (st = upload(T.conv_eff, ceff)) ||
       (st = upload(T.conv_cf, cf)) || (st = upload(T.conv_cw, cw)) || (st = upload(T.coarse_e, co)) ||
       (st = upload(T.coarse_t, ct)))
     return st;
   T.d.conv_e = T.conv_e.as<double>();
   T.d.conv_eff = T.conv_eff.as<float2>();
-  T.d.conv_inv_emid = T.conv_inv_emid.as<float>();
   T.d.conv_cf = T.conv_cf.as<float>();
   T.d.conv_cw = T.conv_cw.as<float2>();
   T.d.conv_pos1 = pos1;
