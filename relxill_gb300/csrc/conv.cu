@@ -653,7 +653,7 @@ cudaError_t launch_relconv(cudaStream_t s, const RelxTables &tab, int n_sets, in
   relconv_rebin_kernel<<<dim3(n_sets, kN / kConvThreads), kConvThreads, 0, s>>>(tab, sin, sst, user_e, user_f, xs);
   relconv_conv_kernel<<<n_sets, kConvThreads, sizeof(ConvSmem), s>>>(tab, sin, sst, prof, tsum, nblk, nza, user_f, xs,
                                                                      cout, sflag, err);
-  finalize_relconv_kernel<<<dim3(n_sets, out_parts(n_sets, n_bins, kFinThreads, 608)), kFinThreads, 0, s>>>(
+  finalize_relconv_kernel<<<dim3(n_sets, out_parts(n_sets, n_bins, kFinThreads, 4 * kSMs)), kFinThreads, 0, s>>>(
       tab, sin, sst, cout, nza, user_e, flux, so);
   return cudaGetLastError();
 }
@@ -669,7 +669,7 @@ cudaError_t launch_finalize_relxill(cudaStream_t s, bool few, int n_sets, int64_
                                     const double *user_e, double *flux, const NthTable *nth, const StatusOut &so) {
   if (n_sets <= 0) return cudaSuccess;
   if (few)
-    finalize_relxill_kernel<512><<<dim3(n_sets, out_parts(n_sets, n_bins, 512, 304)), 512, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e, flux, nth, so);
+    finalize_relxill_kernel<512><<<dim3(n_sets, out_parts(n_sets, n_bins, 512, 2 * kSMs)), 512, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e, flux, nth, so);
   else
     finalize_relxill_kernel<kFinThreads><<<n_sets, kFinThreads, sizeof(FinSmem), s>>>(tab, sin, sst, cout, nza, user_e, flux, nth, so);
   return cudaGetLastError();

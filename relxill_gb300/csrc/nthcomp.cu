@@ -420,7 +420,7 @@ static_assert(3 * (sizeof(NthCoopSmem) + 1024) <= 228 * 1024, "three CTAs per SM
 constexpr int kNthCoopThreads = 128;
 constexpr int kNthChunk = 64;
 // one wave of three CTAs per SM (456 continua 108 us, by four lanes each 197 us; 912 209 us and 199 us)
-constexpr int kNthCoop = 3 * 152;
+constexpr int kNthCoop = 3 * kSMs;
 
 __global__ void __launch_bounds__(kNthCoopThreads) nthcomp_coop_kernel(const NthGrid *__restrict__ G,
                                                                        const RelxSetIn *__restrict__ sin,
@@ -575,7 +575,7 @@ size_t nthcomp_scratch_bytes(int n_sets, int nza, bool params) {
 // lanes per continuum: as many as still run in one wave of three CTAs per SM (us with 1 / 2 / 4 lanes: 3.3k continua
 // 407 / 289 / 215, 11k 409 / 320 / 277, 15k 413 / 328 / 446, 26k 464 / 381 / 525, 33k 473 / 653 / 712)
 static int nth_lanes(int64_t ncont) {
-  constexpr int64_t wave = 3 * 152 * (int64_t) kNthThreads;
+  constexpr int64_t wave = 3 * kSMs * (int64_t) kNthThreads;
   return 4 * ncont <= wave ? 4 : 2 * ncont <= wave ? 2 : 1;
 }
 

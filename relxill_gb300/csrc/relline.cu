@@ -1520,6 +1520,9 @@ cudaError_t relline_set_smem(int nr, int ng) {
 // zone 1024 sets 1280 / 1040, 2048 1690 / 2000.  Between few table points the interpolant jumps so far that most bins
 // need more than two Romberg levels, which a warp does one after the other: one zone, 20 points, 1600 sets
 // 2670 / 1540, 4096 5020 / 3420 (12 points, 8192 sets 6890 / 6730); from 24 points on as above (4096 sets 2860 / 2950).
+// A limb law always runs in the team kernel: there is no solo form with the law's twice as many table functions, which
+// leave a warp 12 KB.  Line profile of relline with a law, us, now / by a CTA per 512 bins before: 153 sets 430 / 860, 1100
+// 1570 / 1900, 4096 5350 / 5540 (64 points 5570 / 5650).
 static bool line_solo(int n_sets, int nza, int ng) {
   return nza > 1 ? (int64_t) n_sets * nza >= 2560 : n_sets >= 1536 && ng >= 24;
 }
@@ -1546,7 +1549,7 @@ static void launch_team(int n_sets, int nblk, cudaStream_t s, const RelxTables &
   // 39 / 36 / 31, 8 54 / 47 / 54, 32 86 / 89 / 110.  (A limb law doubles the transfer functions: 16 at most.)
   const int nw = nza > 1 ? (n_sets * nza <= 160 ? 16 : 8) : LIMB ? (n_sets <= 64 ? 16 : 8)
                  : n_sets <= 32 ? 32 : n_sets <= 128 ? 16 : 8;
-  const int gx = std::max(1, std::min(nblk + nza, 4 * 152 * 32 / (nw * n_sets)));
+  const int gx = std::max(1, std::min(nblk + nza, 4 * kSMs * 32 / (nw * n_sets)));
   const dim3 grid(gx, n_sets);
 #define TEAM(NW)                                                                                             \
   if (nw == NW)                                                                                              \
@@ -1564,7 +1567,7 @@ cudaError_t launch_relline(int n_sets, int nblk, cudaStream_t s, const RelxTable
                            double *tsum, bool any_limb, const float4 *htab, const uint2 *list, int *cnt) {
   if (list && line_solo(n_sets, nza, tab.rel_ng)) {
     const int64_t most = (int64_t) line_list_entries(n_sets, nza, nblk);
-    const int grid = (int) std::min<int64_t>(152 * kSoloCtas, (most + kSoloWarps - 1) / kSoloWarps);
+    const int grid = (int) std::min<int64_t>(kSMs * kSoloCtas, (most + kSoloWarps - 1) / kSoloWarps);
     relline_solo_kernel<kSoloTile><<<grid, kSoloWarps * 32, line_solo_smem(tab.rel_ng), s>>>(
         tab, sin, sst, srad, line_e, htab, nza, prof, tsum, nblk, list, cnt, line_const(tab.rel_ng));
   } else {

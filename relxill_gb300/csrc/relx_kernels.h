@@ -10,6 +10,7 @@
 
 namespace relx {
 
+constexpr int kSMs = 152;          // of the GPU the launch shapes are measured on
 constexpr int kSumBinsH = 32;    // bins per profile-sum block (tsum)
 constexpr int kLineTileH = 128;   // bins per task of the line profile of many sets
 constexpr int kConvThreadsH = 256;

@@ -1088,7 +1088,7 @@ static bool kernel_reaches(const void *p, size_t size) {
   return at.devicePointer != nullptr;
 }
 // CTAs for n grid-stride items
-static int stage_ctas(int64_t n) { return (int) std::max<int64_t>(1, std::min<int64_t>((n + kStageThreads - 1) / kStageThreads, 8 * 152)); }
+static int stage_ctas(int64_t n) { return (int) std::max<int64_t>(1, std::min<int64_t>((n + kStageThreads - 1) / kStageThreads, 8 * kSMs)); }
 
 // ---- optional per-kernel timing with CUDA events on the launching stream ----
 enum ProfKernel { PK_PACK, PK_SETUP, PK_LINE, PK_XILL, PK_CONV, PK_FIN, PK_STATUS, PK_NTH, PK_HIST, PK_N };
@@ -1346,7 +1346,7 @@ static int launch_range(Context &C, Workspace &W, const BatchShape &b, cudaStrea
     }
     {
       ProfScope ps(PK_FIN, s);
-      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * 152, n, b.n_edges - b.n_sets, tab, sin, sst, cout, b.nza, user_e, flux, ntab, so));
+      RELX_CUDA(launch_finalize_relxill(s, b.n_sets < 2 * kSMs, n, b.n_edges - b.n_sets, tab, sin, sst, cout, b.nza, user_e, flux, ntab, so));
     }
   } else if (kind == RELX_RELCONV) {
     ProfScope ps(PK_CONV, s, kRelconvKernels);

@@ -539,8 +539,9 @@ __global__ void __launch_bounds__(NT, NT == kSetupThreads ? 4 : 1) setup_kernel(
     const double *ue = user_e + in.e_off;
     double *le = line_e + in.e_off;
     gn = in.n_ener;
-    // e / lineE (shift_energy_grid_1keV, XspecSpectrum.h:61-65) from the reciprocal and one exact remainder: within
-    // 2^-51 of an ulp of the quotient before its rounding.  A division is a dozen instructions of the FP64
+    // e / lineE (shift_energy_grid_1keV, XspecSpectrum.h:61-65) from the reciprocal and one exact remainder
+    // (Markstein, IBM J. Res. Dev. 34, 1990): within 2^-51 of an ulp of the quotient before its rounding, which is no
+    // proof that it is the division's result, but 4e8 random quotients all were.  A division is a dozen instructions of the FP64
     // pipe, which a warp holds 16 cycles each (one set of 3000 edges: set-up 54 us with divisions, 50 us so)
     const double lE = s.lineE, iE = m.inv_lineE;
     for (int j = tid; j <= gn; j += NT) {
@@ -1325,7 +1326,7 @@ cudaError_t setup_set_smem() {
 cudaError_t launch_setup(cudaStream_t s, int n_sets, const RelxTables &tab, int model, const RelxSetIn *sin,
                          const double *user_e, double *line_e, RelxSetState *sout, RelxRadial *rout,
                          RelxCorners *cout, RelxZoneCorners *zcout) {
-  if (n_sets <= 152)
+  if (n_sets <= kSMs)
     setup_kernel<kSetupFewThreads><<<n_sets, kSetupFewThreads, setup_smem_bytes(), s>>>(tab, model, sin, user_e, line_e,
                                                                                        sout, rout, cout, zcout);
   else

@@ -269,8 +269,8 @@ cudaError_t launch_xillver_model(cudaStream_t s, const RelxTables &tab, int n_se
   // a CTA of 1024 threads per SM while that takes one wave (152 sets 29 us, with 256 threads 39 us; 200 sets 43 us
   // and 47 us, 608 sets 89 us and 76 us), their output bins spread over the idle SMs (one set of 3000
   // bins 41 us by one CTA, 17 us by 12: the rebin's FP64 instructions hold an SM's pipe 16 cycles each)
-  if (n_sets <= 152)
-    xillver_model_kernel<1024><<<dim3(n_sets, out_parts(n_sets, n_bins, 256, 152)), 1024, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth, so);
+  if (n_sets <= kSMs)
+    xillver_model_kernel<1024><<<dim3(n_sets, out_parts(n_sets, n_bins, 256, kSMs)), 1024, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth, so);
   else
     xillver_model_kernel<256><<<n_sets, 256, smem, s>>>(tab, sin, user_e, sst, flux, nthq, nth, so);
   return cudaGetLastError();
