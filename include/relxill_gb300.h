@@ -121,8 +121,10 @@ int relx_eval_batch_sets(int model, int n_sets, const double *params, const doub
                          const int *ion_grad_type, const double *iongrad_index);
 
 /* Same with device buffers, asynchronous on `stream` (a cudaStream_t; NULL:
- * the library's stream).  flux_in (relconv) uses the energy-edge layout
- * (set i at energy_offsets[i]).  h_energy_offsets and h_ion_grad_type are host
+ * the library's stream).  Grids, spectra, fluxes and statuses that a kernel of the
+ * current device cannot use where they are (another device's memory without peer
+ * access, arrays not aligned to their elements) go by way of copies.  flux_in
+ * (relconv) uses the energy-edge layout (set i at energy_offsets[i]).  h_energy_offsets and h_ion_grad_type are host
  * copies used to size the launch; for relxilllpCp, whose ionisation-gradient
  * type is parameter 15, h_ion_grad_type carries those values (NULL: all 0; a
  * set that needs more zones than the launch was sized for fails with

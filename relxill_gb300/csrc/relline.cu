@@ -16,7 +16,7 @@
 //    and 1), so the lanes stay together (28 of 32 active in the loops over the runs of bins).  A
 //    warp per radius with its lanes on 32 consecutive bins used 20 of 32 and set every radius
 //    up alone: 5.22 ms per 4096 relxilllp sets of 10 zones, now 2.36 ms; instructions per set
-//    1.17 M, now 0.50 M.
+//    1.17 M, now 0.54 M.
 //  * Many sets: relline_solo_kernel, a warp per (set, zone, tile of 128 bins), no synchronisation
 //    between warps.  Few sets: relline_team_kernel, a CTA per (set, zone, tile of 32 bins) whose
 //    warps take groups in parallel and whose threads then add their values in the classes'
